@@ -125,6 +125,16 @@ int pb_assemble_f64(const double *vx, const double *vy, const double *vz, const 
 int pb_relax_f64(double *solution, const double *rhs, const double *screen, int64_t n,
                  double point_weight, int64_t iterations, void *stream);
 
+/* `cycles` whole V(pre, post) cycles (core.py:141-193: 40 sweeps on the 3^3
+ * grid) on a hierarchy of sides 2^k + 1, finest first, halving down to 3.  grids: four device
+ * pointers per level, (iterate, scratch, right-hand side, screen), each of the level's n^3
+ * doubles; the finest iterate is updated in place, the coarser iterates and right-hand sides and
+ * every scratch grid are overwritten.  workspace: pb_residual_workspace_size(sides[0]) + 256
+ * bytes.  Bit-exact.  (No counterpart in the reference, whose driver calls the operators.) */
+int pb_vcycles_f64(int64_t levels, const int64_t *sides, void *const *grids, double point_weight,
+                   int64_t pre, int64_t post, int64_t cycles, void *workspace, size_t workspace_bytes,
+                   void *stream);
+
 /* mpr_residual_f64 (_lib.py:26; capi.mojo:474-553): residual = rhs - A x
  * (bit-exact) and *norm = ||residual||_2 (device; summation order differs
  * from the serial reference by rounding only). */

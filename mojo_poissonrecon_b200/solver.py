@@ -22,6 +22,7 @@ Two solve modes:
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass, field
 
 import torch
@@ -54,7 +55,7 @@ class SolveStats:
 class Hierarchy64:
     """FP64 grids of every level, allocated once and reused across cycles."""
 
-    def __init__(self, screen: torch.Tensor, point_weight: float, workspace: nat.Workspace):
+    def __init__(self, screen: torch.Tensor, rhs: torch.Tensor, point_weight: float, workspace: nat.Workspace):
         self.device = screen.device
         self.pw = float(point_weight)
         self.sizes = level_sizes(screen.shape[0])
@@ -69,45 +70,34 @@ class Hierarchy64:
             nat.check(L.pb_restrict_f64(fine.data_ptr(), coarse.data_ptr(), fine.shape[0], s), "restrict")
             nat.check(L.pb_scale_f64(coarse.data_ptr(), coarse.numel(), 4.0, s), "scale")
             self.screens.append(coarse)
-        self.solutions = [torch.empty((n, n, n), dtype=torch.float64, device=self.device) for n in self.sizes]
-        self.rhs = [None] + [torch.empty((n, n, n), dtype=torch.float64, device=self.device) for n in self.sizes[1:]]
-        self.residuals = [torch.empty((n, n, n), dtype=torch.float64, device=self.device) for n in self.sizes]
+        grids = lambda sizes: [torch.empty((n, n, n), dtype=torch.float64, device=self.device) for n in sizes]
+        self.solutions = grids(self.sizes)
+        self.scratch = grids(self.sizes)
+        self.rhs = [rhs] + grids(self.sizes[1:])
         self.norm = torch.empty(1, dtype=torch.float64, device=self.device)
+        k = len(self.sizes)
+        self._sides = (ctypes.c_int64 * k)(*self.sizes)
+        self._grids = (ctypes.c_void_p * (4 * k))(*[t.data_ptr() for level in zip(
+            self.solutions, self.scratch, self.rhs, self.screens) for t in level])
 
     def fill(self, value: float) -> None:
-        for t in self.solutions:
-            nat.check(self.lib.pb_fill_f64(t.data_ptr(), t.numel(), value, self.stream), "fill")
+        """The finest iterate; the coarser ones start each cycle at zero."""
+        t = self.solutions[0]
+        nat.check(self.lib.pb_fill_f64(t.data_ptr(), t.numel(), value, self.stream), "fill")
 
-    def relax(self, level: int, iterations: int) -> None:
-        n = self.sizes[level]
-        nat.check(self.lib.pb_relax_f64(self.solutions[level].data_ptr(), self.rhs[level].data_ptr(),
-                                        self.screens[level].data_ptr(), n, self.pw, iterations, self.stream),
-                  "relax")
-
-    def residual(self, level: int, out_norm: torch.Tensor | None = None) -> None:
-        n = self.sizes[level]
+    def residual(self) -> None:
+        """The finest level's ||b - A x||_2 into `norm`."""
+        n = self.sizes[0]
         ptr, size = self.ws.get(self.lib.pb_residual_workspace_size(n))
-        norm = self.norm if out_norm is None else out_norm
-        nat.check(self.lib.pb_residual_f64(self.solutions[level].data_ptr(), self.rhs[level].data_ptr(),
-                                           self.screens[level].data_ptr(), self.residuals[level].data_ptr(), n,
-                                           self.pw, norm.data_ptr(), ptr, size, self.stream), "residual")
+        nat.check(self.lib.pb_residual_f64(self.solutions[0].data_ptr(), self.rhs[0].data_ptr(),
+                                           self.screens[0].data_ptr(), self.scratch[0].data_ptr(), n,
+                                           self.pw, self.norm.data_ptr(), ptr, size, self.stream), "residual")
 
-    def v_cycle(self, level: int, pre: int = 3, post: int = 3) -> None:
-        """core.py:141-193."""
-        L, s = self.lib, self.stream
-        n = self.sizes[level]
-        if n <= 3:
-            self.relax(level, 40)
-            return
-        self.relax(level, pre)
-        self.residual(level)
-        nat.check(L.pb_restrict_f64(self.residuals[level].data_ptr(), self.rhs[level + 1].data_ptr(), n, s),
-                  "restrict")
-        coarse = self.solutions[level + 1]
-        nat.check(L.pb_fill_f64(coarse.data_ptr(), coarse.numel(), 0.0, s), "fill")
-        self.v_cycle(level + 1, pre, post)
-        nat.check(L.pb_prolong_add_f64(coarse.data_ptr(), self.solutions[level].data_ptr(), n, s), "prolong")
-        self.relax(level, post)
+    def v_cycles(self, count: int, pre: int = 3, post: int = 3) -> None:
+        """core.py:141-193, `count` times in one library call."""
+        ptr, size = self.ws.get(self.lib.pb_residual_workspace_size(self.sizes[0]) + 256)
+        nat.check(self.lib.pb_vcycles_f64(len(self.sizes), self._sides, self._grids, self.pw, pre, post, count,
+                                          ptr, size, self.stream), "V-cycles")
 
 
 def norm(values: torch.Tensor, workspace: nat.Workspace, out: torch.Tensor) -> torch.Tensor:
@@ -125,30 +115,28 @@ def solve_fp64(rhs: torch.Tensor, screen: torch.Tensor, point_weight: float, wor
 
     Returns the level-0 solution and stats; stats.residual_norm is the absolute
     final ||rhs - A x||_2 as the reference reports it."""
-    h = Hierarchy64(screen, point_weight, workspace)
-    h.rhs[0] = rhs
+    h = Hierarchy64(screen, rhs, point_weight, workspace)
     stats = SolveStats()
     h.fill(0.5)  # core.py:270
     if has_points:
         if tol is None:
-            for _ in range(cycles):
-                h.v_cycle(0)
+            h.v_cycles(cycles)
             stats.cycles = cycles
         else:
             rhs_norm = norm(rhs, workspace, torch.empty(1, dtype=torch.float64, device=rhs.device))
             stats.rhs_norm = float(rhs_norm.item())
             target = tol * stats.rhs_norm
             while stats.cycles < max_cycles:
-                h.v_cycle(0)
+                h.v_cycles(1)
                 stats.cycles += 1
-                h.residual(0)
+                h.residual()
                 r = float(h.norm.item())
                 stats.history.append(r)
                 if r <= target:
                     break
     else:
         nat.check(h.lib.pb_fill_f64(h.solutions[0].data_ptr(), h.solutions[0].numel(), 0.0, h.stream), "fill")
-    h.residual(0)  # core.py:289-296: absolute final residual norm
+    h.residual()  # core.py:289-296: absolute final residual norm
     stats.residual_norm = float(h.norm.item())
     if stats.rhs_norm != stats.rhs_norm:  # nan: not computed yet
         rhs_norm = norm(rhs, workspace, torch.empty(1, dtype=torch.float64, device=rhs.device))
