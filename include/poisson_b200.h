@@ -125,15 +125,24 @@ int pb_assemble_f64(const double *vx, const double *vy, const double *vz, const 
 int pb_relax_f64(double *solution, const double *rhs, const double *screen, int64_t n,
                  double point_weight, int64_t iterations, void *stream);
 
-/* `cycles` whole V(pre, post) cycles (core.py:141-193: 40 sweeps on the 3^3
- * grid) on a hierarchy of sides 2^k + 1, finest first, halving down to 3.  grids: four device
- * pointers per level, (iterate, scratch, right-hand side, screen), each of the level's n^3
- * doubles; the finest iterate is updated in place, the coarser iterates and right-hand sides and
- * every scratch grid are overwritten.  workspace: pb_residual_workspace_size(sides[0]) + 256
- * bytes.  Bit-exact.  (No counterpart in the reference, whose driver calls the operators.) */
+/* `cycles` whole V(pre, post) cycles (core.py:141-193: 40 sweeps on the 3^3 grid) on a
+ * hierarchy of sides 2^k + 1 <= 1025, finest first, halving down to 3 (no counterpart in the
+ * reference, whose driver calls the operators; same bits as those).  grids: four device pointers per
+ * level, (iterate, right-hand side, screening flags, dense screen): the first three hold
+ * pb_vcycle_level_size's doubles, doubles and bytes in a layout of the library's own (levels of side
+ * <= 17: dense, no flags; below the first of these only the screen is read) and are prepared by
+ * pb_vcycle_setup_f64 from the finest dense right-hand side, the finest iterate starting at `init`;
+ * the screens are the caller's, dense, and non-negative as point_weight is.  norm (may be null) gets
+ * the finest ||rhs - A x||_2 after the last cycle; pb_vcycle_field_f64 the finest iterate as a dense
+ * grid. */
+int pb_vcycle_level_size(int64_t n, int64_t *doubles, int64_t *flag_bytes);
+int pb_vcycle_setup_f64(int64_t levels, const int64_t *sides, void *const *grids, const double *rhs,
+                        double init, void *stream);
+size_t pb_vcycle_workspace_size(int64_t n);
 int pb_vcycles_f64(int64_t levels, const int64_t *sides, void *const *grids, double point_weight,
-                   int64_t pre, int64_t post, int64_t cycles, void *workspace, size_t workspace_bytes,
-                   void *stream);
+                   int64_t pre, int64_t post, int64_t cycles, double *norm, void *workspace,
+                   size_t workspace_bytes, void *stream);
+int pb_vcycle_field_f64(int64_t n, const double *iterate, double *field, void *stream);
 
 /* mpr_residual_f64 (_lib.py:26; capi.mojo:474-553): residual = rhs - A x
  * (bit-exact) and *norm = ||residual||_2 (device; summation order differs

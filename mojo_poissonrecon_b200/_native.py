@@ -38,7 +38,11 @@ _SIGNATURES = {
     "pb_sample_attributes_f64": ([P, I, P, I, P, I, P, P], C),
     "pb_assemble_f64": ([P, P, P, P, P, I, F, F, P], C),
     "pb_relax_f64": ([P, P, P, I, F, I, P], C),
-    "pb_vcycles_f64": ([I, P, P, F, I, I, I, P, S, P], C),
+    "pb_vcycle_level_size": ([I, P, P], C),
+    "pb_vcycle_setup_f64": ([I, P, P, P, F, P], C),
+    "pb_vcycle_workspace_size": ([I], S),
+    "pb_vcycles_f64": ([I, P, P, F, I, I, I, P, P, S, P], C),
+    "pb_vcycle_field_f64": ([I, P, P, P], C),
     "pb_residual_workspace_size": ([I], S),
     "pb_residual_f64": ([P, P, P, P, I, F, P, P, S, P], C),
     "pb_norm_f64": ([P, I, P, P, S, P], C),

@@ -53,9 +53,11 @@ class SolveStats:
 
 
 class Hierarchy64:
-    """FP64 grids of every level, allocated once and reused across cycles."""
+    """FP64 levels of one solve: the iterate and right-hand side of each, in the
+    library's layout (pb_vcycle_level_size), and its dense screen."""
 
-    def __init__(self, screen: torch.Tensor, rhs: torch.Tensor, point_weight: float, workspace: nat.Workspace):
+    def __init__(self, screen: torch.Tensor, rhs: torch.Tensor, point_weight: float, workspace: nat.Workspace,
+                 init: float = 0.5):  # core.py:270
         self.device = screen.device
         self.pw = float(point_weight)
         self.sizes = level_sizes(screen.shape[0])
@@ -70,34 +72,35 @@ class Hierarchy64:
             nat.check(L.pb_restrict_f64(fine.data_ptr(), coarse.data_ptr(), fine.shape[0], s), "restrict")
             nat.check(L.pb_scale_f64(coarse.data_ptr(), coarse.numel(), 4.0, s), "scale")
             self.screens.append(coarse)
-        grids = lambda sizes: [torch.empty((n, n, n), dtype=torch.float64, device=self.device) for n in sizes]
-        self.solutions = grids(self.sizes)
-        self.scratch = grids(self.sizes)
-        self.rhs = [rhs] + grids(self.sizes[1:])
+        self.levels = []
+        for n in self.sizes:
+            doubles, flags = ctypes.c_int64(), ctypes.c_int64()
+            nat.check(L.pb_vcycle_level_size(n, ctypes.byref(doubles), ctypes.byref(flags)), "level size")
+            self.levels.append((torch.empty(doubles.value, dtype=torch.float64, device=self.device),
+                                torch.empty(doubles.value, dtype=torch.float64, device=self.device),
+                                torch.empty(max(flags.value, 1), dtype=torch.uint8, device=self.device)))
         self.norm = torch.empty(1, dtype=torch.float64, device=self.device)
         k = len(self.sizes)
         self._sides = (ctypes.c_int64 * k)(*self.sizes)
-        self._grids = (ctypes.c_void_p * (4 * k))(*[t.data_ptr() for level in zip(
-            self.solutions, self.scratch, self.rhs, self.screens) for t in level])
-
-    def fill(self, value: float) -> None:
-        """The finest iterate; the coarser ones start each cycle at zero."""
-        t = self.solutions[0]
-        nat.check(self.lib.pb_fill_f64(t.data_ptr(), t.numel(), value, self.stream), "fill")
-
-    def residual(self) -> None:
-        """The finest level's ||b - A x||_2 into `norm`."""
-        n = self.sizes[0]
-        ptr, size = self.ws.get(self.lib.pb_residual_workspace_size(n))
-        nat.check(self.lib.pb_residual_f64(self.solutions[0].data_ptr(), self.rhs[0].data_ptr(),
-                                           self.screens[0].data_ptr(), self.scratch[0].data_ptr(), n,
-                                           self.pw, self.norm.data_ptr(), ptr, size, self.stream), "residual")
+        self._grids = (ctypes.c_void_p * (4 * k))(*[t.data_ptr() for level, scr in zip(self.levels, self.screens)
+                                                    for t in (*level, scr)])
+        nat.check(L.pb_vcycle_setup_f64(k, self._sides, self._grids, rhs.data_ptr(), init, s), "V-cycle set-up")
 
     def v_cycles(self, count: int, pre: int = 3, post: int = 3) -> None:
-        """core.py:141-193, `count` times in one library call."""
-        ptr, size = self.ws.get(self.lib.pb_residual_workspace_size(self.sizes[0]) + 256)
+        """core.py:141-193, `count` times in one library call; the finest
+        ||b - A x||_2 after them into `norm`."""
+        ptr, size = self.ws.get(self.lib.pb_vcycle_workspace_size(self.sizes[0]))
         nat.check(self.lib.pb_vcycles_f64(len(self.sizes), self._sides, self._grids, self.pw, pre, post, count,
-                                          ptr, size, self.stream), "V-cycles")
+                                          self.norm.data_ptr(), ptr, size, self.stream), "V-cycles")
+
+    def field(self) -> torch.Tensor:
+        """The finest iterate as a dense grid; the levels' other arrays are released."""
+        n = self.sizes[0]
+        iterate = self.levels[0][0]
+        self.levels = self._grids = None  # the right-hand side's memory holds the grid where it is large
+        out = torch.empty((n, n, n), dtype=torch.float64, device=self.device)
+        nat.check(self.lib.pb_vcycle_field_f64(n, iterate.data_ptr(), out.data_ptr(), self.stream), "V-cycle field")
+        return out
 
 
 def norm(values: torch.Tensor, workspace: nat.Workspace, out: torch.Tensor) -> torch.Tensor:
@@ -115,30 +118,28 @@ def solve_fp64(rhs: torch.Tensor, screen: torch.Tensor, point_weight: float, wor
 
     Returns the level-0 solution and stats; stats.residual_norm is the absolute
     final ||rhs - A x||_2 as the reference reports it."""
-    h = Hierarchy64(screen, rhs, point_weight, workspace)
     stats = SolveStats()
-    h.fill(0.5)  # core.py:270
-    if has_points:
-        if tol is None:
-            h.v_cycles(cycles)
-            stats.cycles = cycles
-        else:
-            rhs_norm = norm(rhs, workspace, torch.empty(1, dtype=torch.float64, device=rhs.device))
-            stats.rhs_norm = float(rhs_norm.item())
-            target = tol * stats.rhs_norm
-            while stats.cycles < max_cycles:
-                h.v_cycles(1)
-                stats.cycles += 1
-                h.residual()
-                r = float(h.norm.item())
-                stats.history.append(r)
-                if r <= target:
-                    break
+    h = Hierarchy64(screen, rhs, point_weight, workspace, 0.5 if has_points else 0.0)
+    if not has_points:
+        h.v_cycles(0)
+    elif tol is None:
+        h.v_cycles(cycles)
+        stats.cycles = cycles
     else:
-        nat.check(h.lib.pb_fill_f64(h.solutions[0].data_ptr(), h.solutions[0].numel(), 0.0, h.stream), "fill")
-    h.residual()  # core.py:289-296: absolute final residual norm
-    stats.residual_norm = float(h.norm.item())
+        rhs_norm = norm(rhs, workspace, torch.empty(1, dtype=torch.float64, device=rhs.device))
+        stats.rhs_norm = float(rhs_norm.item())
+        target = tol * stats.rhs_norm
+        if max_cycles < 1:
+            h.v_cycles(0)
+        while stats.cycles < max_cycles:
+            h.v_cycles(1)
+            stats.cycles += 1
+            r = float(h.norm.item())
+            stats.history.append(r)
+            if r <= target:
+                break
+    stats.residual_norm = float(h.norm.item())  # core.py:289-296: absolute final residual norm
     if stats.rhs_norm != stats.rhs_norm:  # nan: not computed yet
         rhs_norm = norm(rhs, workspace, torch.empty(1, dtype=torch.float64, device=rhs.device))
         stats.rhs_norm = float(rhs_norm.item())
-    return h.solutions[0], stats
+    return h.field(), stats
