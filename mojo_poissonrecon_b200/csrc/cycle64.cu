@@ -288,12 +288,15 @@ static int launch_tail(int64_t n, const TailArgs& a, cudaStream_t s) {
 // sum needs no test.  A pass reads the other colour, its own right-hand side and a
 // byte per two nodes, and writes its own colour: 12.5 bytes per node of the grid.
 // The byte says whether either node has screening; only then is the dense screen
-// read (2 % of the nodes at 257^3) and the general division taken.  Without
+// read (2 % of the nodes at 257^3) and the general division taken.  On the finest
+// level it also says whether either right-hand side is not zero, and the pass moves
+// 8.5 bytes per node.  Without
 // screening the diagonal is 3 h^-2 .. 6 h^-2, and with y = RN(1 / d) off by at most
 // 2^-54 relative for these (h^-2 a power of two), a y is within one ulp of the
 // quotient and a single correction of Markstein's (above) rounds it correctly.
-// Measured on B200 at 257^3, one colour of one sweep: dense 110 us, split 45 us
-// (212 MB at 4.7 TB/s); a whole V(3,3) cycle 2.0 -> 1.1 ms.
+// Measured on B200 at 257^3, one colour of one sweep: dense 110 us, split 42 us
+// (126 MB of DRAM traffic; latency-bound: half of the warps resident, 58 % of issue
+// slots); a whole V(3,3) cycle 2.0 -> 1.0 ms.
 struct Split {
     int n, pitch, groups;  // entries per row (even), pairs of entries per row
     uint32_t plane, count;  // entries per plane and per colour, ghosts included (n <= 1025: below 2^31)
@@ -307,10 +310,14 @@ struct Split {
     __host__ __device__ __forceinline__ uint32_t node(int x, int y, int z) const { return at(x >> 1, y, z); }
 };
 
+// Of a pair of entries: either node has screening; either right-hand side is not zero (set everywhere below the
+// finest level, whose right-hand side is zero but for the nodes around the samples).
+constexpr uint8_t kScreened = 1, kSource = 2;
+
 struct SplitLevel {
     double* x[2];          // iterate by colour
     double* f[2];          // right-hand side by colour
-    uint8_t* screened[2];  // per pair of entries: either node has screening
+    uint8_t* flags[2];     // per pair of entries: kScreened, kSource
     const double* screen;  // dense
 };
 
@@ -329,16 +336,43 @@ struct Inverse {
     }
 };
 
-__device__ __forceinline__ double unscreened_quotient(double a, int degree, const Inverse& v) {
-    double d = v.d6, y = v.y6;
-    if (degree != 6) {
-        d = (double)degree * v.h2;
-        y = degree == 5 ? v.y5 : degree == 4 ? v.y4 : v.y3;
+__device__ __forceinline__ bool plain_exponent(double a) {  // |a| in [2^-900, 2^901)
+    return ((uint32_t)__double2hiint(a) & 0x7ff00000u) - (123u << 20) <= (1800u << 20);
+}
+
+// a / d by one correction of a y (above).
+__device__ __forceinline__ double corrected(double a, double d, double y) {
+    const double q = a * y;
+    return __fma_rn(__fma_rn(-d, q, a), y, q);
+}
+
+__device__ __forceinline__ double degree_inverse(int degree, const Inverse& v) {
+    return degree == 6 ? v.y6 : degree == 5 ? v.y5 : degree == 4 ? v.y4 : v.y3;
+}
+
+// The quotients of a pair of entries without screening.  `inner`: the pair's row is inside the y and z faces (the
+// same for nearly every warp), where only the first node can have fewer than six neighbours (x_face: at x = 0 or
+// n - 1; n - 1 is a multiple of four, so the second never lies there).
+__device__ __forceinline__ double2 unscreened_pair(double a0, double a1, bool inner, bool x_face, int degree_yz,
+                                                   const Inverse& v) {
+    double d0 = v.d6, y0 = v.y6, d1 = v.d6, y1 = v.y6;
+    if (inner) {
+        if (x_face) {
+            d0 = 5.0 * v.h2;
+            y0 = v.y5;
+        }
+    } else {
+        const int k0 = degree_yz + (x_face ? 1 : 2), k1 = degree_yz + 2;
+        d0 = (double)k0 * v.h2;
+        y0 = degree_inverse(k0, v);
+        d1 = (double)k1 * v.h2;
+        y1 = degree_inverse(k1, v);
     }
-    const uint32_t e = (uint32_t)__double2hiint(a) & 0x7ff00000u;
-    double q = a * y;
-    q = __fma_rn(__fma_rn(-d, q, a), y, q);
-    if (e - (123u << 20) > (1800u << 20)) q = a == 0.0 ? a : a / d;  // outside [2^-900, 2^901)
+    double2 q = make_double2(corrected(a0, d0, y0), corrected(a1, d1, y1));
+    if (!plain_exponent(a0) || !plain_exponent(a1)) {
+        if (!plain_exponent(a0)) q.x = a0 == 0.0 ? a0 : a0 / d0;
+        if (!plain_exponent(a1)) q.y = a1 == 0.0 ? a1 : a1 / d1;
+    }
     return q;
 }
 
@@ -356,7 +390,7 @@ __global__ void __launch_bounds__(256) split_setup_kernel(Split g, SplitLevel L,
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         double v[2] = {0.0, 0.0}, f[2] = {0.0, 0.0};
-        bool screened = false;
+        bool screened = false, source = !rhs;
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
             const int x = 4 * k + 2 * m + ((y + z + c) & 1);
@@ -364,13 +398,14 @@ __global__ void __launch_bounds__(256) split_setup_kernel(Split g, SplitLevel L,
                 const int64_t i = ((int64_t)z * g.n + y) * g.n + x;
                 v[m] = init;
                 if (rhs) f[m] = 0.0 + rhs[i];
+                source |= f[m] != 0.0;
                 screened |= L.screen[i] != 0.0;
             }
         }
         const uint32_t at = g.at(2 * k, y, z);
         *reinterpret_cast<double2*>(L.x[c] + at) = make_double2(v[0], v[1]);
         *reinterpret_cast<double2*>(L.f[c] + at) = make_double2(f[0], f[1]);
-        if (in) L.screened[c][((uint32_t)z * g.n + y) * g.groups + k] = screened;
+        if (in) L.flags[c][((uint32_t)z * g.n + y) * g.groups + k] = (screened ? kScreened : 0) | (source ? kSource : 0);
     }
 }
 
@@ -389,12 +424,14 @@ __device__ __forceinline__ double2 pair_at(const double* p, uint32_t i) {
 // One colour of one sweep: own <- from other.  A thread takes two neighbouring
 // entries of a row and marches down z with the other colour's planes z - 1, z and
 // z + 1 in registers.  ZERO: the other colour is zero (a coarse level's first
-// pass).  Bound by memory latency: five blocks per SM (48 registers) measured best.
-template <bool ZERO>
+// pass).  SPARSE (the finest level): the right-hand side is read only where it is
+// not zero, its flag having been read a plane ahead.  Bound by memory latency: five
+// blocks per SM (48 registers) measured best.
+template <bool ZERO, bool SPARSE>
 __global__ void __launch_bounds__(256, 5) split_relax_kernel(Split g, double* __restrict__ own,
                                                              const double* __restrict__ other,
                                                              const double* __restrict__ f,
-                                                             const uint8_t* __restrict__ screened,
+                                                             const uint8_t* __restrict__ flags,
                                                              const double* __restrict__ screen, Inverse v, int colour,
                                                              int planes) {
     const uint32_t t = blockIdx.x * 256u + threadIdx.x;
@@ -407,12 +444,28 @@ __global__ void __launch_bounds__(256, 5) split_relax_kernel(Split g, double* __
         below = pair_at(other, at - g.plane);
         here = pair_at(other, at);
     }
-    const int degree_y = (y > 0) + (y + 1 < n);
+    const int degree_y = (y > 0) + (y + 1 < n), k_last = (n - 1) / 4 - 1;
+    const bool k_face = k == 0 || 4 * k == n - 1;
+    int flag_here = SPARSE ? flags[((uint32_t)z0 * n + y) * g.groups + k] : 0;
     for (int z = z0; z < z1; ++z, at += g.plane) {
         const int odd = (y + z + colour) & 1, x = 4 * k + odd;  // nodes x and x + 2
         double s0 = 0.0, s1 = 0.0;
-        const int flag = screened[((uint32_t)z * n + y) * g.groups + k];
-        const double2 rhs = pair_at(f, at);
+        double2 rhs = make_double2(0.0, 0.0);
+        int flag, ahead = 0;
+        if (SPARSE) {
+            flag = flag_here;
+            if (z + 1 < z1) ahead = flags[((uint32_t)(z + 1) * n + y) * g.groups + k];
+            if (flag & kSource) rhs = pair_at(f, at);
+        } else {
+            flag = flags[((uint32_t)z * n + y) * g.groups + k];
+            rhs = pair_at(f, at);
+        }
+        double scr0 = 0.0, scr1 = 0.0;
+        if (flag & kScreened) {
+            const double* scr = screen + ((int64_t)z * n + y) * n + x;
+            if (x < n) scr0 = scr[0];
+            if (x + 2 < n) scr1 = scr[2];
+        }
         if (!ZERO) {
             above = pair_at(other, at + g.plane);
             const double2 up = pair_at(other, at - g.pitch), down = pair_at(other, at + g.pitch);
@@ -430,28 +483,30 @@ __global__ void __launch_bounds__(256, 5) split_relax_kernel(Split g, double* __
         }
         const double a0 = rhs.x + s0 * v.h2, a1 = rhs.y + s1 * v.h2;
         const int degree = degree_y + (z > 0) + (z + 1 < n);
-        const int d0 = degree + (x > 0) + (x + 1 < n), d1 = degree + 1 + (x + 3 < n);
+        const bool x_face = k_face && !odd;
         double2 q;
-        if (!flag) {
-            q.x = unscreened_quotient(a0, d0, v);
-            q.y = unscreened_quotient(a1, d1, v);
+        if (!(flag & kScreened)) {
+            q = unscreened_pair(a0, a1, degree == 4, x_face, degree, v);
         } else {
-            const double* scr = screen + ((int64_t)z * n + y) * n + x;
-            const double e0 = (double)d0 * v.h2 + v.pw * (x < n ? scr[0] : 0.0) * v.h2;
-            const double e1 = (double)d1 * v.h2 + v.pw * (x + 2 < n ? scr[2] : 0.0) * v.h2;
+            const int d0 = degree + (x_face ? 1 : 2), d1 = degree + 2;
+            const double e0 = (double)d0 * v.h2 + v.pw * scr0 * v.h2, e1 = (double)d1 * v.h2 + v.pw * scr1 * v.h2;
             q.x = e0 > 1.0e-30 ? a0 / e0 : own[at];
             q.y = e1 > 1.0e-30 ? a1 / e1 : own[at + 1];
         }
-        if (x >= n) q.x = 0.0;  // the row's zero entries
-        if (x + 2 >= n) q.y = 0.0;
+        if (k >= k_last) {  // the row's zero entries
+            if (x >= n) q.x = 0.0;
+            if (x + 2 >= n) q.y = 0.0;
+        }
         *reinterpret_cast<double2*>(own + at) = q;
         below = here;
         here = above;
+        flag_here = ahead;
     }
 }
 
 // r = rhs - A x (capi.mojo:413-553) at the four nodes 4k .. 4k + 3 of row y, plane by plane down z, with both
 // colours' planes z - 1, z and z + 1 in registers.
+template <bool SPARSE>
 struct ResidualMarch {
     const Split g;
     const SplitLevel& L;
@@ -459,6 +514,7 @@ struct ResidualMarch {
     const int y, k, degree_y;
     uint32_t at;
     double2 below[2], here[2], above[2];  // by colour
+    int flag[2];
 
     __device__ __forceinline__ ResidualMarch(const Split& split, const SplitLevel& level, const Inverse& inverse,
                                              int row, int group, int z0)
@@ -468,6 +524,13 @@ struct ResidualMarch {
         below[1] = pair_at(L.x[1], at - g.plane);
         here[0] = pair_at(L.x[0], at);
         here[1] = pair_at(L.x[1], at);
+        read_flags(z0);
+    }
+
+    __device__ __forceinline__ void read_flags(int z) {
+        const uint32_t i = ((uint32_t)z * g.n + y) * g.groups + k;
+        flag[0] = L.flags[0][i];
+        flag[1] = L.flags[1][i];
     }
 
     __device__ __forceinline__ void step(int z, double (&r)[4]) {
@@ -475,11 +538,15 @@ struct ResidualMarch {
         above[0] = pair_at(L.x[0], at + g.plane);
         above[1] = pair_at(L.x[1], at + g.plane);
         const uint32_t row = (uint32_t)z * n + y;
+        const int now[2] = {flag[0], flag[1]};
+        if (z + 1 < n) read_flags(z + 1);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const int first = odd ^ c, x = 4 * k + first;  // colour c: nodes x and x + 2
             const double* o = L.x[1 - c];
-            const double2 up = pair_at(o, at - g.pitch), down = pair_at(o, at + g.pitch), f = pair_at(L.f[c], at);
+            const double2 up = pair_at(o, at - g.pitch), down = pair_at(o, at + g.pitch);
+            double2 f = make_double2(0.0, 0.0);
+            if (!SPARSE || (now[c] & kSource)) f = pair_at(L.f[c], at);
             const double outer = o[first ? at + 2 : at - 1];
             const double2 mid = here[1 - c];
             double s0 = mid.x + (first ? mid.y : outer), s1 = mid.y + (first ? outer : mid.x);
@@ -492,7 +559,7 @@ struct ResidualMarch {
             s0 += above[1 - c].x;
             s1 += above[1 - c].y;
             double e0 = (double)(degree + (x > 0) + (x + 1 < n)) * v.h2, e1 = (double)(degree + 1 + (x + 3 < n)) * v.h2;
-            if (L.screened[c][row * g.groups + k]) {
+            if (now[c] & kScreened) {
                 const double* scr = L.screen + (int64_t)row * n + x;
                 if (x < n) e0 += v.pw * scr[0] * v.h2;
                 if (x + 2 < n) e1 += v.pw * scr[2] * v.h2;
@@ -520,14 +587,16 @@ struct ResidualMarch {
 // without storing it: a block owns up to kCoarseX x kCoarseY coarse columns and
 // marches down z; each fine residual plane over them goes to shared memory once
 // (two by parity: one barrier per plane) and is added to the coarse sums it belongs
-// to, in the reference's order.  SPLIT_OUT: the coarse level is colour-split (else
+// to, in the reference's order.  257^3: 115 us (tiles of 34 x 9, 34 x 4 and 18 x 9
+// coarse columns 118-124) against 170 for the dense residual and 100 for the dense
+// restriction.  SPLIT_OUT: the coarse level is colour-split (else
 // dense: the tail's top level).
-constexpr int kCoarseX = 34, kCoarseY = 9;  // kCoarseX even: 129 = 4 x 33 coarse columns in four tiles
+constexpr int kCoarseX = 34, kCoarseY = 6;  // kCoarseX even: 129 = 4 x 33 coarse columns in four tiles
 constexpr int kResGroups = kCoarseX / 2 + 1, kResRows = 2 * kCoarseY + 1, kResPitch = 4 * kResGroups;
 constexpr int kRestrictThreads = (kResGroups * kResRows + 31) / 32 * 32;
 
-template <bool SPLIT_OUT>
-__global__ void __launch_bounds__(kRestrictThreads, 2) split_restrict_kernel(Split g, const SplitLevel L, Inverse v,
+template <bool SPLIT_OUT, bool SPARSE>
+__global__ void __launch_bounds__(kRestrictThreads, 3) split_restrict_kernel(Split g, const SplitLevel L, Inverse v,
                                                                              double* __restrict__ out0,
                                                                              double* __restrict__ out1, int width,
                                                                              int height, int planes) {
@@ -544,7 +613,7 @@ __global__ void __launch_bounds__(kRestrictThreads, 2) split_restrict_kernel(Spl
     const Split cg(cn);
     double acc = 0.0;
     const int z0 = max(2 * Z0 - 1, 0), z1 = min(2 * Z1 - 1, n - 1);
-    ResidualMarch march(g, L, v, in ? y : 0, in ? k : 0, z0);
+    ResidualMarch<SPARSE> march(g, L, v, in ? y : 0, in ? k : 0, z0);
     for (int z = z0; z <= z1; ++z) {
         double* plane = res[z & 1];
         double r[4];
@@ -621,7 +690,7 @@ __global__ void __launch_bounds__(256) split_norm_kernel(Split g, const SplitLev
     if (t < (uint32_t)g.n * g.groups) {
         const int y = t / (uint32_t)g.groups, k = t - y * g.groups;
         const int z0 = blockIdx.y * planes, z1 = min(g.n, z0 + planes);
-        ResidualMarch march(g, L, v, y, k, z0);
+        ResidualMarch<true> march(g, L, v, y, k, z0);
         for (int z = z0; z < z1; ++z) {
             double r[4];
             march.step(z, r);
@@ -666,36 +735,35 @@ static int norm_blocks(const Split& g) { return norm_grid(g).x * norm_grid(g).y;
 // 4: 8.3, 1: 10.3, 8: 12.4; smaller levels are one wave of latency whatever the split, so one plane each.
 static int relax_planes(int n) { return n >= 257 ? 6 : n >= 129 ? 4 : 1; }
 
-template <bool ZERO>
+template <bool ZERO, bool SPARSE>
 static int launch_split_relax(const SplitLevel& L, int n, double pw, int colour, cudaStream_t s) {
     const Split g(n);
     const int planes = relax_planes(n);
-    split_relax_kernel<ZERO><<<dim3(tiles(n * g.groups, 256), tiles(n, planes)), 256, 0, s>>>(
-        g, L.x[colour], L.x[1 - colour], L.f[colour], L.screened[colour], L.screen, Inverse(n, pw), colour, planes);
+    split_relax_kernel<ZERO, SPARSE><<<dim3(tiles(n * g.groups, 256), tiles(n, planes)), 256, 0, s>>>(
+        g, L.x[colour], L.x[1 - colour], L.f[colour], L.flags[colour], L.screen, Inverse(n, pw), colour, planes);
     PB_CHECK_LAUNCH("split_relax_kernel");
     return PB_OK;
 }
 
-static int launch_split_sweeps(const SplitLevel& L, int n, double pw, int sweeps, bool from_zero, cudaStream_t s) {
+static int launch_split_sweeps(const SplitLevel& L, int n, double pw, int sweeps, bool finest, bool from_zero,
+                               cudaStream_t s) {
     for (int k = 0; k < 2 * sweeps; ++k)
-        PB_TRY(k == 0 && from_zero ? launch_split_relax<true>(L, n, pw, 0, s)
-                                   : launch_split_relax<false>(L, n, pw, k & 1, s));
+        PB_TRY(finest                ? (launch_split_relax<false, true>(L, n, pw, k & 1, s))
+               : k == 0 && from_zero ? (launch_split_relax<true, false>(L, n, pw, 0, s))
+                                     : (launch_split_relax<false, false>(L, n, pw, k & 1, s)));
     return PB_OK;
 }
 
-static int launch_split_restrict(const SplitLevel& L, int n, double pw, const SplitLevel& below, bool split_below,
-                                 cudaStream_t s) {
+static int launch_split_restrict(const SplitLevel& L, int n, double pw, bool finest, const SplitLevel& below,
+                                 bool split_below, cudaStream_t s) {
     const Split g(n);
     const int cn = (n + 1) / 2, width = (tiles(cn, tiles(cn, kCoarseX)) + 1) / 2 * 2, height = tiles(cn, tiles(cn, kCoarseY));
     const int planes = cn >= 129 ? 8 : cn >= 65 ? 4 : 1;
     const dim3 grid(tiles(cn, width), tiles(cn, height), tiles(cn, planes));
     const Inverse v(n, pw);
-    if (split_below)
-        split_restrict_kernel<true><<<grid, kRestrictThreads, 0, s>>>(g, L, v, below.f[0], below.f[1], width, height,
-                                                                      planes);
-    else
-        split_restrict_kernel<false><<<grid, kRestrictThreads, 0, s>>>(g, L, v, below.f[0], nullptr, width, height,
-                                                                       planes);
+    auto kernel = split_below ? (finest ? split_restrict_kernel<true, true> : split_restrict_kernel<true, false>)
+                              : (finest ? split_restrict_kernel<false, true> : split_restrict_kernel<false, false>);
+    kernel<<<grid, kRestrictThreads, 0, s>>>(g, L, v, below.f[0], below.f[1], width, height, planes);
     PB_CHECK_LAUNCH("split_restrict_kernel");
     return PB_OK;
 }
@@ -728,8 +796,8 @@ static SplitLevel level_of(void* const* grids, int64_t l, int64_t n) {
         const Split g((int)n);
         L.x[1] = L.x[0] + g.count;
         L.f[1] = L.f[0] + g.count;
-        L.screened[0] = (uint8_t*)grids[4 * l + 2];
-        L.screened[1] = L.screened[0] + (size_t)n * n * g.groups;
+        L.flags[0] = (uint8_t*)grids[4 * l + 2];
+        L.flags[1] = L.flags[0] + (size_t)n * n * g.groups;
     }
     return L;
 }
@@ -852,14 +920,14 @@ extern "C" int pb_vcycles_f64(int64_t levels, const int64_t* sides, void* const*
         for (int64_t c = 0; c < cycles; ++c) {
             for (int64_t l = 0; l < top; ++l) {
                 const int n = (int)sides[l];
-                PB_TRY(launch_split_sweeps(level[l], n, point_weight, (int)pre, l > 0, s));
-                PB_TRY(launch_split_restrict(level[l], n, point_weight, level[l + 1], l + 1 < top, s));
+                PB_TRY(launch_split_sweeps(level[l], n, point_weight, (int)pre, l == 0, true, s));
+                PB_TRY(launch_split_restrict(level[l], n, point_weight, l == 0, level[l + 1], l + 1 < top, s));
             }
             PB_TRY(launch_tail(sides[top], tail, s));
             for (int64_t l = top - 1; l >= 0; --l) {
                 const int n = (int)sides[l];
                 PB_TRY(launch_split_prolong(level[l], n, level[l + 1], l + 1 < top, s));
-                PB_TRY(launch_split_sweeps(level[l], n, point_weight, (int)post, false, s));
+                PB_TRY(launch_split_sweeps(level[l], n, point_weight, (int)post, l == 0, false, s));
             }
         }
     }
