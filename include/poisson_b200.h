@@ -237,6 +237,14 @@ size_t pb_defect_workspace_size(int64_t n);
 int pb_defect_f64(const double *x_old, const float *e, double *x_new, const double *rhs,
                   const double *screen, int64_t n, double point_weight, float *r32, double *r64,
                   double *norm2, void *workspace, size_t workspace_bytes, void *stream);
+/* The start of a refined solve in one pass over the dense rhs and screen: level 0's D, 1/D and
+ * weights as pb_level_setup_f32, x0 = 1/2 (dense FP64), r32 = b - A x0 (padded), *norm2 =
+ * ||b - A x0||^2, *bnorm = ||b||, and copies of rhs and screen (either NULL: none). */
+size_t pb_refine_start_workspace_size(int64_t n);
+int pb_refine_start_f64(const double *rhs, const double *screen, int64_t n, double point_weight,
+                        double *rhs_copy, double *screen_copy, double *x0, float *D, float *invD, float *weights,
+                        float *r32, double *norm2, double *bnorm, void *workspace, size_t workspace_bytes,
+                        void *stream);
 /* FP64 flexible conjugate gradients, FCG(1), preconditioned by the FP32
  * V-cycle, in two passes per iteration (no counterpart in the reference, which
  * repeats V-cycles, core.py:274-285).  Device scalars scal[0..4]: (p, Ap),
@@ -380,7 +388,8 @@ int pb_coarse27_cycle_f32(int64_t count, const int64_t *sizes, const float *imag
                           int64_t pre, int64_t post, int64_t inner, void *stream);
 
 /* A whole preconditioner hierarchy's set-up from one call: the launches of
- * pb_level_setup_f32 (level 0 from the FP64 screen; for a 27-point level 0 also
+ * pb_level_setup_f32 (level 0 from the FP64 screen, or, screen NULL, none: its arrays are there
+ * already; for a 27-point level 0 also
  * pb_level27_from7_f32 and pb_level27_finish_f32), then per level l >= 1
  * pb_galerkin_f32 from level l-1, pb_level27_finish_f32, and pb_pack27_f32 of
  * level l-1 when it is packed; pb_coarse_inverse_f64 of the last level and
@@ -475,14 +484,13 @@ int pb_batch_loop_condition(unsigned long long handle, const double *scal, const
  *   SWEEP_Z_CHUNK          planes per block of pb_sweep_tma_f32 when its z_chunk <= 0
  *   RESTRICT_PLANES        coarse planes per block of pb_residual_restrict_f32 (default 4)
  *   PROLONG_PLANES         fine planes per block of pb_prolong_fac_f32
- *   FCG_DIRECTION_PLANES   planes per block of pb_fcg_direction_f64 (default 24, at least 8)
- *   FCG_UPDATE_PLANES      planes per block of pb_fcg_update_f64 (default 24, at least 8)
+ *   FCG_DIRECTION_PLANES   planes per block of pb_fcg_direction_f64 (default 24; 8 at n <= 129, 4 at n <= 65; at least 4)
+ *   FCG_UPDATE_PLANES      planes per block of pb_fcg_update_f64 (as FCG_DIRECTION_PLANES)
  *   FCG_DIRECTION_VARIANT  register budget of pb_fcg_direction_f64: 0 = 4 resident
  *                          blocks per SM, 1 = 6, 2 = 8
- *   RESTRICT_VARIANT       pb_residual_restrict_f32: 1 = both fine planes of a coarse
- *                          plane in one loop over their items; 2 = the FP32 cycle
- *                          calls pb_residual_restrict_tma_f32 instead; 3 = as 1 with
- *                          320 threads per block
+ *   RESTRICT_VARIANT       pb_residual_restrict_f32: 0 (and 1) = 256 threads per block;
+ *                          2 = the FP32 cycle calls pb_residual_restrict_tma_f32 instead;
+ *                          3 = 320 threads per block
  *   RELAX27_VARIANT        pb_relax27p_f32 (per level side): 1 = the neighbour planes
  *                          staged in shared memory
  *   RESIDUAL27_VARIANT     pb_residual_restrict27p_f32 (per level side): 1 = the
@@ -493,9 +501,8 @@ int pb_batch_loop_condition(unsigned long long handle, const double *scal, const
  *                          computes only the lanes it updates: (5 planes, 2 blocks),
  *                          (6, 2), (4, 3); 6, 7, 8 = the same with one barrier per
  *                          plane (a ring slot refilled one step earlier)
- *   FCG_UPDATE_VARIANT     pb_fcg_update_f64: 0 = 5 resident blocks per SM,
- *                          1 = 6 resident blocks per SM, 2 = 8, 3 = the next two planes
- *                          prefetched into shared memory by cp.async, 4 = three planes
+ *   FCG_UPDATE_VARIANT     pb_fcg_update_f64: planes prefetched into shared memory by
+ *                          cp.async: 0 (and 1 to 3) = the next two, 4 = three
  * The plane counts also apply to the grouped launches described after they are
  * set.  value 0 clears an entry.  Results do not depend on these values, except
  * the FCG passes' planes per block: they shape the inner products' partial-sum

@@ -67,6 +67,8 @@ _SIGNATURES = {
     "pb_level_setup_f32": ([P, I, F, P, P, P, P], C),
     "pb_defect_workspace_size": ([I], S),
     "pb_defect_f64": ([P, P, P, P, P, I, F, P, P, P, P, S, P], C),
+    "pb_refine_start_workspace_size": ([I], S),
+    "pb_refine_start_f64": ([P, P, I, F, P, P, P, P, P, P, P, P, P, P, S, P], C),
     "pb_fcg_workspace_size": ([I], S),
     "pb_fcg_direction_f64": ([P, P, P, P, P, I, F, P, P, P, S, P], C),
     "pb_fcg_update_f64": ([P, P, P, P, P, P, P, P, I, F, P, P, P, S, P], C),

@@ -44,7 +44,7 @@ import torch
 
 from . import _native as nat
 from . import _sync, _trace, core
-from .solver import SolveStats, norm
+from .solver import SolveStats
 from .solver32 import (GRAPH_CAPTURE_LOCK, MAX_ITER, TMA_MIN_N, Hierarchy32, apply_tuning, galerkin_scratch_bytes,
                        level0_sweeps)
 
@@ -150,16 +150,14 @@ def _lane_streams(device: torch.device, count: int) -> list:
 
 
 class _PrologueLane:
-    """One prologue lane's stream and scratch (Galerkin, defect, norm)."""
+    """One prologue lane's stream and scratch (Galerkin products, the start's sums)."""
 
     def __init__(self, lib, device: torch.device, stream: torch.cuda.Stream, galerkin_ws: torch.Tensor,
-                 defect_bytes: int):
+                 start_bytes: int):
         self.stream = stream
         self.galerkin_ws = galerkin_ws
-        self.defect_ws = nat.Workspace(device)
-        self.defect_ptr, self.defect_size = self.defect_ws.get(defect_bytes)
-        self.norm_ws = nat.Workspace(device)
-        self.norm_ws.get(1 << 16)
+        self.start_ws = nat.Workspace(device)
+        self.start_ws.get(start_bytes)
 
 
 def _take_cloud(n: int, device: torch.device, galerkin_ws: torch.Tensor) -> _Cloud:
@@ -227,13 +225,13 @@ class BatchSolver:
             parts = [int(self.lib.pb_batch_fcg_partials(n)) for n in self.sides]
             self.part_offsets = np.concatenate([[0], np.cumsum(parts)]).astype(np.int64)
             self.partials = torch.zeros(int(self.part_offsets[-1]), dtype=torch.float64, device=self.device)
-            defect = max(int(self.lib.pb_defect_workspace_size(n)) for n in set(self.sides))
+            start = max(int(self.lib.pb_refine_start_workspace_size(n)) for n in set(self.sides))
             lanes = min(PROLOGUE_LANES, K) if scratch <= PROLOGUE_SCRATCH else 1
             streams = [self.stream] if lanes == 1 else _lane_streams(self.device, lanes)
-            self.lanes = [_PrologueLane(self.lib, self.device, streams[0], self.galerkin_ws, defect)]
+            self.lanes = [_PrologueLane(self.lib, self.device, streams[0], self.galerkin_ws, start)]
             for j in range(1, lanes):
                 ws = torch.empty_like(self.galerkin_ws)
-                self.lanes.append(_PrologueLane(self.lib, self.device, streams[j], ws, defect))
+                self.lanes.append(_PrologueLane(self.lib, self.device, streams[j], ws, start))
             for k, c in enumerate(self.clouds):  # cloud k's set-up runs on lane k % lanes
                 c.h.galerkin_ws = self.lanes[k % lanes].galerkin_ws
         self.graph = ctypes.c_void_p()
@@ -398,23 +396,17 @@ class BatchSolver:
         return [x.clone() for x in xs], stats  # on the caller's stream
 
     def _prologue_lane(self, j: int, start: torch.cuda.Event, rhs, screen, pws) -> None:
-        """Lane j's clouds (k = j, j + lanes, ...): levels' set-up, x0 = 0.5 and its
-        residual, ||b||; on the lane's stream, after `start`."""
-        L, lane = self.lib, self.lanes[j]
+        """Lane j's clouds (k = j, j + lanes, ...): level 0, x0 = 0.5 and its residual,
+        ||b||, the coarse levels' set-up; on the lane's stream, after `start`."""
+        lane = self.lanes[j]
         if lane.stream is not self.stream:
             lane.stream.wait_event(start)
         with torch.cuda.device(self.device), torch.cuda.stream(lane.stream):  # a worker thread's device too
-            s = nat.stream_handle()
             for k in range(j, len(self.clouds), len(self.lanes)):
                 c = self.clouds[k]
-                c.h.setup(screen[k], pws[k])
-                x0 = c.xs[0]
-                nat.check(L.pb_fill_f64(x0.data_ptr(), x0.numel(), 0.5, s), "fill")  # core.py:270
-                nat.check(L.pb_defect_f64(x0.data_ptr(), None, None, rhs[k].data_ptr(), screen[k].data_ptr(),
-                                          c.n, pws[k], c.h.levels[0].rhs.data_ptr(), None,
-                                          self.norm2[k:k + 1].data_ptr(), lane.defect_ptr, lane.defect_size, s),
-                          "defect")
-                norm(rhs[k], lane.norm_ws, self.bnorm[k:k + 1])
+                c.h.start(rhs[k], screen[k], pws[k], (None, None), c.xs[0], self.norm2[k:k + 1],
+                          self.bnorm[k:k + 1], lane.start_ws)
+                c.h.setup(None, pws[k])
 
     def _prologue(self, rhs, screen, pws) -> None:
         """Every cloud's prologue, spread over the prologue lanes (host threads

@@ -26,16 +26,21 @@
 // direction, and the residual is recomputed from x in FP64 every iteration,
 // so the rounding perturbs alpha and beta by ~1e-7 relative and never the
 // measured residual.
+#include <type_traits>
+
 #include "batch.cuh"
 #include "common.cuh"
 
 namespace pb {
 namespace fcg {
 
-// pass 1: 256 (x, y) columns per block; both passes kTZ planes deep unless the
-// autotuner chose otherwise (measured: 16 -> 24, pass 1 82 -> 78 us).  Partial
-// sums are sized for the shallowest depth a launch may use, kMinTZ.
-constexpr int kTZ = 24, kMinTZ = 8, kThreads = 256;
+// pass 1: 256 (x, y) columns per block; both passes planes_of(n) planes deep unless
+// the autotuner chose otherwise (257^3, pass 1: 16 planes 82 us, 24 planes 78).  A
+// block walks its planes one after another, so small grids take fewer planes for
+// more blocks: at 65^3, 24 planes leave 81 blocks of pass 2 for 148 SMs (26.6 us),
+// 4 planes 459.  Partial sums are sized for the shallowest depth a launch may use, kMinTZ.
+constexpr int kTZ = 24, kMinTZ = 4, kThreads = 256;
+__host__ __device__ constexpr int planes_of(int n) { return n <= 65 ? 4 : n <= 129 ? 8 : kTZ; }
 
 // Pass 2 tile: 32 x 8 nodes per block, kTZ planes deep.
 constexpr int kUX = 32, kUY = 8, kUThreads = kUX * kUY;
@@ -78,6 +83,15 @@ __device__ __forceinline__ int64_t block_index() {
     return ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
 }
 
+// The multiply-adds of both passes are written out: left to the compiler, two
+// instantiations of a body (single and grouped launches, planes known or not) may
+// fuse differently, and a cloud would differ in the last bits alone and in a batch.
+
+// (A v)_i: degree and screening at the node, its value and its neighbours' sum s.
+__device__ __forceinline__ double applied(int degree, double pw, double screen, double h2, double value, double s) {
+    return __fma_rn(__fma_rn(__dmul_rn(pw, screen), h2, __dmul_rn((double)degree, h2)), value, -__dmul_rn(s, h2));
+}
+
 // Pass 1: per-block (z, Az), (Az, p_prev), (z, r32), (p_prev, r32); flags[1]
 // (iterations done) selects p_prev = p[it & 1]; flags[0] != 0 on the first step.
 // Each thread marches down its column with z of planes k - 1 and k in
@@ -115,14 +129,14 @@ __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z,
             zb = zm;
             zm = za;
             const int deg = degxy + (k > 0) + (k + 1 < n);
-            const double az = ((double)deg * h2 + pw * screen[i] * h2) * zc - s * h2;
+            const double az = applied(deg, pw, screen[i], h2, zc, s);
             const double rc = (double)r32[c];
-            v[0] += zc * az;
-            v[2] += zc * rc;
+            v[0] = __fma_rn(zc, az, v[0]);
+            v[2] = __fma_rn(zc, rc, v[2]);
             if (!first) {
                 const double pv = (double)pp[i];
-                v[1] += az * pv;
-                v[3] += pv * rc;
+                v[1] = __fma_rn(az, pv, v[1]);
+                v[3] = __fma_rn(pv, rc, v[3]);
             }
         }
     }
@@ -161,8 +175,9 @@ __device__ __forceinline__ void direction_finish_body(const double* __restrict__
     const bool first = flags[0] != 0;
     const double pap_prev = scal[0];
     const double beta = first || !(pap_prev > 0.0) ? 0.0 : zq / pap_prev;
-    const double pap = first ? zz : zz - 2.0 * beta * zq + beta * beta * pap_prev;
-    const double prn = first ? zr : zr - beta * pr;
+    const double pap =
+        first ? zz : __fma_rn(__dmul_rn(beta, beta), pap_prev, __fma_rn(__dmul_rn(-2.0, beta), zq, zz));
+    const double prn = first ? zr : __fma_rn(-beta, pr, zr);
     scal[0] = pap;
     scal[1] = beta;
     scal[2] = pap > 0.0 ? prn / pap : 0.0;
@@ -209,109 +224,14 @@ struct Halo {
 // registers (about 7 global loads per node instead of 23 with every neighbour
 // formed from memory).  Nodes outside the domain hold 0 and
 // the neighbour sum adds x-, x+, y-, y+, z-, z+ in that order.
-template <int TZC>
-__device__ __forceinline__ void update_residual_body(const float* __restrict__ z, Pad g, float* p0, float* p1,
-                                                     double* x0, double* x1, const double* __restrict__ b,
-                                                     const double* __restrict__ screen, double pw,
-                                                     const double* __restrict__ scal, const int* __restrict__ flags,
-                                                     float* __restrict__ r32, double* __restrict__ part, int tz,
-                                                     int tile_x, int tile_y, int tile_z, int64_t block) {
-    __shared__ double tiles[2][kUY + 2][kUX + 2];  // by plane parity: one barrier per plane
-    __shared__ double shared[1][32];
-    const int n = g.n;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kUX + tx;
-    const int bx = tile_x * kUX, by = tile_y * kUY;
-    const int x = bx + tx, y = by + ty;
-    const int tzv = TZC > 0 ? TZC : tz;
-    const int z0 = tile_z * tzv, z1 = min(n, z0 + tzv);
-    const double h = (double)(n - 1), h2 = h * h;
-    const int odd = flags[1] & 1;
-    const bool first = flags[0] != 0;
-    const float* __restrict__ pp = odd ? p1 : p0;
-    float* __restrict__ pn = odd ? p0 : p1;
-    const double* __restrict__ xc = odd ? x1 : x0;
-    double* __restrict__ xn = odd ? x0 : x1;
-    const double beta = first ? 0.0 : scal[1], alpha = scal[2];
-    const int64_t nn = (int64_t)n * n;
-    auto dir_at = [&](int64_t ii, int64_t cc) -> double {
-        double val = (double)z[cc];
-        if (!first) val -= beta * (double)pp[ii];
-        return val;
-    };
-    const Halo hl(tid, bx, by);
-    const bool halo_in = hl.inside(n);
-    int64_t hi = 0, hc = 0;
-    if (halo_in) {
-        hi = (int64_t)z0 * nn + (int64_t)hl.hy * n + hl.hx;
-        hc = g.at(hl.hx, hl.hy, z0);
-    }
-    const bool inside = x < n && y < n;
-    int64_t i = 0, c = 0;
-    double dm = 0.0, xm = 0.0, xb = 0.0;
-    if (inside) {
-        i = (int64_t)z0 * nn + (int64_t)y * n + x;
-        c = g.at(x, y, z0);
-        dm = dir_at(i, c);
-        xm = xc[i] + alpha * dm;
-        xb = z0 > 0 ? xc[i - nn] + alpha * dir_at(i - nn, c - g.plane) : 0.0;
-    }
-    const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
-    double v[1] = {0.0};
-    for (int k = z0; k < z1; ++k) {
-        const double hv = halo_in ? xc[hi] + alpha * dir_at(hi, hc) : 0.0;
-        const bool up = k + 1 < n;
-        double da = 0.0, xa = 0.0, bi = 0.0, sc = 0.0;
-        if (inside) {
-            if (up) {
-                da = dir_at(i + nn, c + g.plane);
-                xa = xc[i + nn] + alpha * da;
-            }
-            bi = b[i];
-            sc = screen[i];
-        }
-        // plane k - 2's reads of this tile ended before plane k - 1's barrier
-        double(*tile)[kUX + 2] = tiles[k & 1];
-        tile[ty + 1][tx + 1] = inside ? xm : 0.0;
-        if (hl.has) tile[hl.sy][hl.sx] = hv;
-        __syncthreads();
-        if (inside) {
-            double s = 0.0;
-            s += tile[ty + 1][tx];
-            s += tile[ty + 1][tx + 2];
-            s += tile[ty][tx + 1];
-            s += tile[ty + 2][tx + 1];
-            s += xb;
-            s += xa;
-            const int deg = degxy + (k > 0) + up;
-            PB_GUARD(i, nn * n, kSiteFcgStore) {
-                pn[i] = (float)dm;
-                xn[i] = xm;
-            }
-            const double r = bi - (((double)deg * h2 + pw * sc * h2) * xm - s * h2);
-            PB_GUARD(c, (int64_t)(n + 2) * g.plane, kSiteFcgStore)
-            r32[c] = (float)r;
-            v[0] += r * r;
-            i += nn;
-            c += g.plane;
-        }
-        xb = xm;
-        xm = xa;
-        dm = da;
-        hi += nn;
-        hc += g.plane;
-    }
-    block_sums<1>(v, shared);
-    if (lin_tid() == 0) part[block] = v[0];
-}
-
-// ---- pass 2 with the next planes prefetched by cp.async -------------------------
-// The same arithmetic as update_residual_body, in the same order.  Each
-// thread copies the values it will read of plane k + RING - 1 (its x, z, p, b
-// and screen, and its halo node's x, z, p) into its own shared-memory slots
-// with cp.async while it works on plane k, so RING - 1 planes of loads are in
-// flight per thread without holding registers; a thread only reads its own
-// slots, so cp.async.wait_group suffices (the tile of new iterates keeps its
-// barrier).  RING = 3 by default, 4 as a tuning variant.
+//
+// Each thread copies the values it will read of plane k + RING - 1 (its x, z, p, b
+// and screen, and its halo node's x, z, p) into its own shared-memory slots with
+// cp.async while it works on plane k, so RING - 1 planes of loads are in flight per
+// thread without holding registers (257^3: 168 us against 237 with the loads in
+// registers); a thread only reads its own slots, so cp.async.wait_group suffices
+// (the tile of new iterates keeps its barrier).  RING = 3 by default, 4 as a tuning
+// variant.
 constexpr int kRing = 3;
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
@@ -358,12 +278,12 @@ __device__ __forceinline__ void update_residual_prefetch_body(
     const int64_t nn = (int64_t)n * n;
     auto dir_at = [&](int64_t ii, int64_t cc) -> double {
         double val = (double)z[cc];
-        if (!first) val -= beta * (double)pp[ii];
+        if (!first) val = __fma_rn(-beta, (double)pp[ii], val);
         return val;
     };
     auto dir_of = [&](float zv, float pv) -> double {  // dir_at from prefetched values
         double val = (double)zv;
-        if (!first) val -= beta * (double)pv;
+        if (!first) val = __fma_rn(-beta, (double)pv, val);
         return val;
     };
     const Halo hl(tid, bx, by);
@@ -402,8 +322,8 @@ __device__ __forceinline__ void update_residual_prefetch_body(
     if (inside) {
         const int sl = z0 % RING;
         dm = dir_of(rf[sl][0][tid], rf[sl][1][tid]);
-        xm = rd[sl][0][tid] + alpha * dm;
-        xb = z0 > 0 ? xc[i0 - nn] + alpha * dir_at(i0 - nn, c0 - g.plane) : 0.0;
+        xm = __fma_rn(alpha, dm, rd[sl][0][tid]);
+        xb = z0 > 0 ? __fma_rn(alpha, dir_at(i0 - nn, c0 - g.plane), xc[i0 - nn]) : 0.0;
     }
     int64_t i = i0, c = c0;
     const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
@@ -412,13 +332,13 @@ __device__ __forceinline__ void update_residual_prefetch_body(
         issue(k + RING - 1);  // into the slot of plane k - 1, read by this thread alone in the previous step
         cp_wait<RING - 2>();  // planes up to k + 1 have landed
         const int sk = k % RING, sn = (k + 1) % RING;
-        const double hv = halo_in ? hd[sk][tid] + alpha * dir_of(hf[sk][0][tid], hf[sk][1][tid]) : 0.0;
+        const double hv = halo_in ? __fma_rn(alpha, dir_of(hf[sk][0][tid], hf[sk][1][tid]), hd[sk][tid]) : 0.0;
         const bool up = k + 1 < n;
         double da = 0.0, xa = 0.0, bi = 0.0, sc = 0.0;
         if (inside) {
             if (up) {
                 da = dir_of(rf[sn][0][tid], rf[sn][1][tid]);
-                xa = rd[sn][0][tid] + alpha * da;
+                xa = __fma_rn(alpha, da, rd[sn][0][tid]);
             }
             bi = rd[sk][1][tid];
             sc = rd[sk][2][tid];
@@ -440,10 +360,10 @@ __device__ __forceinline__ void update_residual_prefetch_body(
                 pn[i] = (float)dm;
                 xn[i] = xm;
             }
-            const double r = bi - (((double)deg * h2 + pw * sc * h2) * xm - s * h2);
+            const double r = __dsub_rn(bi, applied(deg, pw, sc, h2, xm, s));
             PB_GUARD(c, (int64_t)(n + 2) * g.plane, kSiteFcgStore)
             r32[c] = (float)r;
-            v[0] += r * r;
+            v[0] = __fma_rn(r, r, v[0]);
             i += nn;
             c += g.plane;
         }
@@ -463,16 +383,6 @@ __global__ void __launch_bounds__(kUThreads) update_residual_prefetch_kernel(
     float* __restrict__ r32, double* __restrict__ part, int tz) {
     update_residual_prefetch_body<TZC, RING>(z, g, p0, p1, x0, x1, b, screen, pw, scal, flags, r32, part, tz,
                                              blockIdx.x, blockIdx.y, blockIdx.z, block_index());
-}
-
-// MINB as above (PB_TUNE_FCG_UPDATE_VARIANT; the default 5 matches a 48-register budget).
-template <int MINB, int TZC>
-__global__ void __launch_bounds__(kUThreads, MINB) update_residual_kernel(
-    const float* __restrict__ z, Pad g, float* p0, float* p1, double* x0, double* x1, const double* __restrict__ b,
-    const double* __restrict__ screen, double pw, const double* __restrict__ scal, const int* __restrict__ flags,
-    float* __restrict__ r32, double* __restrict__ part, int tz) {
-    update_residual_body<TZC>(z, g, p0, p1, x0, x1, b, screen, pw, scal, flags, r32, part, tz, blockIdx.x, blockIdx.y,
-                         blockIdx.z, block_index());
 }
 
 // out[0] = sum over blocks of part[b] (fixed order).
@@ -506,11 +416,11 @@ __global__ void loop_kernel(cudaGraphConditionalHandle handle, int use_handle, c
 }
 
 static int direction_planes(int n) {
-    const int64_t tz = tuned(PB_TUNE_FCG_DIRECTION_PLANES, n, kTZ);
+    const int64_t tz = tuned(PB_TUNE_FCG_DIRECTION_PLANES, n, planes_of(n));
     return tz < kMinTZ ? kMinTZ : (int)tz;
 }
 static int update_planes(int n) {
-    const int64_t tz = tuned(PB_TUNE_FCG_UPDATE_PLANES, n, kTZ);
+    const int64_t tz = tuned(PB_TUNE_FCG_UPDATE_PLANES, n, planes_of(n));
     return tz < kMinTZ ? kMinTZ : (int)tz;
 }
 static dim3 flat_grid_of(int n, int tz) { return dim3((n * n + kThreads - 1) / kThreads, (n + tz - 1) / tz); }
@@ -539,10 +449,14 @@ __global__ void __launch_bounds__(kThreads, 4) direction_sums_grouped_kernel(con
     int bx, by, bz;
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
-    direction_sums_body<kTZ>((const float*)d.ptr[0], pad_of((int)d.n), (const float*)d.ptr[1], (const float*)d.ptr[2],
-                        (const float*)d.ptr[3], (const double*)d.ptr[4], aux_double(d.aux[0]),
-                        flags + d.cloud * batch::kFlagStride, (double*)d.ptr[5], (int)d.aux[1], bx, by,
-                        bx + d.gx * (int64_t)by);
+    auto run = [&](auto planes) {  // the same instantiation as the single launch of that side
+        direction_sums_body<decltype(planes)::value>(
+            (const float*)d.ptr[0], pad_of((int)d.n), (const float*)d.ptr[1], (const float*)d.ptr[2],
+            (const float*)d.ptr[3], (const double*)d.ptr[4], aux_double(d.aux[0]),
+            flags + d.cloud * batch::kFlagStride, (double*)d.ptr[5], (int)d.aux[1], bx, by, bx + d.gx * (int64_t)by);
+    };
+    if (d.aux[1] == kTZ) run(std::integral_constant<int, kTZ>());
+    else run(std::integral_constant<int, 0>());
 }
 
 // One block per cloud: ptr[0] partials, ptr[1] the cloud's scalars; aux[0] pass-1 blocks.
@@ -562,7 +476,7 @@ __global__ void __launch_bounds__(kUThreads, 4) update_residual_grouped_kernel(c
     int bx, by, bz;
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
-    update_residual_prefetch_body<kTZ>((const float*)d.ptr[0], pad_of((int)d.n), (float*)d.ptr[1], (float*)d.ptr[2],
+    update_residual_prefetch_body<0>((const float*)d.ptr[0], pad_of((int)d.n), (float*)d.ptr[1], (float*)d.ptr[2],
                          (double*)d.ptr[3], (double*)d.ptr[4], (const double*)d.ptr[5], (const double*)d.ptr[6],
                          aux_double(d.aux[0]), (const double*)d.ptr[8], flags + d.cloud * batch::kFlagStride,
                          (float*)d.ptr[7], (double*)d.ptr[9], (int)d.aux[1], bx, by, bz,
@@ -613,7 +527,7 @@ int describe_fcg_direction(GridDesc& d) {
     for (int k = 0; k < 6; ++k)
         if (!d.ptr[k]) return fail(PB_ERR_INVALID, "batch fcg direction: bad args");
     if (n < 2 || n > 4097 || d.ptr[1] == d.ptr[2]) return fail(PB_ERR_INVALID, "batch fcg direction: bad args");
-    const int tz = fcg::kTZ;  // grouped launches keep the built-in planes per block
+    const int tz = fcg::planes_of(n);  // grouped launches keep the built-in planes per block
     const dim3 g = fcg::flat_grid_of(n, tz);
     d.gx = g.x;
     d.gy = g.y;
@@ -628,7 +542,7 @@ int describe_fcg_update(GridDesc& d) {
         if (!d.ptr[k]) return fail(PB_ERR_INVALID, "batch fcg update: bad args");
     if (n < 2 || n > 4097 || d.ptr[1] == d.ptr[2] || d.ptr[3] == d.ptr[4])
         return fail(PB_ERR_INVALID, "batch fcg update: bad args");
-    const int tz = fcg::kTZ;
+    const int tz = fcg::planes_of(n);
     const dim3 g = fcg::tile_grid_of(n, tz);
     d.gx = g.x;
     d.gy = g.y;
@@ -645,8 +559,8 @@ int describe_fcg_reduce(GridDesc& d) {
 
 // Partial-sum doubles one cloud of side n needs (both FCG passes).
 int64_t fcg_partials(int n) { return (int64_t)fcg::blocks_of(n) * 4; }
-int64_t fcg_direction_blocks(int n) { return fcg::count(fcg::flat_grid_of(n, fcg::kTZ)); }
-int64_t fcg_update_blocks(int n) { return fcg::count(fcg::tile_grid_of(n, fcg::kTZ)); }
+int64_t fcg_direction_blocks(int n) { return fcg::count(fcg::flat_grid_of(n, fcg::planes_of(n))); }
+int64_t fcg_update_blocks(int n) { return fcg::count(fcg::tile_grid_of(n, fcg::planes_of(n))); }
 
 int launch_fcg(int kind, const GridDesc* descs, int count, int64_t blocks, const int* flags, cudaStream_t s) {
     switch (kind) {
@@ -740,17 +654,12 @@ extern "C" int pb_fcg_update_f64(const float* z, float* p0, float* p1, double* x
     const int tz = update_planes((int)n);
     const dim3 grid = tile_grid_of((int)n, tz);
     const bool fixed = tz == kTZ;
-    auto upd = fixed ? update_residual_kernel<5, kTZ> : update_residual_kernel<5, 0>;
-    switch (tuned(PB_TUNE_FCG_UPDATE_VARIANT, n, 0)) {
-        case 1: upd = fixed ? update_residual_kernel<6, kTZ> : update_residual_kernel<6, 0>; break;
-        case 2: upd = fixed ? update_residual_kernel<8, kTZ> : update_residual_kernel<8, 0>; break;
-        case 3: upd = fixed ? update_residual_prefetch_kernel<kTZ> : update_residual_prefetch_kernel<0>; break;
-        case 4: upd = fixed ? update_residual_prefetch_kernel<kTZ, 4> : update_residual_prefetch_kernel<0, 4>; break;
-        default: break;
-    }
+    auto upd = fixed ? update_residual_prefetch_kernel<kTZ> : update_residual_prefetch_kernel<0>;
+    if (tuned(PB_TUNE_FCG_UPDATE_VARIANT, n, 0) == 4)
+        upd = fixed ? update_residual_prefetch_kernel<kTZ, 4> : update_residual_prefetch_kernel<0, 4>;
     upd<<<grid, dim3(kUX, kUY), 0, s>>>(z, pad_of((int)n), p0, p1, x0, x1, b, screen, point_weight, scal, flags,
                                         r32, part, tz);
-    PB_CHECK_LAUNCH("fcg update_residual_kernel");
+    PB_CHECK_LAUNCH("fcg update_residual_prefetch_kernel");
     sum_kernel<<<1, 1024, 0, s>>>(part, (int)count(grid), scal + 4);
     PB_CHECK_LAUNCH("fcg sum_kernel");
     return PB_OK;

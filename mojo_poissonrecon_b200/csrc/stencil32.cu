@@ -109,6 +109,83 @@ __global__ void sum_partials_kernel(const double* __restrict__ partial, int coun
     if (threadIdx.x == 0) *out = t;
 }
 
+// ---- the start of a refined solve in one pass --------------------------------------
+// From the dense right-hand side and screen: level 0's D, 1/D and weights
+// (level_setup_kernel's expressions), x0 = 1/2 (core.py:270) and its residual,
+// ||r||^2 and ||b||^2; optionally copies of both in buffers of the solver's own (a
+// captured iteration needs fixed pointers).  With x0 constant the neighbour sum is
+// degree / 2, exactly, so no neighbour is read.  Threads flattened over a plane's
+// (x, y), a few planes each.  Bound by memory: 16 bytes read and 24 (40 with the
+// copies) written per node, against 108 of the two dense copies, level set-up, fill,
+// defect and norm that it replaces (257^3: 390 -> 221 us).
+constexpr int kStartZ = 8;
+
+__global__ void __launch_bounds__(256) refine_start_kernel(const double* __restrict__ rhs,
+                                                           const double* __restrict__ screen, Geom g, double pw,
+                                                           double* __restrict__ rhs_copy,
+                                                           double* __restrict__ screen_copy, double* __restrict__ x0,
+                                                           float* __restrict__ D, float* __restrict__ invD,
+                                                           float* __restrict__ weights, float* __restrict__ r32,
+                                                           double* __restrict__ partial) {
+    __shared__ double shared[2][32];
+    const int n = g.n;
+    const unsigned t = blockIdx.x * 256u + threadIdx.x;
+    const int z0 = blockIdx.y * kStartZ, z1 = min(n, z0 + kStartZ);
+    const double h = (double)(n - 1), h2 = h * h;
+    double rr = 0.0, bb = 0.0;
+    if (t < (unsigned)(n * n)) {
+        const int y = (int)(t / (unsigned)n), x = (int)(t - (unsigned)y * n);
+        const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
+        const int64_t nn = (int64_t)n * n;
+        int64_t i = z0 * nn + t, p = g.at(x, y, z0);
+        const float inv6 = (float)(1.0 / (6.0 * h2));
+#pragma unroll 4
+        for (int z = z0; z < z1; ++z, i += nn, p += g.plane) {
+            const double b = rhs[i], sc = screen[i];
+            if (rhs_copy) rhs_copy[i] = b;
+            if (screen_copy) screen_copy[i] = sc;
+            x0[i] = 0.5;
+            const int deg = degxy + (z > 0) + (z + 1 < n);
+            const double d = (double)deg * h2 + pw * sc * h2;
+            D[p] = (float)d;
+            // without screening the diagonal is degree h^-2: the weight is 1, and 1/D the same at every interior node
+            const bool plain = sc == 0.0;
+            invD[p] = plain && deg == 6 ? inv6 : (float)(1.0 / d);
+            weights[p] = !plain && ((x | y | z) & 1) ? (float)((double)deg * h2 / d) : 1.0f;
+            const double r = b - (d * 0.5 - (double)deg * 0.5 * h2);
+            r32[p] = (float)r;
+            rr += r * r;
+            bb += b * b;
+        }
+    }
+    rr = warp_block_sum(rr, shared[0]);
+    bb = warp_block_sum(bb, shared[1]);
+    if (threadIdx.x == 0) {
+        double* out = partial + 2 * ((int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+        out[0] = rr;
+        out[1] = bb;
+    }
+}
+
+// norm2 = ||r||^2, bnorm = ||b||, from the blocks' sums in a fixed order.
+__global__ void __launch_bounds__(1024) refine_start_finish_kernel(const double* __restrict__ partial, int count,
+                                                                   double* __restrict__ norm2,
+                                                                   double* __restrict__ bnorm) {
+    __shared__ double shared[2][32];
+    double rr = 0.0, bb = 0.0;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        rr += partial[2 * i];
+        bb += partial[2 * i + 1];
+    }
+    const double r = warp_block_sum(rr, shared[0]), b = warp_block_sum(bb, shared[1]);
+    if (threadIdx.x == 0) {
+        *norm2 = r;
+        *bnorm = sqrt(b);
+    }
+}
+
+static dim3 refine_start_grid(int n) { return dim3((n * n + 255) / 256, (n + kStartZ - 1) / kStartZ); }
+
 // ---- level-0 residual fused with the scaled restriction -------------------------
 // coarse_rhs = P^T (s (rhs - A e)) / 8 (mg27.cu) without writing the fine
 // residual.  A block owns a 64 x 4 tile of coarse (x, y) and marches coarse z.
@@ -126,12 +203,11 @@ constexpr int kRrFX = 2 * kRrCX + 8, kRrFY = 2 * kRrCY + 1;  // 136 x 9 fine nod
 constexpr int kRrGroups = kRrFX / 4;                            // float4 groups per ring row
 constexpr int kRrThreads = 256;
 
-// PAIRED: the two fine planes of a coarse plane are computed in one loop over
-// their 612 float4 items (three rounds of 256 threads instead of two rounds per
-// plane, 80 % of the lanes busy instead of 60 %); each item's arithmetic is the
-// same, so the results are too.  THREADS = 320 (tuning variant 3, paired):
-// the 612 items in two rounds (96 % busy); the first 256 threads restrict.
-template <bool PAIRED, int THREADS = kRrThreads>
+// The two fine planes of a coarse plane are computed in one loop over their 612
+// float4 items (three rounds of 256 threads instead of two rounds per plane, 80 %
+// of the lanes busy instead of 60 %: 98 -> 83 us at 257^3).  THREADS = 320 (tuning
+// variant 3): the 612 items in two rounds (96 % busy); the first 256 threads restrict.
+template <int THREADS = kRrThreads>
 __device__ __forceinline__ void residual_restrict32_body(const float* __restrict__ e, const float* __restrict__ rhs,
                                                          const float* __restrict__ D, const float* __restrict__ w,
                                                          Geom gf, float h2, float* __restrict__ coarse, Geom gc,
@@ -173,19 +249,11 @@ __device__ __forceinline__ void residual_restrict32_body(const float* __restrict
             *reinterpret_cast<float4*>(&dst[ly][4 * g]) = r;
         }
     };
-    auto fine_plane = [&](int f) {
-        for (int i = tid; i < kItems; i += THREADS) fine_item(f, i);
-    };
-    fine_plane(2 * zc0 - 1);
+    for (int i = tid; i < kItems; i += THREADS) fine_item(2 * zc0 - 1, i);
     for (int zc = zc0; zc < zc1; ++zc) {
-        if (PAIRED) {
-            for (int j = tid; j < 2 * kItems; j += THREADS) {
-                const int second = j >= kItems;
-                fine_item(2 * zc + second, j - second * kItems);
-            }
-        } else {
-            fine_plane(2 * zc);
-            fine_plane(2 * zc + 1);
+        for (int j = tid; j < 2 * kItems; j += THREADS) {
+            const int second = j >= kItems;
+            fine_item(2 * zc + second, j - second * kItems);
         }
         __syncthreads();
         {
@@ -219,25 +287,16 @@ __global__ void __launch_bounds__(kRrThreads) residual_restrict32_kernel(const f
                                                                           const float* __restrict__ w, Geom gf,
                                                                           float h2, float* __restrict__ coarse,
                                                                           Geom gc, int cz) {
-    residual_restrict32_body<false>(e, rhs, D, w, gf, h2, coarse, gc, cz, blockIdx.x, blockIdx.y, blockIdx.z);
+    residual_restrict32_body<>(e, rhs, D, w, gf, h2, coarse, gc, cz, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-__global__ void __launch_bounds__(kRrThreads) residual_restrict32_paired_kernel(const float* __restrict__ e,
-                                                                                 const float* __restrict__ rhs,
-                                                                                 const float* __restrict__ D,
-                                                                                 const float* __restrict__ w, Geom gf,
-                                                                                 float h2, float* __restrict__ coarse,
-                                                                                 Geom gc, int cz) {
-    residual_restrict32_body<true>(e, rhs, D, w, gf, h2, coarse, gc, cz, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-__global__ void __launch_bounds__(320) residual_restrict32_paired320_kernel(const float* __restrict__ e,
+__global__ void __launch_bounds__(320) residual_restrict32_wide_kernel(const float* __restrict__ e,
                                                                           const float* __restrict__ rhs,
                                                                           const float* __restrict__ D,
                                                                           const float* __restrict__ w, Geom gf,
                                                                           float h2, float* __restrict__ coarse,
                                                                           Geom gc, int cz) {
-    residual_restrict32_body<true, 320>(e, rhs, D, w, gf, h2, coarse, gc, cz, blockIdx.x, blockIdx.y, blockIdx.z);
+    residual_restrict32_body<320>(e, rhs, D, w, gf, h2, coarse, gc, cz, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // Grouped (batch.cuh): ptr[0] e, ptr[1] rhs, ptr[2] D, ptr[3] weights, ptr[4] coarse rhs.
@@ -247,7 +306,7 @@ __global__ void __launch_bounds__(kRrThreads) residual_restrict32_grouped_kernel
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
     const int n = (int)d.n;
-    residual_restrict32_body<false>((const float*)d.ptr[0], (const float*)d.ptr[1], (const float*)d.ptr[2],
+    residual_restrict32_body<>((const float*)d.ptr[0], (const float*)d.ptr[1], (const float*)d.ptr[2],
                              (const float*)d.ptr[3], geom(n), (float)((n - 1) * (n - 1)), (float*)d.ptr[4],
                              geom((n + 1) / 2), (int)d.aux[0], bx, by, bz);
 }
@@ -280,6 +339,33 @@ extern "C" int pb_level_setup_f32(const double* screen, int64_t n, double point_
     level_setup_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(screen, geom((int)n), point_weight, D, invD,
                                                                  weights);
     PB_CHECK_LAUNCH("level_setup_kernel");
+    return PB_OK;
+}
+
+extern "C" size_t pb_refine_start_workspace_size(int64_t n) {
+    const dim3 g = refine_start_grid((int)(n < 2 ? 2 : n > 4097 ? 4097 : n));
+    return (size_t)g.x * g.y * 2 * sizeof(double) + 256;
+}
+
+// The start of a refined solve (refine_start_kernel).  rhs_copy, screen_copy (either
+// may be null) and x0: dense FP64; the rest padded FP32 (ghosts untouched);
+// *norm2 = ||r||^2, *bnorm = ||b||.
+extern "C" int pb_refine_start_f64(const double* rhs, const double* screen, int64_t n, double point_weight,
+                                   double* rhs_copy, double* screen_copy, double* x0, float* D, float* invD,
+                                   float* weights, float* r32, double* norm2, double* bnorm, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+    if (n < 2 || n > 4097 || !rhs || !screen || !x0 || !D || !invD || !weights || !r32 || !norm2 || !bnorm)
+        return fail(PB_ERR_INVALID, "refine start: bad args");
+    const dim3 grid = refine_start_grid((int)n);
+    const int blocks = (int)(grid.x * grid.y);
+    if (!workspace || workspace_bytes < (size_t)blocks * 2 * sizeof(double))
+        return fail(PB_ERR_WORKSPACE, "refine start: workspace needs %zu bytes", pb_refine_start_workspace_size(n));
+    cudaStream_t s = (cudaStream_t)stream;
+    refine_start_kernel<<<grid, 256, 0, s>>>(rhs, screen, geom((int)n), point_weight, rhs_copy, screen_copy, x0,
+                                             D, invD, weights, r32, (double*)workspace);
+    PB_CHECK_LAUNCH("refine_start_kernel");
+    refine_start_finish_kernel<<<1, 1024, 0, s>>>((const double*)workspace, blocks, norm2, bnorm);
+    PB_CHECK_LAUNCH("refine_start_finish_kernel");
     return PB_OK;
 }
 
@@ -318,9 +404,7 @@ extern "C" int pb_residual_restrict_f32(const float* e, const float* rhs, const 
     const int cz = (int)tuned(PB_TUNE_RESTRICT_PLANES, n, kRrCZ);
     const dim3 grid((cn + kRrCX - 1) / kRrCX, (cn + kRrCY - 1) / kRrCY, (cn + cz - 1) / cz);
     const int64_t variant = tuned(PB_TUNE_RESTRICT_VARIANT, n, 0);
-    auto kernel = variant == 1 ? residual_restrict32_paired_kernel
-                  : variant == 3 ? residual_restrict32_paired320_kernel
-                                 : residual_restrict32_kernel;
+    auto kernel = variant == 3 ? residual_restrict32_wide_kernel : residual_restrict32_kernel;
     kernel<<<grid, variant == 3 ? 320 : kRrThreads, 0, (cudaStream_t)stream>>>(e, rhs, D, weights, geom((int)n), h2,
                                                                                coarse_rhs, geom(cn), cz);
     PB_CHECK_LAUNCH("residual_restrict32_kernel");

@@ -14,8 +14,9 @@ flexible conjugate gradients:
 One iteration touches the same buffers every time, so the engine captures it
 once as the body of a CUDA graph WHILE node whose condition a device kernel
 sets from ||r||^2 (pb_loop_condition); a solve is then one graph launch with
-no host synchronisation per iteration.  The prologue (level set-up, x0 and its
-residual, ||b||) is captured once as a second graph.  Engines (hierarchy,
+no host synchronisation per iteration.  A solve starts with one pass over the
+right-hand side and screen (pb_refine_start_f64); the coarse levels' set-up is
+captured once as a second graph.  Engines (hierarchy,
 vectors, graphs) are cached per device, grid side, point weight and slot and
 reused across solves.
 
@@ -193,9 +194,9 @@ class Hierarchy32:
         return sum(t.numel() * t.element_size() for lv in self.levels for t in lv.tensors()) + \
             self.inverse.numel() * 8 + self.image.numel() * 4 + self.galerkin_ws.numel() * 4
 
-    def setup(self, screen: torch.Tensor, point_weight: float) -> None:
-        """Level 0 from the FP64 screen (D = (deg + pw*screen) h^-2, core.py:150-163),
-        then each coarser level's Galerkin operator from the one above it, the
+    def setup(self, screen: torch.Tensor | None, point_weight: float) -> None:
+        """Level 0 from the FP64 screen (D = (deg + pw*screen) h^-2, core.py:150-163;
+        None: `start` has set it up), then each coarser level's Galerkin operator from the one above it, the
         packed forms, the 3^3 inverse and the coarse image: one library call
         (pb_hierarchy_setup_f32)."""
         self.pw = float(point_weight)
@@ -209,7 +210,8 @@ class Hierarchy32:
             for k, t in enumerate(row):
                 arrays[i * A + k] = None if t is None else t.data_ptr()
         sides = (ctypes.c_int64 * K)(*[lv.n for lv in self.levels])
-        nat.check(self.lib.pb_hierarchy_setup_f32(K, sides, arrays, self.first_coarse, screen.data_ptr(), self.pw,
+        nat.check(self.lib.pb_hierarchy_setup_f32(K, sides, arrays, self.first_coarse,
+                                                  None if screen is None else screen.data_ptr(), self.pw,
                                                   self.galerkin_ws.data_ptr(), self.galerkin_ws.numel() * 4,
                                                   self.inverse.data_ptr(), self.image.data_ptr(),
                                                   self.image.numel() * 4, self.stream), "hierarchy setup")
@@ -217,6 +219,17 @@ class Hierarchy32:
             for lv in self.levels:
                 if lv.packed is not None:
                     lv.coef = None  # freed once this stream's set-up has run (stream-ordered allocator)
+
+    def start(self, rhs: torch.Tensor, screen: torch.Tensor, point_weight: float, copies, x0, norm2, bnorm,
+              workspace: nat.Workspace) -> None:
+        """Level 0 and everything else a refined solve starts with, in one pass
+        (pb_refine_start_f64); copies: buffers for rhs and screen, or (None, None)."""
+        L, lv = self.lib, self.levels[0]
+        ptr, size = workspace.get(L.pb_refine_start_workspace_size(lv.n))
+        nat.check(L.pb_refine_start_f64(rhs.data_ptr(), screen.data_ptr(), lv.n, float(point_weight),
+                                        *(None if t is None else t.data_ptr() for t in copies), x0.data_ptr(),
+                                        lv.D.data_ptr(), lv.invD.data_ptr(), lv.weights.data_ptr(), lv.rhs.data_ptr(),
+                                        norm2.data_ptr(), bnorm.data_ptr(), ptr, size, self.stream), "refine start")
 
     def _sweep(self, lv: Level32, src, dst, mode: int, coarse=None) -> None:
         """One red-black sweep dst <- S(src); mode 1 starts from zero, mode 2
@@ -350,10 +363,8 @@ class RefinedEngine:
         self.norm2 = torch.empty(1, dtype=torch.float64, device=device)
         self.bnorm = torch.empty(1, dtype=torch.float64, device=device)
         self.ws = nat.Workspace(device)
-        self.ws_ptr, self.ws_size = self.ws.get(max(self.lib.pb_defect_workspace_size(n),
+        self.ws_ptr, self.ws_size = self.ws.get(max(self.lib.pb_refine_start_workspace_size(n),
                                                     self.lib.pb_fcg_workspace_size(n)))
-        self.norm_ws = nat.Workspace(device)
-        self.norm_ws.get(1 << 16)
         self.graph = ctypes.c_void_p()
         self.exec = ctypes.c_void_p()
         self.setup_graph = None
@@ -422,17 +433,14 @@ class RefinedEngine:
         nat.check(L.pb_loop_capture_end(s, self.graph, ctypes.byref(self.exec)), "loop capture end")
         self.body_launches = L.pb_launch_count() - before
 
-    def _start(self) -> None:
-        """x[0] = 0.5, r = b - A x (its FP32 copy for the first V-cycle), ||r||^2;
-        iteration counter and first-step flag reset."""
-        L, s = self.lib, nat.stream_handle()
-        x0 = self.xs[0]
-        nat.check(L.pb_fill_f64(x0.data_ptr(), x0.numel(), 0.5, s), "fill")  # core.py:270
-        nat.check(L.pb_defect_f64(x0.data_ptr(), None, None, self.b.data_ptr(), self.screen.data_ptr(), self.n,
-                                  self.pw, self.h.levels[0].rhs.data_ptr(), None, self.norm2.data_ptr(),
-                                  self.ws_ptr, self.ws_size, s), "defect")
+    def _start(self, rhs: torch.Tensor, screen: torch.Tensor) -> None:
+        """Level 0, x[0] = 0.5 and its residual (FP32, for the first V-cycle), ||r||^2,
+        ||b||; iteration counter and first-step flag reset.  Engines that are not
+        lean copy rhs and screen: their graph reads them there."""
+        copies = (None, None) if self.lean else (self.b, self.screen)
+        self.h.start(rhs, screen, self.pw, copies, self.xs[0], self.norm2, self.bnorm, self.ws)
         self.flags.zero_()
-        self.flags[0:1].fill_(1)  # a device fill, no host copy (capturable)
+        self.flags[0:1].fill_(1)
 
     def solve(self, rhs: torch.Tensor, screen: torch.Tensor, tol: float,
               max_cycles: int) -> tuple[torch.Tensor, SolveStats]:
@@ -452,31 +460,24 @@ class RefinedEngine:
             x.record_stream(caller)  # allocated on the engine's stream, used on the caller's from here
         return x, stats
 
-    def _prologue(self) -> None:
-        """The per-solve work before the iterations, on the engine's own buffers:
-        the levels' set-up (D, Galerkin products, packing, coarse image), x0 and
-        its residual, ||b||."""
-        self.h.setup(self.screen, self.pw)
-        self._start()
-        norm(self.b, self.norm_ws, self.bnorm)
-
-    def _run_prologue(self) -> None:
-        """The prologue as one graph launch: its ~45 launches touch the same
-        pointers on every solve, so they are captured once per engine (after one
-        eager run that sets kernel attributes and loads the modules) and
-        replayed, which takes their host launch cost off small solves.  Lean
-        engines run it eagerly (their pointers change per solve)."""
+    def _run_setup(self) -> None:
+        """The coarse levels' set-up (Galerkin products, packing, coarse image) as
+        one graph launch: its ~35 launches touch the same pointers on every solve,
+        so they are captured once per engine (after one eager run that sets kernel
+        attributes and loads the modules) and replayed, which takes their host
+        launch cost off small solves.  Lean engines run it eagerly (their pointers
+        change per solve)."""
         if not SETUP_GRAPH or EAGER_LOOP or self.lean:
-            self._prologue()
+            self.h.setup(None, self.pw)
             return
         if self.setup_graph is None:
-            self._prologue()
+            self.h.setup(None, self.pw)
             g = torch.cuda.CUDAGraph()
             with GRAPH_CAPTURE_LOCK:
                 before = self.lib.pb_launch_count()
                 g.capture_begin(capture_error_mode="thread_local")  # other threads (serving lanes) stay free
                 try:
-                    self._prologue()
+                    self.h.setup(None, self.pw)
                 finally:
                     g.capture_end()
             self.prologue_launches = self.lib.pb_launch_count() - before
@@ -491,11 +492,8 @@ class RefinedEngine:
             self.screen, self.b = screen, rhs
             self._vectors()
             self._drop_graph()
-        else:
-            self.screen.copy_(screen)
-            self.b.copy_(rhs)
         try:
-            x, stats = self._iterate(stats, tol, max_cycles)
+            x, stats = self._iterate(stats, rhs, screen, tol, max_cycles)
         finally:
             if self.lean:  # nothing of this solve stays bound to the engine
                 self.screen = self.b = None
@@ -503,9 +501,10 @@ class RefinedEngine:
                 self._drop_graph()
         return x, stats
 
-    def _iterate(self, stats: SolveStats, tol: float, max_cycles: int):
+    def _iterate(self, stats: SolveStats, rhs: torch.Tensor, screen: torch.Tensor, tol: float, max_cycles: int):
         L, s = self.lib, nat.stream_handle()
-        self._run_prologue()
+        self._start(rhs, screen)
+        self._run_setup()
         _sync.wait("solver prologue")
         both = torch.cat([self.norm2, self.bnorm]).cpu()
         stats.rhs_norm = float(both[1])
@@ -531,7 +530,8 @@ class RefinedEngine:
                         # kernels' modules outside any capture (once per process and
                         # side); its effect is discarded by restarting below
                         self._iteration(0)
-                        self._start()
+                        self._start(rhs, screen)
+                        self._run_setup()  # a 27-point level 0 forms its 1/diagonal and weights there
                         _WARM.add(warm_key)
                     self._capture()
                 nat.check(L.pb_graph_launch(self.exec, s), "graph launch")
