@@ -303,6 +303,10 @@ int pb_note_launches(long long count);
 size_t pb_extract_workspace_size(int64_t n);
 int pb_extract_count_f64(const double *field, int64_t n, const double *iso, int64_t *counts, void *workspace,
                          size_t workspace_bytes, void *stream);
+/* The same, and counts[2] (device int64[3]): 1 if a field value is not finite, plus 2 if a density
+ * value (density may be NULL) is not. */
+int pb_extract_count_checked_f64(const double *field, const double *density, int64_t n, const double *iso,
+                                 int64_t *counts, void *workspace, size_t workspace_bytes, void *stream);
 int pb_extract_emit_f64(const double *field, const double *density, int64_t n, const double *iso, double *vertices,
                         double *vertex_density, int64_t *faces, void *workspace, size_t workspace_bytes,
                         void *stream);

@@ -85,6 +85,7 @@ _SIGNATURES = {
     "pb_mesh_normals_count_f64": ([P, I, P, I, P, P, S, P], C),
     "pb_mesh_normals_emit_f64": ([P, I, P, I, P, P, P, S, P], C),
     "pb_extract_count_f64": ([P, I, P, P, P, S, P], C),
+    "pb_extract_count_checked_f64": ([P, P, I, P, P, P, S, P], C),
     "pb_extract_emit_f64": ([P, P, I, P, P, P, P, P, S, P], C),
     "pb_residual_restrict_f32": ([P, P, P, P, P, I, P], C),
     "pb_residual_restrict_tma_f32": ([P, P, P, P, P, I, P, P], C),

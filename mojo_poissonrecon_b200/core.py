@@ -353,21 +353,37 @@ def solve_screened_poisson(
 EXTRACT_FAST_MAX_SIDE = 1025
 
 
-def _extract_device(ctx: _Context, field: torch.Tensor, density: torch.Tensor, iso: torch.Tensor):
+_FIELD_FINITE = "field and iso_value must be finite"
+_DENSITY_FINITE = "density must be finite"
+
+
+def _extract_device(ctx: _Context, field: torch.Tensor, density: torch.Tensor, iso: torch.Tensor,
+                    check: tuple[bool, bool] = (False, False)):
     """Dual contouring on device tensors; returns (vertices, faces, vdens).
 
     Sides up to 1025 use the bit-array extraction (count, one host read of the
     two counts, emit); larger ones the reference-shaped two-pass entry points.
-    Both give the reference's mesh (capi.mojo:798-1129) bit for bit."""
+    Both give the reference's mesh (capi.mojo:798-1129) bit for bit.
+    check: whether (field, density) may hold values that are not finite, which
+    raises ValueError (sides up to 1025: in the count's own passes)."""
     L = ctx.lib
     n = field.shape[0]
     if n <= EXTRACT_FAST_MAX_SIDE:
         ptr, size = ctx.ws.get(L.pb_extract_workspace_size(n))
-        counts = torch.empty(2, dtype=torch.int64, device=ctx.device)
-        ctx.check(L.pb_extract_count_f64(field.data_ptr(), n, iso.data_ptr(), counts.data_ptr(), ptr, size,
-                                         ctx.stream), "extract count")
+        counts = torch.empty(3, dtype=torch.int64, device=ctx.device)
+        if any(check):
+            ctx.check(L.pb_extract_count_checked_f64(field.data_ptr(), density.data_ptr() if check[1] else None, n,
+                                                     iso.data_ptr(), counts.data_ptr(), ptr, size, ctx.stream),
+                      "extract count")
+        else:
+            ctx.check(L.pb_extract_count_f64(field.data_ptr(), n, iso.data_ptr(), counts.data_ptr(), ptr, size,
+                                             ctx.stream), "extract count")
         _sync.wait("extract count")
-        nv, nf = (int(v) for v in counts.cpu())
+        nv, nf, bad = (int(v) for v in counts.cpu())
+        if check[0] and bad & 1:
+            raise ValueError(_FIELD_FINITE)
+        if check[1] and bad & 2:
+            raise ValueError(_DENSITY_FINITE)
         vertices = torch.empty((nv, 3), dtype=torch.float64, device=ctx.device)
         vdens = torch.empty(nv, dtype=torch.float64, device=ctx.device)
         faces = torch.empty((nf, 3), dtype=torch.int64, device=ctx.device)
@@ -424,19 +440,29 @@ def extract_isosurface(field, *, iso_value: float = 0.0, density=None, device_ou
             return bool(np.isfinite(values).all())
         return bool(torch.isfinite(values).all())
 
-    if not all_finite(field):
-        raise ValueError("field and iso_value must be finite")
+    def deferred(values) -> bool:  # checked by the extraction's own passes
+        return isinstance(values, torch.Tensor) and values.is_cuda and values.shape[0] <= EXTRACT_FAST_MAX_SIDE
+
+    check_field = deferred(field)
     if density is not None:
         density = f64(density)
         if tuple(density.shape) != tuple(field.shape):
+            if not all_finite(field):
+                raise ValueError(_FIELD_FINITE)
             raise ValueError("density must have the same shape as field")
+    check_density = density is not None and check_field and deferred(density)
+    if not check_field and not all_finite(field):
+        raise ValueError(_FIELD_FINITE)
+    if density is not None and not check_density:
+        if check_field and not all_finite(field):
+            raise ValueError(_FIELD_FINITE)
         if not all_finite(density):
-            raise ValueError("density must be finite")
+            raise ValueError(_DENSITY_FINITE)
     ctx = _Context()
     dfield = _to_device(field, ctx.device)
     ddens = torch.zeros_like(dfield) if density is None else _to_device(density, ctx.device)
     iso = torch.full((1,), iso_value, dtype=torch.float64, device=ctx.device)
-    v, f, d = _extract_device(ctx, dfield, ddens, iso)
+    v, f, d = _extract_device(ctx, dfield, ddens, iso, (check_field, check_density))
     return Mesh(*_host_all([v, f, d], device_out), iso_value)
 
 

@@ -8,6 +8,8 @@
 // element i at (tile offset + rank).  Ids, vertex order and face order are
 // therefore identical to the serial reference; vertex coordinates are exact
 // restatements (compiled with -fmad=false).
+#include <algorithm>
+
 #include "scan.cuh"
 
 namespace pb {
@@ -345,260 +347,273 @@ static int dual_faces(const double* field, int64_t n, IsoArg iso, const int64_t*
 
 
 // ---- extraction for reconstruct(): sign bits and rank structures ----------------
-// Same output, order and arithmetic as the two-pass kernels above, but the
-// passes over all cells and edges read a bit per node (field < iso) instead of
-// the FP64 field, and vertex ids are ranks in a bit array of active cells
-// (prefix sum per 32-cell word + popcount) instead of a dense cell map.  Only
-// active cells read field and density values.  Sides up to 1025 (32-bit
-// node, cell and per-sweep edge indices).
+// Same output, order and arithmetic as the two-pass kernels above.  One pass over
+// the field leaves one bit per node (field < iso), rows (y, z) starting on a 32-bit
+// word of their own.  The 32 cells, and the 32 edges of each sweep, that start in a
+// word of row (y, z) then follow from the words of rows (y .. y + 1, z .. z + 1) and
+// the same words shifted by one node, all 32 at once: four words of active cells and
+// sign-changing x-, y- and z-edges per row word, in four segments that a prefix sum
+// of popcounts ranks in the reference's order (word order is z, y, x order).  The
+// emission writes every active item's place into the first slot of its own output,
+// one thread per word, and then runs one thread per vertex and per quad; vertex ids
+// are ranks in the cell words.  Only active cells read field and density values.
+// Sides up to 1025.
+// Against one ballot per 32 cells or edges and one thread per word emitting its
+// items, all kernels together at 230^3 with 677 K vertices: 340 -> 115 us on B200
+// (sign rows 23, words and ranks 12, places 24, vertices 34, quads 23).
 namespace fast {
 
 constexpr int kT = 256;
 constexpr int64_t kMaxSide = 1025;
+constexpr int kTileWords = kScanThreads * kScanItems;  // words per block of the popcount scan
 
-__device__ __forceinline__ uint32_t bit_at(const uint32_t* __restrict__ bits, uint32_t i) {
-    return (bits[i >> 5] >> (i & 31)) & 1u;
-}
 __device__ __forceinline__ uint32_t lanes_below(uint32_t word, uint32_t b) { return __popc(word & ((1u << b) - 1u)); }
 
-// bits: bit b of word w = (field[32w + b] < iso).
-__global__ void __launch_bounds__(kT) sign_bits_kernel(const double* __restrict__ field, uint32_t nodes, IsoArg iso_arg,
-                                                       uint32_t* __restrict__ bits) {
-    const double iso = iso_arg.get();
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < nodes; i += stride) {
-        const uint32_t m = __ballot_sync(0xffffffffu, i < nodes && field[i] < iso);
-        if (lane == 0) bits[i >> 5] = m;
-    }
-}
-
-// active cells (corners on both sides, capi.mojo:946-960) as bits, and the
-// popcount of each 32-cell word (scanned in place into the word's first id).
-__global__ void __launch_bounds__(kT) cell_words_kernel(const uint32_t* __restrict__ bits, uint32_t n, FastDiv dc,
-                                                        uint32_t cells3, uint32_t* __restrict__ active,
-                                                        uint32_t* __restrict__ counts) {
-    const uint32_t c = n - 1, nn = n * n, lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < cells3; i += stride) {
-        bool a = false;
-        if (i < cells3) {
-            const uint32_t ci = (uint32_t)i, t = dc.div(ci), x = ci - t * c, z = dc.div(t), y = t - z * c;
-            const uint32_t i0 = (z * n + y) * n + x;
-            const uint32_t below = bit_at(bits, i0) + bit_at(bits, i0 + 1) + bit_at(bits, i0 + n) +
-                                   bit_at(bits, i0 + n + 1) + bit_at(bits, i0 + nn) + bit_at(bits, i0 + nn + 1) +
-                                   bit_at(bits, i0 + nn + n) + bit_at(bits, i0 + nn + n + 1);
-            a = below != 0 && below != 8;
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, a);
-        if (lane == 0) {
-            active[i >> 5] = m;
-            counts[i >> 5] = __popc(m);
-        }
-    }
-}
-
-// Edge `local` of sweep s (capi.mojo:1090-1128): its lower node; sweep order z, y, x.
-struct SideDiv {  // the cell count per axis c and c - 1, as invariant divisors
-    uint32_t c;
-    FastDiv dc, dm;
+// Row words of the sign bits (n + 31) / 32 and of the cells' (c + 31) / 32, c = n - 1.
+struct Rows {
+    uint32_t n, c, sign_words, words, segment;  // segment: c^2 words of one kind, rounded up to whole scan tiles
+    FastDiv by_words, by_c;
+    __host__ explicit Rows(int64_t side)
+        : n((uint32_t)side), c(n - 1), sign_words((n + 31) / 32), words((c + 31) / 32),
+          segment((c * c * words + kTileWords - 1) / kTileWords * kTileWords), by_words(words), by_c(c) {}
 };
 
-__device__ __forceinline__ void sweep_edge(int s, uint32_t local, const SideDiv& sd, uint32_t& x, uint32_t& y,
-                                           uint32_t& z) {
-    const uint32_t c = sd.c, cm1 = c - 1;
-    if (s == 0) {  // x-edges: z, y in [1, c), x in [0, c)
-        const uint32_t t = sd.dc.div(local), u = sd.dm.div(t);
-        x = local - t * c;
-        y = 1 + (t - u * cm1);
-        z = 1 + u;
-    } else if (s == 1) {  // y-edges: z in [1, c), y in [0, c), x in [1, c)
-        const uint32_t t = sd.dm.div(local), u = sd.dc.div(t);
-        x = 1 + (local - t * cm1);
-        y = t - u * c;
-        z = 1 + u;
-    } else {  // z-edges: z in [0, c), y, x in [1, c)
-        const uint32_t t = sd.dm.div(local), u = sd.dm.div(t);
-        x = 1 + (local - t * cm1);
-        y = 1 + (t - u * cm1);
-        z = u;
-    }
-}
-
-// Sign-changing edges of the three sweeps as bits (word w of sweep s at
-// s * words + w) and per-word popcounts.  An interior edge that changes sign
-// lies on four active cells, so it always yields a quad.
-__global__ void __launch_bounds__(kT) edge_words_kernel(const uint32_t* __restrict__ bits, uint32_t n, SideDiv sd,
-                                                        uint32_t per_sweep, uint32_t words,
-                                                        uint32_t* __restrict__ fwords, uint32_t* __restrict__ counts) {
-    const int s = blockIdx.y;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t step = s == 0 ? 1u : (s == 1 ? n : n * n);
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e - lane < per_sweep; e += stride) {
-        bool a = false;
-        if (e < per_sweep) {
-            uint32_t x, y, z;
-            sweep_edge(s, (uint32_t)e, sd, x, y, z);
-            const uint32_t i0 = (z * n + y) * n + x;
-            a = bit_at(bits, i0) != bit_at(bits, i0 + step);
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, a);
-        if (lane == 0) {
-            fwords[(uint64_t)s * words + (e >> 5)] = m;
-            counts[(uint64_t)s * words + (e >> 5)] = __popc(m);
-        }
-    }
-}
-
-__global__ void store_counts_kernel(const uint32_t* __restrict__ totals, int64_t* __restrict__ counts) {
-    counts[0] = totals[0];
-    counts[1] = 2 * (int64_t)totals[1];  // two triangles per quad
-}
-
-// One thread per 32-cell word: each active cell's vertex at id = its rank.
-__global__ void __launch_bounds__(kT) vertex_words_kernel(const double* __restrict__ field,
-                                                          const double* __restrict__ density, uint32_t n, FastDiv dc,
-                                                          IsoArg iso_arg, const uint32_t* __restrict__ active,
-                                                          const uint32_t* __restrict__ first, uint32_t cell_words,
-                                                          double* __restrict__ vertices,
-                                                          double* __restrict__ vertex_density) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= cell_words) return;
-    uint32_t m = active[w];
-    if (!m) return;
+// bits: bit x & 31 of word x >> 5 of row (y, z) = (field < iso), one warp per row;
+// *bad |= 1 (bad may be null) if a value is not finite.
+__global__ void __launch_bounds__(kT) sign_rows_kernel(const double* __restrict__ field, Rows g, IsoArg iso_arg,
+                                                       uint32_t* __restrict__ bits, uint32_t* __restrict__ bad) {
     const double iso = iso_arg.get();
-    const uint32_t c = n - 1;
-    const double cells_d = (double)c;
-    uint32_t id = first[w];
-    while (m) {
-        const uint32_t b = __ffs(m) - 1;
-        m &= m - 1;
-        const uint32_t ci = 32 * w + b, t = dc.div(ci), x = ci - t * c, z = dc.div(t), y = t - z * c;
-        cell_vertex(field, density, n, x, y, z, iso, cells_d, vertices + 3 * (int64_t)id, vertex_density + id);
-        ++id;
+    const uint32_t lane = threadIdx.x & 31, row = blockIdx.x * (kT / 32) + (threadIdx.x >> 5);
+    if (row >= g.n * g.n) return;
+    const double* __restrict__ f = field + (uint64_t)row * g.n;
+    bool broken = false;
+#pragma unroll 4
+    for (uint32_t w = 0; w < g.sign_words; ++w) {
+        const uint32_t x = 32 * w + lane;
+        const double v = x < g.n ? f[x] : 0.0;
+        broken |= !isfinite(v);
+        const uint32_t m = __ballot_sync(0xffffffffu, x < g.n && v < iso);
+        if (lane == 0) bits[(uint64_t)row * g.sign_words + w] = m;
+    }
+    if (bad && broken) atomicOr(bad, 1u);
+}
+
+// *bad |= flag if a value is not finite.
+__global__ void __launch_bounds__(kT) finite_kernel(const double* __restrict__ values, uint64_t count,
+                                                    uint32_t* __restrict__ bad, uint32_t flag) {
+    bool broken = false;
+    const uint64_t stride = (uint64_t)gridDim.x * kT;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)blockIdx.x * kT + threadIdx.x; i < count; i += stride) broken |= !isfinite(values[i]);
+    if (broken) atomicOr(bad, flag);
+}
+
+// Word t of each segment: active cells (corners on both sides, capi.mojo:946-960) and
+// sign-changing edges of the three sweeps (capi.mojo:1090-1128: x-edges with y, z >= 1,
+// y-edges with x, z >= 1, z-edges with x, y >= 1; coordinates below c).  An interior edge
+// that changes sign lies on four active cells, so it always yields a quad.
+__global__ void __launch_bounds__(kT) item_words_kernel(const uint32_t* __restrict__ bits, Rows g,
+                                                        uint32_t* __restrict__ items) {
+    const uint32_t t = blockIdx.x * kT + threadIdx.x;
+    if (t >= g.segment) return;
+    uint32_t out[4] = {0, 0, 0, 0};
+    const uint32_t row = g.by_words.div(t), w = t - row * g.words;
+    if (row < g.c * g.c) {
+        const uint32_t z = g.by_c.div(row), y = row - z * g.c;
+        uint32_t any = 0, all = ~0u, here = 0, shifted = 0, up_y = 0, up_z = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t at = ((uint64_t)(z + (k >> 1)) * g.n + y + (k & 1)) * g.sign_words + w;
+            const uint32_t b = bits[at], next = w + 1 < g.sign_words ? bits[at + 1] : 0u, s = __funnelshift_r(b, next, 1);
+            any |= b | s;
+            all &= b & s;
+            if (k == 0) {
+                here = b;
+                shifted = s;
+            } else if (k == 1) up_y = b;
+            else if (k == 2) up_z = b;
+        }
+        const uint32_t left = g.c - 32 * w, inside = left >= 32 ? ~0u : (1u << left) - 1u;
+        const uint32_t inner = w == 0 ? inside & ~1u : inside;  // x >= 1
+        out[0] = any & ~all & inside;
+        if (y && z) out[1] = (here ^ shifted) & inside;
+        if (z) out[2] = (here ^ up_y) & inner;
+        if (y) out[3] = (here ^ up_z) & inner;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) items[(uint64_t)k * g.segment + t] = out[k];
+}
+
+__global__ void __launch_bounds__(kScanThreads) popcount_tiles_kernel(const uint32_t* __restrict__ items,
+                                                                      uint32_t* __restrict__ tile_sums) {
+    __shared__ uint32_t warp_sums[32];
+    const uint4* __restrict__ p =
+        reinterpret_cast<const uint4*>(items + (uint64_t)blockIdx.x * kTileWords) + 2 * threadIdx.x;
+    const uint4 a = p[0], b = p[1];
+    uint32_t total;
+    block_exclusive_scan<uint32_t>(__popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) +
+                                       __popc(b.z) + __popc(b.w),
+                                   warp_sums, total);
+    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+}
+static_assert(kScanItems == 8, "two uint4 per thread");
+
+// tile_sums scanned: entry `tiles` of a segment is the number of cells, the last the number of items.
+__global__ void store_counts_kernel(const uint32_t* __restrict__ tile_sums, uint32_t tiles, const uint32_t* total,
+                                    const uint32_t* bad, int64_t* __restrict__ counts) {
+    counts[0] = tile_sums[tiles];
+    counts[1] = 2 * (int64_t)(*total - tile_sums[tiles]);  // two triangles per quad
+    if (bad) counts[2] = *bad;
+}
+
+// Every item's place (kind, row and x) into the first slot of its output, in order, and the
+// words' first cell ids.
+__device__ __forceinline__ uint64_t place_of(uint32_t kind, uint32_t row, uint32_t x) {
+    return ((uint64_t)kind << 60) | ((uint64_t)row << 16) | x;
+}
+
+__global__ void __launch_bounds__(kScanThreads) place_kernel(const uint32_t* __restrict__ items, Rows g, uint32_t tiles,
+                                                             const uint32_t* __restrict__ tile_sums,
+                                                             uint32_t* __restrict__ first,
+                                                             uint64_t* __restrict__ vertex_slots,
+                                                             uint64_t* __restrict__ face_slots) {
+    __shared__ uint32_t warp_sums[32];
+    const uint32_t kind = blockIdx.x / tiles, t0 = (blockIdx.x - kind * tiles) * kTileWords + threadIdx.x * kScanItems;
+    const uint4* __restrict__ p = reinterpret_cast<const uint4*>(items + (uint64_t)kind * g.segment + t0);
+    const uint4 a = p[0], b = p[1];
+    const uint32_t word[kScanItems] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) sum += __popc(word[k]);
+    uint32_t id = tile_sums[blockIdx.x] + block_exclusive_scan<uint32_t>(sum, warp_sums, total);
+    const uint32_t cells = tile_sums[tiles];
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        const uint32_t t = t0 + k;
+        if (kind == 0) first[t] = id;
+        uint32_t m = word[k];
+        const uint32_t row = g.by_words.div(t), x0 = 32 * (t - row * g.words);
+        while (m) {
+            const uint64_t place = place_of(kind, row, x0 + __ffs(m) - 1);
+            m &= m - 1;
+            if (kind == 0) {
+                if (vertex_slots) vertex_slots[id] = place;
+            } else if (face_slots) {
+                face_slots[6 * (uint64_t)(id - cells)] = place;
+            }
+            ++id;
+        }
     }
 }
 
-__device__ __forceinline__ int64_t cell_id(const uint32_t* __restrict__ active, const uint32_t* __restrict__ first,
-                                           uint32_t ci) {
-    return (int64_t)first[ci >> 5] + lanes_below(active[ci >> 5], ci & 31);
-}
-
-// One thread per 32-edge word: each sign-changing edge's two triangles at
-// quad = its rank (capi.mojo:1040-1071).
-__global__ void __launch_bounds__(kT) face_words_kernel(const uint32_t* __restrict__ bits, uint32_t n, SideDiv sd,
-                                                        uint32_t words, const uint32_t* __restrict__ fwords,
-                                                        const uint32_t* __restrict__ ffirst,
-                                                        const uint32_t* __restrict__ active,
-                                                        const uint32_t* __restrict__ first,
-                                                        int64_t* __restrict__ faces) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= words) return;
-    const int s = blockIdx.y;
-    uint32_t m = fwords[(uint64_t)s * words + w];
-    if (!m) return;
-    const uint32_t c = n - 1;
-    int64_t quad = ffirst[(uint64_t)s * words + w];
-    while (m) {
-        const uint32_t b = __ffs(m) - 1;
-        m &= m - 1;
-        uint32_t x, y, z;
-        sweep_edge(s, 32 * w + b, sd, x, y, z);
-        const bool reverse = bit_at(bits, (z * n + y) * n + x) != 0;
-        uint32_t q[4];
-        if (s == 0) {
-            q[0] = (uint32_t)grid_index(x, y - 1, z - 1, c);
-            q[1] = (uint32_t)grid_index(x, y, z - 1, c);
-            q[2] = (uint32_t)grid_index(x, y, z, c);
-            q[3] = (uint32_t)grid_index(x, y - 1, z, c);
-        } else if (s == 1) {
-            q[0] = (uint32_t)grid_index(x - 1, y, z - 1, c);
-            q[1] = (uint32_t)grid_index(x - 1, y, z, c);
-            q[2] = (uint32_t)grid_index(x, y, z, c);
-            q[3] = (uint32_t)grid_index(x, y, z - 1, c);
-        } else {
-            q[0] = (uint32_t)grid_index(x - 1, y - 1, z, c);
-            q[1] = (uint32_t)grid_index(x, y - 1, z, c);
-            q[2] = (uint32_t)grid_index(x, y, z, c);
-            q[3] = (uint32_t)grid_index(x - 1, y, z, c);
-        }
-        const int64_t a = cell_id(active, first, q[0]), bb = cell_id(active, first, q[1]);
-        const int64_t cc = cell_id(active, first, q[2]), d = cell_id(active, first, q[3]);
-        int64_t* out = faces + 6 * quad;
-        if (reverse) {
-            out[0] = a; out[1] = d; out[2] = cc; out[3] = a; out[4] = cc; out[5] = bb;
-        } else {
-            out[0] = a; out[1] = bb; out[2] = cc; out[3] = a; out[4] = cc; out[5] = d;
-        }
-        ++quad;
+__global__ void __launch_bounds__(kT) vertices_kernel(const double* __restrict__ field,
+                                                      const double* __restrict__ density, Rows g, IsoArg iso_arg,
+                                                      const uint32_t* __restrict__ cells, double* __restrict__ vertices,
+                                                      double* __restrict__ vertex_density) {
+    const uint32_t count = *cells;
+    for (uint32_t id = blockIdx.x * kT + threadIdx.x; id < count; id += gridDim.x * kT) {
+        const uint64_t place = reinterpret_cast<const uint64_t*>(vertex_density)[id];
+        const uint32_t x = (uint32_t)place & 0xffffu, row = (uint32_t)(place >> 16), z = g.by_c.div(row), y = row - z * g.c;
+        cell_vertex(field, density, g.n, x, y, z, iso_arg.get(), (double)g.c, vertices + 3 * (int64_t)id,
+                    vertex_density + id);
     }
 }
 
-inline uint64_t words_of(uint64_t items) { return (items + 31) / 32; }
+// One thread per quad: its two triangles (capi.mojo:1040-1071).
+__global__ void __launch_bounds__(kT) quads_kernel(const uint32_t* __restrict__ bits, Rows g,
+                                                   const uint32_t* __restrict__ items,
+                                                   const uint32_t* __restrict__ first,
+                                                   const uint32_t* __restrict__ cells, const uint32_t* __restrict__ total,
+                                                   int64_t* __restrict__ faces) {
+    const uint32_t count = *total - *cells;
+    for (uint32_t quad = blockIdx.x * kT + threadIdx.x; quad < count; quad += gridDim.x * kT) {
+        int64_t* out = faces + 6 * (int64_t)quad;
+        const uint64_t place = (uint64_t)out[0];
+        const uint32_t kind = (uint32_t)(place >> 60), x = (uint32_t)place & 0xffffu, row = (uint32_t)(place >> 16);
+        const uint32_t z = g.by_c.div(row), y = row - z * g.c;
+        const bool reverse = (bits[((uint64_t)z * g.n + y) * g.sign_words + (x >> 5)] >> (x & 31)) & 1u;
+        auto cell = [&](uint32_t cx, uint32_t cy, uint32_t cz) -> int64_t {
+            const uint32_t t = (cz * g.c + cy) * g.words + (cx >> 5);
+            return (int64_t)first[t] + lanes_below(items[t], cx & 31);
+        };
+        int64_t a, b, c, d;
+        if (kind == 1) {
+            a = cell(x, y - 1, z - 1);
+            b = cell(x, y, z - 1);
+            c = cell(x, y, z);
+            d = cell(x, y - 1, z);
+        } else if (kind == 2) {
+            a = cell(x - 1, y, z - 1);
+            b = cell(x - 1, y, z);
+            c = cell(x, y, z);
+            d = cell(x, y, z - 1);
+        } else {
+            a = cell(x - 1, y - 1, z);
+            b = cell(x, y - 1, z);
+            c = cell(x, y, z);
+            d = cell(x - 1, y, z);
+        }
+        out[0] = a;
+        out[1] = reverse ? d : b;
+        out[2] = c;
+        out[3] = a;
+        out[4] = c;
+        out[5] = reverse ? b : d;
+    }
+}
 
 // Arrays carved from the workspace, identically in count and emit.
 struct Layout {
-    uint32_t n, c, nodes, cells3, cell_words, per_sweep, words;
-    uint32_t *bits, *active, *first, *fwords, *ffirst, *totals;
-    void* base;
-    size_t bytes, used;
-    Workspace scratch() const {  // the scan scratch after the arrays
-        Workspace w(base, bytes);
-        w.used = used;
-        return w;
+    Rows g;
+    uint32_t tiles;  // scan tiles per segment
+    uint32_t *bits, *items, *first, *tile_sums, *total, *bad;
+    explicit Layout(int64_t n) : g(n), tiles(g.segment / kTileWords) {}
+    void carve(Workspace& w) {
+        bits = w.take<uint32_t>((size_t)g.n * g.n * g.sign_words);
+        items = w.take<uint32_t>((size_t)4 * g.segment);
+        first = w.take<uint32_t>(g.segment);
+        tile_sums = w.take<uint32_t>((size_t)4 * tiles + 1);
+        total = w.take<uint32_t>(1);
+        bad = w.take<uint32_t>(1);
     }
 };
 
-template <class W>
-void carve(W& w, uint64_t nodes, uint64_t cell_words, uint64_t words, uint32_t** out) {
-    out[0] = w.template take<uint32_t>(words_of(nodes));
-    out[1] = w.template take<uint32_t>(cell_words);
-    out[2] = w.template take<uint32_t>(cell_words + 1);
-    out[3] = w.template take<uint32_t>(3 * words + 1);
-    out[4] = w.template take<uint32_t>(3 * words + 1);
-    out[5] = w.template take<uint32_t>(2);
-}
-
-inline Layout layout(int64_t n, void* base, size_t bytes) {
-    Layout L{};
-    L.n = (uint32_t)n;
-    L.c = (uint32_t)(n - 1);
-    L.nodes = (uint32_t)(n * n * n);
-    L.cells3 = L.c * L.c * L.c;
-    L.cell_words = (uint32_t)words_of(L.cells3);
-    L.per_sweep = L.c == 0 ? 0 : L.c * (L.c - 1) * (L.c - 1);
-    L.words = (uint32_t)words_of(L.per_sweep);
-    Workspace w(base, bytes);
-    uint32_t* p[6];
-    carve(w, L.nodes, L.cell_words, L.words, p);
-    L.bits = p[0];
-    L.active = p[1];
-    L.first = p[2];
-    L.fwords = p[3];
-    L.ffirst = p[4];
-    L.totals = p[5];
-    L.base = base;
-    L.bytes = bytes;
-    L.used = w.used;
-    return L;
-}
-
 inline size_t workspace_bytes(int64_t n) {
+    if (n > kMaxSide) n = kMaxSide;
     return measure([&](Workspace& w) {
-        const uint64_t c = n - 1, nodes = (uint64_t)n * n * n, cells3 = c * c * c;
-        const uint64_t per_sweep = c == 0 ? 0 : c * (c - 1) * (c - 1);
-        const uint64_t cw = words_of(cells3), fw = words_of(per_sweep);
-        uint32_t* p[6];
-        carve(w, nodes, cw, fw, p);
-        scan_carve<uint32_t>(w, (int64_t)(cw > 3 * fw ? cw : 3 * fw));
+        Layout L(n);
+        L.carve(w);
+        scan_carve<uint32_t>(w, 4 * (int64_t)L.tiles);
     });
 }
 
-inline unsigned grid_for(uint64_t items) {
-    uint64_t b = (items + kT - 1) / kT;
-    const uint64_t cap = (uint64_t)kSMs * 16;
-    return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
+static int count_items(const double* field, const double* density, int64_t n, const double* iso, int64_t* counts,
+                       bool checked, void* workspace, size_t bytes, cudaStream_t s) {
+    if (n < 2 || n > kMaxSide || !field || !iso || !counts) return fail(PB_ERR_INVALID, "extract count: bad args");
+    if (!workspace || bytes < workspace_bytes(n))
+        return fail(PB_ERR_WORKSPACE, "extract: workspace needs %zu bytes", workspace_bytes(n));
+    Workspace w(workspace, bytes);
+    Layout L(n);
+    L.carve(w);
+    const Rows& g = L.g;
+    if (checked) PB_CHECK_CUDA(cudaMemsetAsync(L.bad, 0, sizeof(uint32_t), s), "extract flags");
+    sign_rows_kernel<<<(g.n * g.n + kT / 32 - 1) / (kT / 32), kT, 0, s>>>(field, g, IsoArg{0.0, iso}, L.bits,
+                                                                          checked ? L.bad : nullptr);
+    PB_CHECK_LAUNCH("sign_rows_kernel");
+    if (checked && density) {
+        const uint64_t nodes = (uint64_t)n * n * n;
+        finite_kernel<<<(unsigned)std::min<uint64_t>((nodes + kT - 1) / kT, (uint64_t)kSMs * 16), kT, 0, s>>>(
+            density, nodes, L.bad, 2u);
+        PB_CHECK_LAUNCH("finite_kernel");
+    }
+    item_words_kernel<<<g.segment / kT, kT, 0, s>>>(L.bits, g, L.items);
+    PB_CHECK_LAUNCH("item_words_kernel");
+    popcount_tiles_kernel<<<4 * L.tiles, kScanThreads, 0, s>>>(L.items, L.tile_sums);
+    PB_CHECK_LAUNCH("popcount_tiles_kernel");
+    PB_TRY(exclusive_scan<uint32_t>(L.tile_sums, L.tile_sums, 4 * (int64_t)L.tiles, L.total, w, s));
+    store_counts_kernel<<<1, 1, 0, s>>>(L.tile_sums, L.tiles, L.total, checked ? L.bad : nullptr, counts);
+    PB_CHECK_LAUNCH("store_counts_kernel");
+    return PB_OK;
 }
 
 }  // namespace fast
@@ -649,34 +664,14 @@ extern "C" size_t pb_extract_workspace_size(int64_t n) { return fast::workspace_
 // with the same field, side, iso and workspace.  Sides 2..1025.
 extern "C" int pb_extract_count_f64(const double* field, int64_t n, const double* iso, int64_t* counts,
                                     void* workspace, size_t workspace_bytes, void* stream) {
-    if (n < 2 || n > fast::kMaxSide || !field || !iso || !counts) return fail(PB_ERR_INVALID, "extract count: bad args");
-    if (!workspace || workspace_bytes < fast::workspace_bytes(n))
-        return fail(PB_ERR_WORKSPACE, "extract: workspace needs %zu bytes", fast::workspace_bytes(n));
-    cudaStream_t s = (cudaStream_t)stream;
-    fast::Layout L = fast::layout(n, workspace, workspace_bytes);
-    const IsoArg ia{0.0, iso};
-    fast::sign_bits_kernel<<<fast::grid_for(L.nodes), fast::kT, 0, s>>>(field, L.nodes, ia, L.bits);
-    PB_CHECK_LAUNCH("sign_bits_kernel");
-    const FastDiv dc(L.n - 1);
-    const fast::SideDiv sd{L.n - 1, dc, FastDiv(L.n - 2)};
-    fast::cell_words_kernel<<<fast::grid_for(L.cells3), fast::kT, 0, s>>>(L.bits, L.n, dc, L.cells3, L.active,
-                                                                           L.first);
-    PB_CHECK_LAUNCH("cell_words_kernel");
-    Workspace scan_ws = L.scratch();
-    PB_TRY(exclusive_scan<uint32_t>(L.first, L.first, L.cell_words, L.totals, scan_ws, s));
-    if (L.per_sweep) {
-        fast::edge_words_kernel<<<dim3(fast::grid_for(L.per_sweep), 3), fast::kT, 0, s>>>(L.bits, L.n, sd,
-                                                                                           L.per_sweep, L.words,
-                                                                                           L.fwords, L.ffirst);
-        PB_CHECK_LAUNCH("edge_words_kernel");
-        Workspace scan_ws2 = L.scratch();
-        PB_TRY(exclusive_scan<uint32_t>(L.ffirst, L.ffirst, 3 * (int64_t)L.words, L.totals + 1, scan_ws2, s));
-    } else {
-        PB_CHECK_CUDA(cudaMemsetAsync(L.totals + 1, 0, sizeof(uint32_t), s), "extract face total");
-    }
-    fast::store_counts_kernel<<<1, 1, 0, s>>>(L.totals, counts);
-    PB_CHECK_LAUNCH("store_counts_kernel");
-    return PB_OK;
+    return fast::count_items(field, nullptr, n, iso, counts, false, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+// The same, and counts[2] (device int64[3]): 1 if a field value is not finite, plus 2 if a
+// density value (density may be null) is not.
+extern "C" int pb_extract_count_checked_f64(const double* field, const double* density, int64_t n, const double* iso,
+                                            int64_t* counts, void* workspace, size_t workspace_bytes, void* stream) {
+    return fast::count_items(field, density, n, iso, counts, true, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 // Emits the counted mesh: vertices (counts[0] x 3), vertex_density
@@ -687,23 +682,29 @@ extern "C" int pb_extract_count_f64(const double* field, int64_t n, const double
 extern "C" int pb_extract_emit_f64(const double* field, const double* density, int64_t n, const double* iso,
                                    double* vertices, double* vertex_density, int64_t* faces, void* workspace,
                                    size_t workspace_bytes, void* stream) {
-    if (n < 2 || n > fast::kMaxSide || !field || !iso || (vertices && (!density || !vertex_density)))
+    using namespace fast;
+    if (n < 2 || n > kMaxSide || !field || !iso || (vertices && (!density || !vertex_density)))
         return fail(PB_ERR_INVALID, "extract emit: bad args");
     if (!workspace || workspace_bytes < fast::workspace_bytes(n))
         return fail(PB_ERR_WORKSPACE, "extract: workspace needs %zu bytes", fast::workspace_bytes(n));
+    if (!vertices && !faces) return PB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    fast::Layout L = fast::layout(n, workspace, workspace_bytes);
-    const IsoArg ia{0.0, iso};
+    Workspace w(workspace, workspace_bytes);
+    Layout L(n);
+    L.carve(w);
+    static_assert(sizeof(double) == sizeof(uint64_t) && sizeof(int64_t) == sizeof(uint64_t), "a place fits a slot");
+    place_kernel<<<4 * L.tiles, kScanThreads, 0, s>>>(L.items, L.g, L.tiles, L.tile_sums, L.first,
+                                                      vertices ? (uint64_t*)vertex_density : nullptr, (uint64_t*)faces);
+    PB_CHECK_LAUNCH("place_kernel");
+    const unsigned blocks = 16 * kSMs;  // grid-stride: the counts stay on the device
     if (vertices) {
-        fast::vertex_words_kernel<<<(L.cell_words + fast::kT - 1) / fast::kT, fast::kT, 0, s>>>(
-            field, density, L.n, FastDiv(L.n - 1), ia, L.active, L.first, L.cell_words, vertices, vertex_density);
-        PB_CHECK_LAUNCH("vertex_words_kernel");
+        vertices_kernel<<<blocks, kT, 0, s>>>(field, density, L.g, IsoArg{0.0, iso}, L.tile_sums + L.tiles, vertices,
+                                              vertex_density);
+        PB_CHECK_LAUNCH("vertices_kernel");
     }
-    if (faces && L.per_sweep) {
-        fast::face_words_kernel<<<dim3((L.words + fast::kT - 1) / fast::kT, 3), fast::kT, 0, s>>>(
-            L.bits, L.n, fast::SideDiv{L.n - 1, FastDiv(L.n - 1), FastDiv(L.n - 2)}, L.words, L.fwords, L.ffirst,
-            L.active, L.first, faces);
-        PB_CHECK_LAUNCH("face_words_kernel");
+    if (faces) {
+        quads_kernel<<<blocks, kT, 0, s>>>(L.bits, L.g, L.items, L.first, L.tile_sums + L.tiles, L.total, faces);
+        PB_CHECK_LAUNCH("quads_kernel");
     }
     return PB_OK;
 }
