@@ -96,6 +96,14 @@ int pb_splat_f64(const double *points, const double *normals, int64_t point_coun
                  int64_t confidence, double *density, double *vx, double *vy, double *vz,
                  double *screen, double samples_per_node, int64_t *accepted,
                  void *workspace, size_t workspace_bytes, void *stream);
+/* Splat and assembly from points to the solver's grids in one call (core.py:228-265): density
+ * (divided by samples_per_node), screen and rhs, n^3 each and overwritten; the bits of zeroed grids
+ * through pb_splat_f64, pb_divide_f64 and pb_assemble_f64, without the three dense vector grids. */
+size_t pb_splat_assemble_workspace_size(int64_t point_count, int64_t n);
+int pb_splat_assemble_f64(const double *points, const double *normals, int64_t point_count, int64_t n,
+                          int64_t confidence, double samples_per_node, double point_weight,
+                          double target_value, double *density, double *screen, double *rhs,
+                          int64_t *accepted, void *workspace, size_t workspace_bytes, void *stream);
 /* Auxiliary attribute interpolation (no counterpart in the reference, which
  * lists it among upstream PoissonRecon features it leaves out, README.md:31-36):
  * per-sample attributes (point_count x channels, row-major FP64) of unit-cube
@@ -111,6 +119,13 @@ int pb_splat_attributes_f64(const double *points, const double *normals, int64_t
                             void *workspace, size_t workspace_bytes, void *stream);
 int pb_sample_attributes_f64(const double *vertices, int64_t vertex_count, const double *map, int64_t n,
                              const double *grids, int64_t channels, double *out, void *stream);
+/* Both in one call: attribute values at the vertices (out: vertex_count x channels), the sums kept
+ * only at the nodes that samples touch.  Same bits. */
+size_t pb_interpolate_attributes_workspace_size(int64_t point_count, int64_t n, int64_t channels);
+int pb_interpolate_attributes_f64(const double *points, const double *normals, int64_t point_count, int64_t n,
+                                  int64_t confidence, const double *attributes, int64_t channels,
+                                  const double *vertices, int64_t vertex_count, const double *map, double *out,
+                                  void *workspace, size_t workspace_bytes, void *stream);
 
 /* mpr_assemble_f64 (_lib.py:24; capi.mojo:228-279):
  * rhs = -div(V) + point_weight * screen * (n-1)^2 * target_value. Bit-exact. */

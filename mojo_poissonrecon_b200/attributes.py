@@ -6,7 +6,7 @@ sample's attributes are splatted on the device with the sample's pass-1
 weights w (the screening weights of `reconstruct` at the same depth and
 scale), summed per grid node in sample order, and a mesh vertex takes the
 ratio of the trilinear interpolants of sum w a and sum w over its cell
-(csrc/splat.cu: pb_splat_attributes_f64, pb_sample_attributes_f64).
+(csrc/splat.cu: pb_interpolate_attributes_f64).
 """
 
 from __future__ import annotations
@@ -55,17 +55,14 @@ def interpolate_attributes(points, normals, attributes, vertices, *, depth: int 
         raise ValueError(f"{points.shape[0] - count} (point, normal) rows are invalid; drop them (and their "
                          "attributes) first")
     n = (1 << depth) + 1
-    grids = torch.empty((channels + 1, n, n, n), dtype=torch.float64, device=ctx.device)
     attrs = core._to_device(values, ctx.device)
-    ptr, size = ctx.ws.get(L.pb_splat_attributes_workspace_size(count))
-    ctx.check(L.pb_splat_attributes_f64(dp.data_ptr(), dn.data_ptr(), count, n, int(bool(confidence)),
-                                        attrs.data_ptr(), channels, grids.data_ptr(), ptr, size, ctx.stream),
-              "splat attributes")
     verts = core._to_device(vertices, ctx.device)
     out = torch.empty((nv, channels), dtype=torch.float64, device=ctx.device)
-    ctx.check(L.pb_sample_attributes_f64(verts.data_ptr() if nv else None, nv, fmap.data_ptr(), n, grids.data_ptr(),
-                                         channels, out.data_ptr() if nv else None, ctx.stream),
-              "sample attributes")
+    ptr, size = ctx.ws.get(L.pb_interpolate_attributes_workspace_size(count, n, channels))
+    ctx.check(L.pb_interpolate_attributes_f64(dp.data_ptr(), dn.data_ptr(), count, n, int(bool(confidence)),
+                                              attrs.data_ptr(), channels, verts.data_ptr() if nv else None, nv,
+                                              fmap.data_ptr(), out.data_ptr() if nv else None, ptr, size, ctx.stream),
+              "interpolate attributes")
     result = core._host_all([out], device_out)[0]
     if one_d:
         result = result[:, 0] if device_out else np.ascontiguousarray(result[:, 0])

@@ -237,24 +237,13 @@ def _splat_assemble(ctx: _Context, points: torch.Tensor, normals: torch.Tensor, 
     L = ctx.lib
     n = (1 << depth) + 1
     count = points.shape[0]
-    grids = {k: torch.empty((n, n, n), dtype=torch.float64, device=ctx.device)
-             for k in ("density", "vx", "vy", "vz", "screen", "rhs")}
-    # the splat accumulates into zeroed grids (core.py:229-236); assembly writes every rhs node
-    for k in ("density", "vx", "vy", "vz", "screen") if count else grids:
-        ctx.check(L.pb_fill_f64(grids[k].data_ptr(), n ** 3, 0.0, ctx.stream), "zero grid")
+    grids = {k: torch.empty((n, n, n), dtype=torch.float64, device=ctx.device) for k in ("density", "screen", "rhs")}
     accepted = torch.zeros(1, dtype=torch.int64, device=ctx.device)
-    if count:
-        ptr, size = ctx.ws.get(L.pb_splat_workspace_size(count, n))
-        ctx.check(L.pb_splat_f64(points.data_ptr(), normals.data_ptr(), count, n, int(confidence),
-                                 grids["density"].data_ptr(), grids["vx"].data_ptr(), grids["vy"].data_ptr(),
-                                 grids["vz"].data_ptr(), grids["screen"].data_ptr(), samples_per_node,
-                                 accepted.data_ptr(), ptr, size, ctx.stream), "splat")
-        ctx.check(L.pb_divide_f64(grids["density"].data_ptr(), n ** 3, samples_per_node, ctx.stream), "divide")
-        ctx.check(L.pb_assemble_f64(grids["vx"].data_ptr(), grids["vy"].data_ptr(), grids["vz"].data_ptr(),
-                                    grids["screen"].data_ptr(), grids["rhs"].data_ptr(), n, point_weight, 0.5,
-                                    ctx.stream), "assemble")
-    for k in ("vx", "vy", "vz"):
-        del grids[k]
+    ptr, size = ctx.ws.get(L.pb_splat_assemble_workspace_size(count, n))
+    ctx.check(L.pb_splat_assemble_f64(points.data_ptr() if count else None, normals.data_ptr() if count else None,
+                                      count, n, int(confidence), samples_per_node, point_weight, 0.5,
+                                      *(grids[k].data_ptr() for k in ("density", "screen", "rhs")),
+                                      accepted.data_ptr(), ptr, size, ctx.stream), "splat and assembly")
     return grids, accepted
 
 

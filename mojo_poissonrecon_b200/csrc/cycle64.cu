@@ -409,12 +409,18 @@ __global__ void __launch_bounds__(256) split_setup_kernel(Split g, SplitLevel L,
     }
 }
 
-// The dense iterate.
-__global__ void __launch_bounds__(256) split_merge_kernel(Split g, SplitLevel L, double* __restrict__ out) {
-    const uint32_t t = blockIdx.x * 256u + threadIdx.x;
-    if (t >= (uint32_t)g.n * g.n * g.n) return;
-    const int row = t / (uint32_t)g.n, x = t - row * g.n, y = row % g.n, z = row / g.n;
-    out[t] = (((x + y + z) & 1) ? L.x[1] : L.x[0])[g.node(x, y, z)];
+// The dense iterate: threads flattened over a plane's (x, y), several planes each so that enough loads are in
+// flight (one node per thread took 73 us at 257^3).
+constexpr int kMergeZ = 8;
+__global__ void __launch_bounds__(256) split_merge_kernel(Split g, const double* __restrict__ x0,
+                                                          const double* __restrict__ x1, double* __restrict__ out) {
+    const uint32_t t = blockIdx.x * 256u + threadIdx.x, n = g.n;
+    if (t >= n * n) return;
+    const uint32_t y = t / n, x = t - y * n, z0 = blockIdx.y * kMergeZ, z1 = min(n, z0 + kMergeZ);
+    uint32_t at = g.node(x, y, z0);
+#pragma unroll
+    for (uint32_t z = z0; z < z0 + kMergeZ; ++z, at += g.plane)
+        if (z < z1) out[((uint64_t)z * n + y) * n + x] = (((x + y + z) & 1) ? x1 : x0)[at];
 }
 
 __device__ __forceinline__ double2 pair_at(const double* p, uint32_t i) {
@@ -871,10 +877,8 @@ extern "C" int pb_vcycle_field_f64(int64_t n, const double* iterate, double* fie
         return PB_OK;
     }
     const Split g((int)n);
-    SplitLevel L = {};
-    L.x[0] = const_cast<double*>(iterate);
-    L.x[1] = L.x[0] + g.count;
-    split_merge_kernel<<<blocks_for(n * n * n, 256), 256, 0, s>>>(g, L, field);
+    split_merge_kernel<<<dim3(blocks_for(n * n, 256), (unsigned)((n + kMergeZ - 1) / kMergeZ)), 256, 0, s>>>(
+        g, iterate, iterate + g.count, field);
     PB_CHECK_LAUNCH("split_merge_kernel");
     return PB_OK;
 }

@@ -153,34 +153,31 @@ __global__ void __launch_bounds__(kNormThreads) sumsq_kernel(const double* __res
 }
 
 // ---- restriction (capi.mojo:557-673) ----------------------------------------
-__global__ void restrict_kernel(const double* __restrict__ fine, double* __restrict__ coarse, int64_t fine_n) {
-    const int64_t cn = (fine_n + 1) / 2;
-    const int64_t total = cn * cn * cn;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = idx % cn, y = (idx / cn) % cn, z = idx / (cn * cn);
-        double sum = 0.0, weight = 0.0;
-        for (int oz = -1; oz <= 1; ++oz) {
-            const int64_t zz = 2 * z + oz;
-            if (zz < 0 || zz >= fine_n) continue;
-            const double wz = oz == 0 ? 2.0 : 1.0;
-            for (int oy = -1; oy <= 1; ++oy) {
-                const int64_t yy = 2 * y + oy;
-                if (yy < 0 || yy >= fine_n) continue;
-                const double wy = oy == 0 ? 2.0 : 1.0;
-                const double* row = fine + (zz * fine_n + yy) * fine_n;
-                for (int ox = -1; ox <= 1; ++ox) {
-                    const int64_t xx = 2 * x + ox;
-                    if (xx < 0 || xx >= fine_n) continue;
-                    const double wx = ox == 0 ? 2.0 : 1.0;
-                    const double w = wx * wy * wz;
-                    sum += row[xx] * w;
-                    weight += w;
-                }
-            }
-        }
-        coarse[idx] = sum / weight;
+// Threads flattened over a coarse plane's (x, y), one plane per blockIdx.y.
+__global__ void __launch_bounds__(256) restrict_kernel(const double* __restrict__ fine, double* __restrict__ coarse,
+                                                       uint32_t fine_n) {
+    const uint32_t cn = (fine_n + 1) / 2, t = blockIdx.x * 256u + threadIdx.x;
+    if (t >= cn * cn) return;
+    const uint32_t y = t / cn, x = t - y * cn, z = blockIdx.y;
+    const double* __restrict__ centre = fine + ((uint64_t)(2 * z) * fine_n + 2 * y) * fine_n + 2 * x;
+    const int64_t sy = fine_n, sz = (int64_t)fine_n * fine_n;
+    double sum = 0.0, weight = 0.0;
+    auto term = [&](int ox, int oy, int oz) {
+        const double w = (ox ? 1.0 : 2.0) * (oy ? 1.0 : 2.0) * (oz ? 1.0 : 2.0);
+        sum += centre[oz * sz + oy * sy + ox] * w;
+        weight += w;
+    };
+    const bool inside = x && y && z && 2 * x + 1 < fine_n && 2 * y + 1 < fine_n && 2 * z + 1 < fine_n;
+    if (inside) {
+#pragma unroll
+        for (int k = 0; k < 27; ++k) term(k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1);
+    } else {
+        for (int oz = -1; oz <= 1; ++oz)
+            for (int oy = -1; oy <= 1; ++oy)
+                for (int ox = -1; ox <= 1; ++ox)
+                    if (2 * z + oz < fine_n && 2 * y + oy < fine_n && 2 * x + ox < fine_n) term(ox, oy, oz);
     }
+    coarse[((uint64_t)z * cn + y) * cn + x] = sum / weight;
 }
 
 // ---- prolongation (capi.mojo:677-742) ---------------------------------------
@@ -313,7 +310,8 @@ extern "C" int pb_restrict_f64(const double* fine, double* coarse, int64_t fine_
     PB_TRY(check_n(fine_n, "restrict"));
     if (!fine || !coarse) return fail(PB_ERR_INVALID, "restrict: null buffer");
     const int64_t cn = (fine_n + 1) / 2;
-    restrict_kernel<<<stride_blocks(cn * cn * cn, 256), 256, 0, (cudaStream_t)stream>>>(fine, coarse, fine_n);
+    restrict_kernel<<<dim3(blocks_for(cn * cn, 256), (unsigned)cn), 256, 0, (cudaStream_t)stream>>>(fine, coarse,
+                                                                                                (uint32_t)fine_n);
     PB_CHECK_LAUNCH("restrict_kernel");
     return PB_OK;
 }

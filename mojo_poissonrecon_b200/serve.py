@@ -81,7 +81,7 @@ def hierarchy_bytes(n: int) -> int:
 
 def footprint_bytes(depth: int, points: int) -> int:
     """Peak device bytes of one FP32-refined reconstruction at `depth` with
-    `points` samples in a batch: the inputs and their prepared copies, the six
+    `points` samples in a batch: the inputs and their prepared copies, the three
     FP64 grids and the splat's workspace while splatting; then density, screen
     and rhs, the FP32 hierarchy, the FCG vectors (x twice in FP64, p twice in
     FP32), the Galerkin scratch and the returned field during the solve, with
@@ -93,13 +93,12 @@ def footprint_bytes(depth: int, points: int) -> int:
     N = n ** 3
     lib = nat.lib()
     inputs = 4 * 24 * points
-    splat_ws = int(lib.pb_splat_workspace_size(max(points, 1), n))
-    splat = 6 * 8 * N + splat_ws
+    splat_ws = int(lib.pb_splat_assemble_workspace_size(max(points, 1), n))
     solve = 3 * 8 * N + hierarchy_bytes(n) + 2 * 8 * N + 2 * 4 * N + solver32.galerkin_scratch_bytes(n) + 8 * N
     extract = int(lib.pb_extract_workspace_size(n)) + 256 * n * n
     # the splat's workspace is counted in both phases: the caching allocator may
     # keep its block resident into the solve
-    return int(inputs + splat_ws + max(6 * 8 * N, solve + extract))
+    return int(inputs + splat_ws + max(3 * 8 * N, solve + extract))
 
 
 @dataclass
