@@ -4,6 +4,9 @@
 // same order (-fmad=false): s = ((((x- + x+) + y-) + y+) + z-) + z+ with absent
 // neighbours adding +0.0 (a sum that starts from +0.0 never becomes -0.0, so
 // adding +0.0 changes no bit), then (rhs + s h^-2) / diagonal.
+#include <map>
+#include <mutex>
+
 #include "common.cuh"
 
 namespace pb {
@@ -80,8 +83,11 @@ struct Around {
         at[4] = z > 0 ? (i - N * N) >> 1 : none;
         at[5] = z + 1 < N ? (i + N * N) >> 1 : none;
     }
-    __device__ __forceinline__ double sum(const double* v) const {  // v: the other colour
-        return 0.0 + (((((v[at[0]] + v[at[1]]) + v[at[2]]) + v[at[3]]) + v[at[4]]) + v[at[5]]);
+    // v: the other colour.  The reference's sum starts from +0.0, so it is +0.0 where six -0.0 meet: the right-hand
+    // sides here are never -0.0 (restricted sums start from +0.0, the finest one is read as 0.0 + rhs), and
+    // rhs + s h^-2 is then the same for either zero.
+    __device__ __forceinline__ double sum(const double* v) const {
+        return ((((v[at[0]] + v[at[1]]) + v[at[2]]) + v[at[3]]) + v[at[4]]) + v[at[5]];
     }
 };
 
@@ -89,7 +95,7 @@ template <int N>
 __device__ __forceinline__ void tail_update(Tail<N>& L, int colour, int p, const Around<N>& a) {
     const double h2 = (double)(N - 1) * (double)(N - 1);
     const double s = a.sum(L.sol[1 - colour]), d = L.diag[colour][p];
-    if (d > 1.0e-30) L.sol[colour][p] = divide(L.rhs[colour][p] + s * h2, d, L.inv[colour][p]);
+    if (d > 1.0e-30) L.sol[colour][p] = divide(__fma_rn(s, h2, L.rhs[colour][p]), d, L.inv[colour][p]);  // s h2 is exact
 }
 
 // Sweeps of level N; every thread below kThreads takes part.
@@ -228,7 +234,7 @@ __device__ __forceinline__ void tail_cycle(TailStack<N>& S, double* res, int pre
 }
 
 struct TailArgs {
-    const double* screens[4];  // top level first
+    const double* screens[5];  // top level first
     const double* rhs;         // of the top level
     double* sol;               // of the top level: the iterate, or (zero_start) written only
     double pw;
@@ -241,7 +247,7 @@ __global__ void __launch_bounds__(kTailThreads) tail_kernel(const TailArgs a) {
     TailSmem<N>& S = *reinterpret_cast<TailSmem<N>*>(raw);
     tail_setup<N>(S.stack, a.screens, a.pw);
     for (int i = threadIdx.x; i < Tail<N>::kNodes; i += kTailThreads) {
-        S.stack.level.rhs[i & 1][i >> 1] = a.rhs[i];
+        S.stack.level.rhs[i & 1][i >> 1] = 0.0 + a.rhs[i];
         S.stack.level.sol[i & 1][i >> 1] = a.zero_start ? 0.0 : a.sol[i];
     }
     __syncthreads();
@@ -252,7 +258,299 @@ __global__ void __launch_bounds__(kTailThreads) tail_kernel(const TailArgs a) {
     for (int i = threadIdx.x; i < Tail<N>::kNodes; i += kTailThreads) a.sol[i] = S.stack.level.sol[i & 1][i >> 1];
 }
 
-static bool tail_side(int64_t n) { return n == 17 || n == 9 || n == 5 || n == 3; }
+// ---- levels 33 and 17 over a cluster of 16 blocks ---------------------------------
+//
+// 33^3 does not fit one block, and as grid launches its twelve one-colour passes,
+// restriction and prolongation take 41 us a cycle, nearly all of it launch latency;
+// 17^3 in one block is bound by that SM's shared-memory accesses (19 us).  Here a
+// cluster of 16 blocks keeps both levels in distributed shared memory as z slabs
+// (two planes of 33^3 and one of 17^3 each, the last block one more), a block holds
+// a copy of the plane on either side of its slab, and an update of a slab's first or
+// last plane is stored to the neighbour's copy too; a phase then ends with one
+// cluster barrier.  The levels below run on block 0 as above.  A node's index,
+// colour and place follow the rule of the tail with the block's own even origin.
+// Measured on B200: a V(3,3) cycle from 33^3 down 124 -> 69 us.
+constexpr int kClusterBlocks = 16, kClusterThreads = 832;  // 1634 nodes of a colour (last block) in two rounds
+
+template <int N, int PLANES>
+struct Slab {
+    static constexpr int kNN = N * N, kSol = ((PLANES + 2) * kNN + 3) / 2, kOwn = (PLANES * kNN + 3) / 2;
+    double sol[2][kSol + 1];  // the last entry stays +0.0: an absent x or y neighbour; absent planes stay +0.0 too
+    double rhs[2][kOwn];
+    double diag[2][kOwn];
+    double inv[2][kOwn];
+};
+
+// The planes [first, last) of block `rank`, and the even origin of its node indices (below plane first - 1).
+template <int N>
+struct SlabPlace {
+    static constexpr int kNN = N * N, kStep = (N - 1) / kClusterBlocks;
+    int first, last, origin, own;  // own: packed index of the slab's first pair of nodes
+    __device__ __forceinline__ explicit SlabPlace(int rank)
+        : first(kStep * rank), last(rank + 1 < kClusterBlocks ? first + kStep : N),
+          origin(((first - 1) * kNN) & ~1), own((first * kNN - origin) >> 1) {}
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The address in block `rank` of this block's shared variable.
+__device__ __forceinline__ uint32_t remote_address(const void* local, uint32_t rank) {
+    uint32_t out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+    return out;
+}
+__device__ __forceinline__ void remote_store(uint32_t address, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(address), "d"(v) : "memory");
+}
+__device__ __forceinline__ double remote_load(uint32_t address) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(address) : "memory");
+    return v;
+}
+
+// Stores node i's value to the neighbour's copy if its plane is the slab's first or last.
+template <int N, int PLANES>
+__device__ __forceinline__ void slab_share(Slab<N, PLANES>& L, const SlabPlace<N>& at, int rank, int i, int z,
+                                           double value) {
+    if (z == at.first && rank > 0) {
+        const int li = i - SlabPlace<N>(rank - 1).origin;
+        remote_store(remote_address(&L.sol[li & 1][li >> 1], rank - 1), value);
+    }
+    if (z == at.last - 1 && rank + 1 < kClusterBlocks) {
+        const int li = i - SlabPlace<N>(rank + 1).origin;
+        remote_store(remote_address(&L.sol[li & 1][li >> 1], rank + 1), value);
+    }
+}
+
+// The neighbours' sum at local node li (global (x, y)), in the reference's order.
+template <int N, int PLANES>
+__device__ __forceinline__ double slab_sum(const Slab<N, PLANES>& L, int li, int x, int y) {
+    const double* v = L.sol[(li & 1) ^ 1];
+    constexpr int none = Slab<N, PLANES>::kSol;
+    const double a = v[x > 0 ? (li - 1) >> 1 : none], b = v[x + 1 < N ? (li + 1) >> 1 : none];
+    const double c = v[y > 0 ? (li - N) >> 1 : none], d = v[y + 1 < N ? (li + N) >> 1 : none];
+    const double e = v[(li - N * N) >> 1], f = v[(li + N * N) >> 1];
+    return ((((a + b) + c) + d) + e) + f;
+}
+
+template <int N, int PLANES>
+__device__ __forceinline__ void slab_relax(Slab<N, PLANES>& L, const SlabPlace<N>& at, int rank, int sweeps) {
+    constexpr int NN = N * N;
+    const double h2 = (double)(N - 1) * (double)(N - 1);
+    for (int phase = 0; phase < 2 * sweeps; ++phase) {
+        const int begin = at.first * NN, i0 = begin + ((begin ^ phase) & 1);
+        for (int i = i0 + 2 * (int)threadIdx.x; i < at.last * NN; i += 2 * kClusterThreads) {
+            const int row = i / N, x = i - row * N, z = row / N, y = row - z * N;
+            const int li = i - at.origin, c = li & 1, p = (li >> 1) - at.own;
+            const double d = L.diag[c][p];
+            if (d > 1.0e-30) {
+                const double s = slab_sum(L, li, x, y);
+                const double value = divide(__fma_rn(s, h2, L.rhs[c][p]), d, L.inv[c][p]);
+                L.sol[c][li >> 1] = value;
+                slab_share(L, at, rank, i, z, value);
+            }
+        }
+        cluster_barrier();
+    }
+}
+
+// Residuals of the slab: out(plane, index in the plane, value).
+template <int N, int PLANES, typename Out>
+__device__ __forceinline__ void slab_residual(const Slab<N, PLANES>& L, const SlabPlace<N>& at, Out&& out) {
+    constexpr int NN = N * N;
+    const double h2 = (double)(N - 1) * (double)(N - 1);
+    for (int i = at.first * NN + (int)threadIdx.x; i < at.last * NN; i += kClusterThreads) {
+        const int row = i / N, x = i - row * N, z = row / N, y = row - z * N;
+        const int li = i - at.origin, c = li & 1, p = (li >> 1) - at.own;
+        const double s = slab_sum(L, li, x, y);
+        out(z, i - z * NN, L.rhs[c][p] - (L.diag[c][p] * L.sol[c][li >> 1] - s * h2));
+    }
+}
+
+// x += P coarse at every node of the slab (capi.mojo:677-742), coarse(x, y, z) giving the coarse values.
+template <int N, int PLANES, typename Coarse>
+__device__ __forceinline__ void slab_prolong(Slab<N, PLANES>& L, const SlabPlace<N>& at, int rank, Coarse&& coarse) {
+    constexpr int NN = N * N, C = (N + 1) / 2;
+    for (int i = at.first * NN + (int)threadIdx.x; i < at.last * NN; i += kClusterThreads) {
+        const int row = i / N, x = i - row * N, z = row / N, y = row - z * N;
+        const int x0 = x / 2, y0 = y / 2, z0 = z / 2;
+        const int x1 = min(x0 + 1, C - 1), y1 = min(y0 + 1, C - 1), z1 = min(z0 + 1, C - 1);
+        const double tx = (x & 1) ? 0.5 : 0.0, ty = (y & 1) ? 0.5 : 0.0, tz = (z & 1) ? 0.5 : 0.0;
+        // planes z1 beyond the copies are read only with weight 0: keep to z0 there
+        const int zb = (z & 1) ? z1 : z0;
+        const double c00 = coarse(x0, y0, z0) * (1.0 - tx) + coarse(x1, y0, z0) * tx;
+        const double c10 = coarse(x0, y1, z0) * (1.0 - tx) + coarse(x1, y1, z0) * tx;
+        const double c01 = coarse(x0, y0, zb) * (1.0 - tx) + coarse(x1, y0, zb) * tx;
+        const double c11 = coarse(x0, y1, zb) * (1.0 - tx) + coarse(x1, y1, zb) * tx;
+        const double c0 = c00 * (1.0 - ty) + c10 * ty;
+        const double c1 = c01 * (1.0 - ty) + c11 * ty;
+        const int li = i - at.origin, c = li & 1;
+        const double value = L.sol[c][li >> 1] + (c0 * (1.0 - tz) + c1 * tz);
+        L.sol[c][li >> 1] = value;
+        slab_share(L, at, rank, i, z, value);
+    }
+    cluster_barrier();
+}
+
+template <int N, int PLANES>
+__device__ __forceinline__ void slab_setup(Slab<N, PLANES>& L, const SlabPlace<N>& at,
+                                           const double* __restrict__ screen, double pw) {
+    constexpr int NN = N * N;
+    const double h2 = (double)(N - 1) * (double)(N - 1);
+    for (int k = threadIdx.x; k < 2 * (Slab<N, PLANES>::kSol + 1); k += kClusterThreads) (&L.sol[0][0])[k] = 0.0;
+    for (int i = at.first * NN + (int)threadIdx.x; i < at.last * NN; i += kClusterThreads) {
+        const int row = i / N, x = i - row * N, z = row / N, y = row - z * N;
+        const int degree = (x > 0) + (x + 1 < N) + (y > 0) + (y + 1 < N) + (z > 0) + (z + 1 < N);
+        const int li = i - at.origin, c = li & 1, p = (li >> 1) - at.own;
+        const double d = (double)degree * h2 + pw * screen[i] * h2;
+        L.diag[c][p] = d;
+        L.inv[c][p] = reciprocal(d);
+    }
+}
+
+struct ClusterSmem {
+    Slab<33, 3> fine;
+    Slab<17, 2> mid;
+    union {
+        double residual33[4][33 * 33];  // planes first - 1 .. last - 1 of this block's slab
+        double residual[17 * 17 * 17];  // block 0: of 17^3, then of the levels below
+    };
+    TailStack<9> below;  // block 0
+};
+
+__global__ void __launch_bounds__(kClusterThreads) cluster_kernel(const TailArgs a) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    ClusterSmem& S = *reinterpret_cast<ClusterSmem*>(raw);
+    constexpr int N = 33, M = 17, NN = N * N, MM = M * M;
+    const int rank = (int)blockIdx.x, tid = (int)threadIdx.x;
+    const SlabPlace<N> at(rank);
+    const SlabPlace<M> mid(rank);
+    slab_setup(S.fine, at, a.screens[0], a.pw);
+    slab_setup(S.mid, mid, a.screens[1], a.pw);
+    if (rank == 0 && tid < kTailThreads) tail_setup<9>(S.below, a.screens + 2, a.pw);
+    cluster_barrier();  // every copy is zero before values are shared
+    for (int i = at.first * NN + tid; i < at.last * NN; i += kClusterThreads) {
+        const int li = i - at.origin, c = li & 1;
+        S.fine.rhs[c][(li >> 1) - at.own] = 0.0 + a.rhs[i];
+        if (!a.zero_start) {
+            const double value = a.sol[i];
+            S.fine.sol[c][li >> 1] = value;
+            slab_share(S.fine, at, rank, i, i / NN, value);
+        }
+    }
+    cluster_barrier();
+    for (int cycle = 0; cycle < a.cycles; ++cycle) {
+        slab_relax(S.fine, at, rank, a.pre);
+        // residual of 33^3; the slab's last plane also to the block above, which restricts from it.  17^3 starts at
+        // zero, its copies too, before the barrier that lets the neighbours share
+        slab_residual(S.fine, at, [&](int z, int k, double r) {
+            S.residual33[z - at.first + 1][k] = r;
+            if (z == at.last - 1 && rank + 1 < kClusterBlocks) remote_store(remote_address(&S.residual33[0][k], rank + 1), r);
+        });
+        for (int k = tid; k < 2 * (Slab<M, 2>::kSol + 1); k += kClusterThreads) (&S.mid.sol[0][0])[k] = 0.0;
+        cluster_barrier();
+        for (int i = mid.first * MM + tid; i < mid.last * MM; i += kClusterThreads) {  // capi.mojo:557-673
+            const int row = i / M, x = i - row * M, z = row / M, y = row - z * M;
+            double sum = 0.0, weight = 0.0;
+#pragma unroll 1
+            for (int oz = -1; oz <= 1; ++oz)
+#pragma unroll
+                for (int oy = -1; oy <= 1; ++oy)
+#pragma unroll
+                    for (int ox = -1; ox <= 1; ++ox) {
+                        const int zz = 2 * z + oz, yy = 2 * y + oy, xx = 2 * x + ox;
+                        const double w = (oz ? 1.0 : 2.0) * (oy ? 1.0 : 2.0) * (ox ? 1.0 : 2.0);
+                        if ((unsigned)zz < N && (unsigned)yy < N && (unsigned)xx < N) {
+                            sum += S.residual33[zz - at.first + 1][yy * N + xx] * w;
+                            weight += w;
+                        }
+                    }
+            const int li = i - mid.origin;
+            S.mid.rhs[li & 1][(li >> 1) - mid.own] = sum / weight;
+        }
+        __syncthreads();
+        slab_relax(S.mid, mid, rank, a.pre);
+        // every block is past its restriction: block 0's residual buffer is free for 17^3's
+        slab_residual(S.mid, mid, [&](int z, int k, double r) {
+            remote_store(remote_address(&S.residual[z * MM + k], 0), r);
+        });
+        cluster_barrier();
+        if (rank == 0 && tid < kTailThreads) {
+            tail_restrict<M, 9>(S.residual, S.below.level);
+            tail_barrier<M>();
+            if (tid < Tail<9>::kThreads) tail_cycle<9>(S.below, S.residual, a.pre, a.post);
+        }
+        cluster_barrier();
+        slab_prolong(S.mid, mid, rank, [&](int x, int y, int z) {
+            const int j = (z * 9 + y) * 9 + x;
+            return remote_load(remote_address(&S.below.level.sol[j & 1][j >> 1], 0));
+        });
+        slab_relax(S.mid, mid, rank, a.post);
+        slab_prolong(S.fine, at, rank, [&](int x, int y, int z) {
+            const int li = (z * M + y) * M + x - mid.origin;
+            return S.mid.sol[li & 1][li >> 1];
+        });
+        slab_relax(S.fine, at, rank, a.post);
+    }
+    for (int i = at.first * NN + tid; i < at.last * NN; i += kClusterThreads) {
+        const int li = i - at.origin;
+        a.sol[i] = S.fine.sol[li & 1][li >> 1];
+    }
+    cluster_barrier();  // no block leaves while another may still store to it
+}
+
+static int launch_cluster(const TailArgs& a, cudaStream_t s, bool only_ask, bool* possible) {
+    static_assert(sizeof(ClusterSmem) <= 227 * 1024, "one block's shared memory");
+    const void* kernel = (const void*)cluster_kernel;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(kClusterBlocks);
+    config.blockDim = dim3(kClusterThreads);
+    config.dynamicSmemBytes = sizeof(ClusterSmem);
+    config.stream = s;
+    cudaLaunchAttribute attribute = {};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = kClusterBlocks;
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (only_ask) {
+        int clusters = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &config);
+        *possible = e == cudaSuccess && clusters >= 1;
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return PB_OK;
+    }
+    PB_CHECK_CUDA(e, "cluster_kernel attributes");
+    void* args[] = {const_cast<TailArgs*>(&a)};
+    PB_CHECK_CUDA(cudaLaunchKernelExC(&config, kernel, args), "cluster_kernel");
+    PB_CHECK_LAUNCH("cluster_kernel");
+    return PB_OK;
+}
+
+// Whether this device can place a cluster of 16 such blocks (asked once per device).
+static bool cluster_possible() {
+    static std::mutex mu;
+    static std::map<int, bool> known;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(device);
+    if (it == known.end()) {
+        bool possible = false;
+        (void)launch_cluster(TailArgs{}, nullptr, true, &possible);
+        it = known.emplace(device, possible).first;
+    }
+    return it->second;
+}
+
+static bool tail_side(int64_t n) { return n == 17 || n == 9 || n == 5 || n == 3 || (n == 33 && cluster_possible()); }
 
 template <int N>
 static int launch_tail_n(const TailArgs& a, cudaStream_t s) {
@@ -267,6 +565,7 @@ static int launch_tail_n(const TailArgs& a, cudaStream_t s) {
 
 static int launch_tail(int64_t n, const TailArgs& a, cudaStream_t s) {
     switch (n) {
+        case 33: return launch_cluster(a, s, false, nullptr);
         case 17: return launch_tail_n<17>(a, s);
         case 9: return launch_tail_n<9>(a, s);
         case 5: return launch_tail_n<5>(a, s);
@@ -487,7 +786,7 @@ __global__ void __launch_bounds__(256, 5) split_relax_kernel(Split g, double* __
             s0 += above.x;
             s1 += above.y;
         }
-        const double a0 = rhs.x + s0 * v.h2, a1 = rhs.y + s1 * v.h2;
+        const double a0 = __fma_rn(s0, v.h2, rhs.x), a1 = __fma_rn(s1, v.h2, rhs.y);  // s h2 is exact: h2 = 4^k
         const int degree = degree_y + (z > 0) + (z + 1 < n);
         const bool x_face = k_face && !odd;
         double2 q;
