@@ -260,6 +260,13 @@ int pb_refine_start_f64(const double *rhs, const double *screen, int64_t n, doub
                         double *rhs_copy, double *screen_copy, double *x0, float *D, float *invD, float *weights,
                         float *r32, double *norm2, double *bnorm, void *workspace, size_t workspace_bytes,
                         void *stream);
+/* The same, and where screen and rhs are not zero (pb_occupancy_size bytes, 4-byte aligned) for
+ * the sparse passes below.  The words' layout is the library's own. */
+size_t pb_occupancy_size(int64_t n);
+int pb_refine_start_sparse_f64(const double *rhs, const double *screen, int64_t n, double point_weight,
+                               double *rhs_copy, double *screen_copy, double *x0, float *D, float *invD,
+                               float *weights, float *r32, void *occupancy, double *norm2, double *bnorm,
+                               void *workspace, size_t workspace_bytes, void *stream);
 /* FP64 flexible conjugate gradients, FCG(1), preconditioned by the FP32
  * V-cycle, in two passes per iteration (no counterpart in the reference, which
  * repeats V-cycles, core.py:274-285).  Device scalars scal[0..4]: (p, Ap),
@@ -278,6 +285,16 @@ int pb_fcg_direction_f64(const float *z, const float *p0, const float *p1, const
 int pb_fcg_update_f64(const float *z, float *p0, float *p1, double *x0, double *x1, const double *b,
                       const double *screen, float *r32, int64_t n, double point_weight, double *scal,
                       const int *flags, void *workspace, size_t workspace_bytes, void *stream);
+/* The two passes reading b and screen only where `occupancy`, as pb_refine_start_sparse_f64
+ * wrote it for them, says that they are not zero (NULL: everywhere); the same results. */
+int pb_fcg_direction_sparse_f64(const float *z, const float *p0, const float *p1, const float *r32,
+                                const double *screen, const void *occupancy, int64_t n, double point_weight,
+                                double *scal, const int *flags, void *workspace, size_t workspace_bytes,
+                                void *stream);
+int pb_fcg_update_sparse_f64(const float *z, float *p0, float *p1, double *x0, double *x1, const double *b,
+                             const double *screen, const void *occupancy, float *r32, int64_t n,
+                             double point_weight, double *scal, const int *flags, void *workspace,
+                             size_t workspace_bytes, void *stream);
 /* One red-black Gauss-Seidel sweep (colour 0 then colour 1), out of place,
  * with TMA-staged planes (n = 2^k + 1 >= 33): mode 0 from e_in, mode 1 from
  * zero (e_in unused).  z_chunk <= 0 picks one.  A bounded wait that gives up
@@ -289,6 +306,9 @@ int pb_sweep_tma_f32(const float *e_in, float *e_out, const float *rhs, const fl
  * pb_level27_finish_f32 below).  Replaces mpr_prolong_add_f64
  * (capi.mojo:677-742) inside the FP32 cycle. */
 int pb_prolong_fac_f32(const float *coarse, float *fine, const float *weights, int64_t fine_n, void *stream);
+/* The same, reading weights only where `occupancy` (pb_refine_start_sparse_f64) has screening: 1 elsewhere. */
+int pb_prolong_fac_sparse_f32(const float *coarse, float *fine, const float *weights, const void *occupancy,
+                              int64_t fine_n, void *stream);
 /* Device-driven iteration (no counterpart in the reference).  Begin: a graph
  * with one WHILE conditional node; `stream` is captured into its body until
  * pb_loop_capture_end, which instantiates it.  The body's last launch must be
@@ -445,7 +465,7 @@ int pb_hierarchy_setup_f32(int64_t levels, const int64_t *sides, const void *con
  * Operands per kind (p = padded FP32 level arrays, d = dense):
  *   SWEEP / SWEEP_ZERO     e_in (ignored from zero), e_out, rhs, 1/D, status word;
  *                          z_chunk <= 0: whole planes per block (sides 2^k + 1 >= 33)
- *   PROLONG32              coarse, fine, weights               (pb_prolong_fac_f32)
+ *   PROLONG32              coarse, fine, weights, [occupancy]  (pb_prolong_fac_sparse_f32)
  *   RESIDUAL_RESTRICT32    e, rhs, D, weights, coarse rhs      (pb_residual_restrict_f32)
  *   RELAX27P / _ZERO       e_prev, e_next, rhs, h0, h1, inv0, inv1   (pb_relax27p_f32)
  *   RESIDUAL27P            e, rhs, h0, h1, inv0, inv1, weights, res
@@ -453,7 +473,7 @@ int pb_hierarchy_setup_f32(int64_t levels, const int64_t *sides, const void *con
  *   COARSE27               image, rhs, e; aux = pre, post, inner; one block per
  *                          grid, every grid of the launch of the same first side
  *                          (pass it as first_side to pb_batch_launch)
- *   FCG_DIRECTION          z, p0, p1, r32, screen (d), partials; aux[0] = point
+ *   FCG_DIRECTION          z, p0, p1, r32, screen (d), partials, [occupancy]; aux[0] = point
  *                          weight as the bits of a double
  *   FCG_DIRECTION_FINISH   partials, the cloud's scalars; aux[0] = the cloud's
  *                          pb_batch_fcg_blocks(n, 0)
@@ -503,10 +523,11 @@ int pb_batch_loop_condition(unsigned long long handle, const double *scal, const
  *   SWEEP_Z_CHUNK          planes per block of pb_sweep_tma_f32 when its z_chunk <= 0
  *   RESTRICT_PLANES        coarse planes per block of pb_residual_restrict_f32 (default 4)
  *   PROLONG_PLANES         fine planes per block of pb_prolong_fac_f32
- *   FCG_DIRECTION_PLANES   planes per block of pb_fcg_direction_f64 (default 24; 8 at n <= 129, 4 at n <= 65; at least 4)
- *   FCG_UPDATE_PLANES      planes per block of pb_fcg_update_f64 (as FCG_DIRECTION_PLANES)
- *   FCG_DIRECTION_VARIANT  register budget of pb_fcg_direction_f64: 0 = 4 resident
- *                          blocks per SM, 1 = 6, 2 = 8
+ *   FCG_DIRECTION_PLANES   planes per block of pb_fcg_direction_f64 (default 24; 12 at n <= 257, 8 at n <= 129,
+ *                          4 at n <= 65; at least 4)
+ *   FCG_UPDATE_PLANES      planes per block of pb_fcg_update_f64 (default 24; 8 at n <= 129, 4 at n <= 65; at least 4)
+ *   FCG_DIRECTION_VARIANT  register budget of pb_fcg_direction_f64: 0 = 6 resident
+ *                          blocks of 128 threads per SM, 1 = 4, 2 = 8
  *   RESTRICT_VARIANT       pb_residual_restrict_f32: 0 (and 1) = 256 threads per block;
  *                          2 = the FP32 cycle calls pb_residual_restrict_tma_f32 instead;
  *                          3 = 320 threads per block

@@ -72,9 +72,13 @@ _SIGNATURES = {
     "pb_defect_workspace_size": ([I], S),
     "pb_defect_f64": ([P, P, P, P, P, I, F, P, P, P, P, S, P], C),
     "pb_refine_start_workspace_size": ([I], S),
+    "pb_occupancy_size": ([I], S),
     "pb_refine_start_f64": ([P, P, I, F, P, P, P, P, P, P, P, P, P, P, S, P], C),
+    "pb_refine_start_sparse_f64": ([P, P, I, F, P, P, P, P, P, P, P, P, P, P, P, S, P], C),
     "pb_fcg_workspace_size": ([I], S),
     "pb_fcg_direction_f64": ([P, P, P, P, P, I, F, P, P, P, S, P], C),
+    "pb_fcg_direction_sparse_f64": ([P, P, P, P, P, P, I, F, P, P, P, S, P], C),
+    "pb_fcg_update_sparse_f64": ([P, P, P, P, P, P, P, P, P, I, F, P, P, P, S, P], C),
     "pb_fcg_update_f64": ([P, P, P, P, P, P, P, P, I, F, P, P, P, S, P], C),
     "pb_loop_capture_begin": ([P, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_ulonglong)], C),
     "pb_loop_condition": ([ctypes.c_ulonglong, P, P, P, I, P, P], C),
@@ -84,6 +88,7 @@ _SIGNATURES = {
     "pb_note_launches": ([ctypes.c_longlong], C),
     "pb_sweep_tma_f32": ([P, P, P, P, I, I, I, P, P], C),
     "pb_prolong_fac_f32": ([P, P, P, I, P], C),
+    "pb_prolong_fac_sparse_f32": ([P, P, P, P, I, P], C),
     "pb_extract_workspace_size": ([I], S),
     "pb_mesh_normals_workspace_size": ([I, I], S),
     "pb_mesh_normals_count_f64": ([P, I, P, I, P, P, S, P], C),

@@ -316,8 +316,8 @@ class BatchSolver:
             add(RELAX27P, [(k, lv[k].n, (lv[k].ea.data_ptr(), lv[k].eb.data_ptr(), lv[k].rhs.data_ptr(),
                                          *lv[k].packed_ptrs())) for k in idx])
         # level 0 up: prolongation into ea, sweeps ea -> eb -> ea
-        add(PROLONG32, [(k, cl[k].n, (result(k, 1).data_ptr(), l0[k].ea.data_ptr(), l0[k].weights.data_ptr()))
-                        for k in range(K)])
+        add(PROLONG32, [(k, cl[k].n, (result(k, 1).data_ptr(), l0[k].ea.data_ptr(), l0[k].weights.data_ptr(),
+                                      cl[k].h.occupancy.data_ptr())) for k in range(K)])
         add(SWEEP, [(k, cl[k].n, (l0[k].ea.data_ptr(), l0[k].eb.data_ptr(), l0[k].rhs.data_ptr(),
                                   l0[k].invD.data_ptr(), st)) for k in range(K)], z_chunk=z_chunk)
         add(SWEEP, [(k, cl[k].n, (l0[k].eb.data_ptr(), l0[k].ea.data_ptr(), l0[k].rhs.data_ptr(),
@@ -326,13 +326,15 @@ class BatchSolver:
         part = [self.partials[int(self.part_offsets[k]):].data_ptr() for k in range(K)]
         scal = [self.scal[k].data_ptr() for k in range(K)]
         add(FCG_DIRECTION, [(k, cl[k].n, (l0[k].ea.data_ptr(), cl[k].ps[0].data_ptr(), cl[k].ps[1].data_ptr(),
-                                          l0[k].rhs.data_ptr(), screen[k].data_ptr(), part[k]), (_bits(pws[k]),))
+                                          l0[k].rhs.data_ptr(), screen[k].data_ptr(), part[k],
+                                          cl[k].h.occupancy.data_ptr()), (_bits(pws[k]),))
                             for k in range(K)])
         add(FCG_DIRECTION_FINISH, [(k, cl[k].n, (part[k], scal[k]), (int(lib.pb_batch_fcg_blocks(cl[k].n, 0)),))
                                    for k in range(K)])
         add(FCG_UPDATE, [(k, cl[k].n, (l0[k].ea.data_ptr(), cl[k].ps[0].data_ptr(), cl[k].ps[1].data_ptr(),
                                        cl[k].xs[0].data_ptr(), cl[k].xs[1].data_ptr(), rhs[k].data_ptr(),
-                                       screen[k].data_ptr(), l0[k].rhs.data_ptr(), scal[k], part[k]),
+                                       screen[k].data_ptr(), l0[k].rhs.data_ptr(), scal[k], part[k],
+                                       cl[k].h.occupancy.data_ptr()),
                           (_bits(pws[k]),)) for k in range(K)])
         add(FCG_SUM, [(k, cl[k].n, (part[k], self.scal[k, 4:].data_ptr()),
                        (int(lib.pb_batch_fcg_blocks(cl[k].n, 1)),)) for k in range(K)])

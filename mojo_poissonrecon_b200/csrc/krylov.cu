@@ -30,17 +30,19 @@
 
 #include "batch.cuh"
 #include "common.cuh"
+#include "occupancy.cuh"
 
 namespace pb {
 namespace fcg {
 
-// pass 1: 256 (x, y) columns per block; both passes planes_of(n) planes deep unless
-// the autotuner chose otherwise (257^3, pass 1: 16 planes 82 us, 24 planes 78).  A
-// block walks its planes one after another, so small grids take fewer planes for
-// more blocks: at 65^3, 24 planes leave 81 blocks of pass 2 for 148 SMs (26.6 us),
-// 4 planes 459.  Partial sums are sized for the shallowest depth a launch may use, kMinTZ.
-constexpr int kTZ = 24, kMinTZ = 4, kThreads = 256;
-__host__ __device__ constexpr int planes_of(int n) { return n <= 65 ? 4 : n <= 129 ? 8 : kTZ; }
+// Planes per block of the two passes unless the autotuner chose otherwise.  A block
+// walks its planes one after another, so small grids take fewer planes for more
+// blocks: at 65^3, 24 planes leave 81 blocks of pass 2 for 148 SMs (26.6 us), 4 planes
+// 459; pass 1 at 257^3 takes 85 us with 24 planes and 79 with 12, at 513^3 417 and 443.
+// Partial sums are sized for the shallowest depth a launch may use, kMinTZ.
+constexpr int kTZ = 24, kMinTZ = 4, kThreads = 128;
+__host__ __device__ constexpr int update_planes_of(int n) { return n <= 65 ? 4 : n <= 129 ? 8 : kTZ; }
+__host__ __device__ constexpr int direction_planes_of(int n) { return n <= 65 ? 4 : n <= 129 ? 8 : n <= 257 ? 12 : kTZ; }
 
 // Pass 2 tile: 32 x 8 nodes per block, kTZ planes deep.
 constexpr int kUX = 32, kUY = 8, kUThreads = kUX * kUY;
@@ -87,6 +89,20 @@ __device__ __forceinline__ int64_t block_index() {
 // instantiations of a body (single and grouped launches, planes known or not) may
 // fuse differently, and a cloud would differ in the last bits alone and in a batch.
 
+constexpr int kW = 4;  // x per thread of pass 1
+template <bool ALIGNED>  // the padded arrays start on 16-byte boundaries, and so do their rows
+__device__ __forceinline__ float4 wide(const float* at) {
+    if constexpr (ALIGNED) return *reinterpret_cast<const float4*>(at);
+    return make_float4(at[0], at[1], at[2], at[3]);
+}
+static bool aligned16(const void* a, const void* b) { return ((uintptr_t)a | (uintptr_t)b) % 16 == 0; }
+__device__ __forceinline__ void widen(float4 f, double (&d)[kW]) {
+    d[0] = (double)f.x;
+    d[1] = (double)f.y;
+    d[2] = (double)f.z;
+    d[3] = (double)f.w;
+}
+
 // (A v)_i: degree and screening at the node, its value and its neighbours' sum s.
 __device__ __forceinline__ double applied(int degree, double pw, double screen, double h2, double value, double s) {
     return __fma_rn(__fma_rn(__dmul_rn(pw, screen), h2, __dmul_rn((double)degree, h2)), value, -__dmul_rn(s, h2));
@@ -94,49 +110,74 @@ __device__ __forceinline__ double applied(int degree, double pw, double screen, 
 
 // Pass 1: per-block (z, Az), (Az, p_prev), (z, r32), (p_prev, r32); flags[1]
 // (iterations done) selects p_prev = p[it & 1]; flags[0] != 0 on the first step.
-// Each thread marches down its column with z of planes k - 1 and k in
-// registers; the ghosts of the padded z are zero, so the 6-neighbour sum needs
-// no tests.  Compiled for 4 resident blocks per SM (64 registers), which keeps
-// more loads in flight than the occupancy-first default.
-// TZC > 0: the planes per block as a compile-time constant (the built-in kTZ),
-// which lets the compiler unroll the z march; 0: the runtime tz.
-template <int TZC>
+// A thread takes four x of a row (the padded rows start 16-byte aligned) and
+// marches down z with the planes k - 1 and k in registers as doubles; the ghosts of
+// the padded z are zero, so the 6-neighbour sum needs no tests, and the nodes past a
+// row's end add zeros.  Bound by latency and by the conversions to double (16 a cycle
+// and SM), not by memory: one x per thread converts 8 values a node and reads the
+// screen everywhere (513^3: 508 us), four x 5.5 and the screen only where it is
+// not zero (417; two x 495).
+template <bool ALIGNED>
 __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z, Pad g, const float* __restrict__ p0,
                                                     const float* __restrict__ p1, const float* __restrict__ r32,
-                                                    const double* __restrict__ screen, double pw,
+                                                    const double* __restrict__ screen,
+                                                    const uint32_t* __restrict__ occupied, double pw,
                                                     const int* __restrict__ flags, double* __restrict__ part, int tz,
                                                     int bx, int by, int64_t block) {
     __shared__ double shared[4][32];
     const int n = g.n;
-    const unsigned t = bx * kThreads + threadIdx.x;  // flattened over the plane's (x, y): full warps
-    const int y = t < (unsigned)(n * n) ? (int)(t / (unsigned)n) : n, x = (int)(t - (unsigned)y * n);
-    const int tzv = TZC > 0 ? TZC : tz;
-    const int z0 = by * tzv, z1 = min(n, z0 + tzv);
+    const unsigned groups = (unsigned)(n + kW - 1) / kW;
+    const unsigned t = bx * kThreads + threadIdx.x;  // flattened over the plane's (group, y): full warps
+    const int y = (int)(t / groups), x = (int)(t - y * groups) * kW;
+    const int z0 = by * tz, z1 = min(n, z0 + tz);
     const double h = (double)(n - 1), h2 = h * h;
     const bool first = flags[0] != 0;
     const float* __restrict__ pp = (flags[1] & 1) ? p1 : p0;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
-    if (x < n && y < n) {
-        const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
+    if (y < n) {
+        const int degy = (y > 0) + (y + 1 < n);
         const int64_t nn = (int64_t)n * n;
+        const int inside = min(kW, n - x);
         int64_t i = (int64_t)z0 * nn + (int64_t)y * n + x, c = g.at(x, y, z0);
-        float zb = z[c - g.plane], zm = z[c];
-        for (int k = z0; k < z1; ++k, i += nn, c += g.plane) {
-            const float za = z[c + g.plane];  // the ghost plane past the last
-            const double s = (double)z[c - 1] + (double)z[c + 1] + (double)z[c - g.P] + (double)z[c + g.P] +
-                             (double)zb + (double)za;
-            const double zc = (double)zm;
-            zb = zm;
-            zm = za;
-            const int deg = degxy + (k > 0) + (k + 1 < n);
-            const double az = applied(deg, pw, screen[i], h2, zc, s);
-            const double rc = (double)r32[c];
-            v[0] = __fma_rn(zc, az, v[0]);
-            v[2] = __fma_rn(zc, rc, v[2]);
-            if (!first) {
-                const double pv = (double)pp[i];
+        uint32_t some = plane_bits(occupied, n, x, y, z0);
+        double zb[kW], zm[kW];
+        widen(wide<ALIGNED>(z + c - g.plane), zb);
+        widen(wide<ALIGNED>(z + c), zm);
+        for (int k = z0; k < z1; ++k, i += nn, c += g.plane, some >>= 1) {
+            const float4 above = wide<ALIGNED>(z + c + g.plane);  // the ghost plane past the last
+            const float4 front = wide<ALIGNED>(z + c - g.P), back = wide<ALIGNED>(z + c + g.P), res = wide<ALIGNED>(r32 + c);
+            const float left = z[c - 1], right = z[c + kW];
+            float prev[kW] = {};
+            if (!first)
+#pragma unroll
+                for (int j = 0; j < kW; ++j)
+                    if (j < inside) prev[j] = pp[i + j];
+            double sc[kW] = {};
+            if (some & 1u)
+#pragma unroll
+                for (int j = 0; j < kW; ++j)
+                    if (j < inside) sc[j] = screen[i + j];
+            double za[kW], ym[kW], yp[kW], rc[kW];
+            widen(above, za);
+            widen(front, ym);
+            widen(back, yp);
+            widen(res, rc);
+            const int degyz = degy + (k > 0) + (k + 1 < n);
+#pragma unroll
+            for (int j = 0; j < kW; ++j) {
+                const double s = (j > 0 ? zm[j - 1] : (double)left) + (j < kW - 1 ? zm[j + 1] : (double)right) + ym[j] +
+                                 yp[j] + zb[j] + za[j];
+                const int deg = degyz + (j > 0 || x > 0) + (x + j + 1 < n);
+                const double az = applied(deg, pw, sc[j], h2, zm[j], s), pv = (double)prev[j];
+                v[0] = __fma_rn(zm[j], az, v[0]);
                 v[1] = __fma_rn(az, pv, v[1]);
-                v[3] = __fma_rn(pv, rc, v[3]);
+                v[2] = __fma_rn(zm[j], rc[j], v[2]);
+                v[3] = __fma_rn(pv, rc[j], v[3]);
+            }
+#pragma unroll
+            for (int j = 0; j < kW; ++j) {
+                zb[j] = zm[j];
+                zm[j] = za[j];
             }
         }
     }
@@ -148,15 +189,16 @@ __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z,
 
 // MINB: resident blocks per SM the compiler must allow (register budget); the
 // autotuner picks among the compiled variants (PB_TUNE_FCG_DIRECTION_VARIANT).
-template <int MINB, int TZC>
+template <int MINB, bool ALIGNED = true>
 __global__ void __launch_bounds__(kThreads, MINB) direction_sums_kernel(const float* __restrict__ z, Pad g,
                                                                      const float* __restrict__ p0,
                                                                      const float* __restrict__ p1,
                                                                      const float* __restrict__ r32,
-                                                                     const double* __restrict__ screen, double pw,
+                                                                     const double* __restrict__ screen,
+                                                                     const uint32_t* __restrict__ occupied, double pw,
                                                                      const int* __restrict__ flags,
                                                                      double* __restrict__ part, int tz) {
-    direction_sums_body<TZC>(z, g, p0, p1, r32, screen, pw, flags, part, tz, blockIdx.x, blockIdx.y, block_index());
+    direction_sums_body<ALIGNED>(z, g, p0, p1, r32, screen, occupied, pw, flags, part, tz, blockIdx.x, blockIdx.y, block_index());
 }
 
 // Sums pass 1's partials (fixed order) and forms the step's scalars:
@@ -226,12 +268,17 @@ struct Halo {
 // the neighbour sum adds x-, x+, y-, y+, z-, z+ in that order.
 //
 // Each thread copies the values it will read of plane k + RING - 1 (its x, z, p, b
-// and screen, and its halo node's x, z, p) into its own shared-memory slots with
-// cp.async while it works on plane k, so RING - 1 planes of loads are in flight per
-// thread without holding registers (257^3: 168 us against 237 with the loads in
-// registers); a thread only reads its own slots, so cp.async.wait_group suffices
-// (the tile of new iterates keeps its barrier).  RING = 3 by default, 4 as a tuning
-// variant.
+// and screen, the last two where the occupancy words have any, and its halo node's x, z,
+// p) into its own shared-memory slots with cp.async while it works on plane k, so
+// RING - 1 planes of loads are in flight per thread without holding registers; a
+// thread only reads its own slots, so cp.async.wait_group suffices (the tile of new
+// iterates keeps its barrier).  The march is unrolled by the ring, so that slots are
+// constants, and a plane's part of an address is the block's: 155 instructions per 32
+// nodes instead of 225, and bound by the shared-memory pipe (72 %) and issue (64 %).
+// 257^3 157 -> 146 us, 513^3 1240 -> 1013.  Tried: two rows per thread with the loads
+// ahead in registers (200 us at 257^3, it waits on them in order), and whole rows
+// copied 16 bytes at a time for all threads (165 us: fewer wavefronts, more
+// instructions).  RING = 3 by default, 4 as a tuning variant.
 constexpr int kRing = 3;
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
@@ -251,12 +298,13 @@ __device__ __forceinline__ void cp_wait() {
 template <int TZC, int RING = kRing>
 __device__ __forceinline__ void update_residual_prefetch_body(
     const float* __restrict__ z, Pad g, float* p0, float* p1, double* x0, double* x1, const double* __restrict__ b,
-    const double* __restrict__ screen, double pw, const double* __restrict__ scal, const int* __restrict__ flags,
-    float* __restrict__ r32, double* __restrict__ part, int tz, int tile_x, int tile_y, int tile_z, int64_t block) {
+    const double* __restrict__ screen, const uint32_t* __restrict__ occupied, double pw,
+    const double* __restrict__ scal, const int* __restrict__ flags, float* __restrict__ r32,
+    double* __restrict__ part, int tz, int tile_x, int tile_y, int tile_z, int64_t block) {
     static_assert(RING >= 3 && RING <= 4, "two or three planes in flight");
-    __shared__ double tiles[2][kUY + 2][kUX + 2];
-    __shared__ double shared[1][32];
     constexpr int kHalo = 2 * (kUX + kUY);     // the threads tid < kHalo own a halo node
+    __shared__ double tiles[RING][kUY + 2][kUX + 2];
+    __shared__ double shared[1][32];
     __shared__ double rd[RING][3][kUThreads];  // own x, b, screen
     __shared__ double hd[RING][kHalo];         // halo x
     __shared__ float rf[RING][2][kUThreads];   // own z, p
@@ -274,102 +322,104 @@ __device__ __forceinline__ void update_residual_prefetch_body(
     float* __restrict__ pn = odd ? p0 : p1;
     const double* __restrict__ xc = odd ? x1 : x0;
     double* __restrict__ xn = odd ? x0 : x1;
-    const double beta = first ? 0.0 : scal[1], alpha = scal[2];
+    const double minus_beta = first ? 0.0 : -scal[1], alpha = scal[2];
     const int64_t nn = (int64_t)n * n;
-    auto dir_at = [&](int64_t ii, int64_t cc) -> double {
-        double val = (double)z[cc];
-        if (!first) val = __fma_rn(-beta, (double)pp[ii], val);
-        return val;
-    };
-    auto dir_of = [&](float zv, float pv) -> double {  // dir_at from prefetched values
-        double val = (double)zv;
-        if (!first) val = __fma_rn(-beta, (double)pv, val);
-        return val;
-    };
     const Halo hl(tid, bx, by);
     const bool halo_in = hl.inside(n);
     const bool inside = x < n && y < n;
-    const int64_t i0 = inside ? (int64_t)z0 * nn + (int64_t)y * n + x : 0;
-    const int64_t c0 = inside ? g.at(x, y, z0) : 0;
-    const int64_t hi0 = halo_in ? (int64_t)z0 * nn + (int64_t)hl.hy * n + hl.hx : 0;
-    const int64_t hc0 = halo_in ? g.at(hl.hx, hl.hy, z0) : 0;
-    auto issue = [&](int p) {  // plane p's values into slot p % RING, one commit group
-        const int sl = p % RING;
-        const int64_t dz = p - z0;
-        if (inside && p < n && p <= z1) {  // own x, z, p of planes z0 .. z1 (z1: the last plane's upper neighbour)
-            const int64_t ip = i0 + dz * nn, cq = c0 + dz * g.plane;
-            cp_async8(&rd[sl][0][tid], xc + ip);
-            cp_async4(&rf[sl][0][tid], z + cq);
-            if (!first) cp_async4(&rf[sl][1][tid], pp + ip);
-            if (p < z1) {
-                cp_async8(&rd[sl][1][tid], b + ip);
-                cp_async8(&rd[sl][2][tid], screen + ip);
+    // offsets within a plane, dense and padded; the plane's own part is the same for the block
+    const uint32_t e = inside ? (uint32_t)y * n + x : 0u, q = inside ? (uint32_t)(y + 1) * g.P + x + 4 : 0u;
+    const uint32_t he = halo_in ? (uint32_t)hl.hy * n + hl.hx : 0u;
+    const uint32_t hq = halo_in ? (uint32_t)(hl.hy + 1) * g.P + hl.hx + 4 : 0u;
+    // planes of the block where a warp's row of the tile has b or screening
+    const uint32_t some =
+        y < n ? plane_bits(occupied, n, bx, y, z0) & (0xffffffffu >> max(0, 32 - (z1 - z0))) : 0u;
+    // A slot that nothing is copied to holds zeros: nodes outside the domain, and p in the first step.
+    for (int sl = 0; sl < RING; ++sl) {
+        if (!inside) rd[sl][0][tid] = 0.0, rf[sl][0][tid] = 0.0f;
+        if (!inside || first) rf[sl][1][tid] = 0.0f;
+        if (hl.has) {
+            if (!halo_in) hd[sl][tid] = 0.0, hf[sl][0][tid] = 0.0f;
+            if (!halo_in || first) hf[sl][1][tid] = 0.0f;
+        }
+    }
+    // plane k's values into its slot, one commit group; own x, z, p of planes z0 .. z1
+    // (z1: the last plane's upper neighbour), the rest of z0 .. z1 - 1
+    auto issue = [&](auto slot, int k) {
+        constexpr int sl = decltype(slot)::value;
+        const int64_t dense = k * nn, padded = (int64_t)(k + 1) * g.plane;
+        if (inside && k <= z1 && k < n) {
+            cp_async8(&rd[sl][0][tid], xc + dense + e);
+            cp_async4(&rf[sl][0][tid], z + padded + q);
+            if (!first) cp_async4(&rf[sl][1][tid], pp + dense + e);
+            if (k < z1 && ((some >> (k - z0)) & 1u)) {
+                cp_async8(&rd[sl][1][tid], b + dense + e);
+                cp_async8(&rd[sl][2][tid], screen + dense + e);
             }
         }
-        if (halo_in && p < z1) {
-            const int64_t hp = hi0 + dz * nn, hq = hc0 + dz * g.plane;
-            cp_async8(&hd[sl][tid], xc + hp);
-            cp_async4(&hf[sl][0][tid], z + hq);
-            if (!first) cp_async4(&hf[sl][1][tid], pp + hp);
+        if (halo_in && k < z1) {
+            cp_async8(&hd[sl][tid], xc + dense + he);
+            cp_async4(&hf[sl][0][tid], z + padded + hq);
+            if (!first) cp_async4(&hf[sl][1][tid], pp + dense + he);
         }
         cp_commit();
     };
-    issue(z0);
-    issue(z0 + 1);
-    if (RING == 4) issue(z0 + 2);
+    issue(std::integral_constant<int, 0>(), z0);
+    issue(std::integral_constant<int, 1>(), z0 + 1);
+    if (RING == 4) issue(std::integral_constant<int, 2>(), z0 + 2);
     cp_wait<RING - 2>();
-    double dm = 0.0, xm = 0.0, xb = 0.0;
-    if (inside) {
-        const int sl = z0 % RING;
-        dm = dir_of(rf[sl][0][tid], rf[sl][1][tid]);
-        xm = __fma_rn(alpha, dm, rd[sl][0][tid]);
-        xb = z0 > 0 ? __fma_rn(alpha, dir_at(i0 - nn, c0 - g.plane), xc[i0 - nn]) : 0.0;
+    double dm = __fma_rn(minus_beta, (double)rf[0][1][tid], (double)rf[0][0][tid]);
+    double xm = __fma_rn(alpha, dm, rd[0][0][tid]), xb = 0.0;
+    if (inside && z0 > 0) {
+        const int64_t dense = (z0 - 1) * nn + e;
+        double d = (double)z[(int64_t)z0 * g.plane + q];
+        if (!first) d = __fma_rn(minus_beta, (double)pp[dense], d);
+        xb = __fma_rn(alpha, d, xc[dense]);
     }
-    int64_t i = i0, c = c0;
+    // the diagonal without screening, between two planes and at the first or last
     const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
+    const double d_mid = __dmul_rn((double)(degxy + 2), h2), d_end = __dmul_rn((double)(degxy + 1), h2);
     double v[1] = {0.0};
-    for (int k = z0; k < z1; ++k) {
-        issue(k + RING - 1);  // into the slot of plane k - 1, read by this thread alone in the previous step
+    auto step = [&](auto slot, int k) {
+        constexpr int sk = decltype(slot)::value, sn = (sk + 1) % RING;
+        issue(std::integral_constant<int, (sk + RING - 1) % RING>(), k + RING - 1);  // plane k - 1's slot: its reader is this thread
         cp_wait<RING - 2>();  // planes up to k + 1 have landed
-        const int sk = k % RING, sn = (k + 1) % RING;
-        const double hv = halo_in ? __fma_rn(alpha, dir_of(hf[sk][0][tid], hf[sk][1][tid]), hd[sk][tid]) : 0.0;
+        double(*tile)[kUX + 2] = tiles[sk];
+        tile[ty + 1][tx + 1] = xm;
+        if (hl.has)
+            tile[hl.sy][hl.sx] = __fma_rn(
+                alpha, __fma_rn(minus_beta, (double)hf[sk][1][tid], (double)hf[sk][0][tid]), hd[sk][tid]);
         const bool up = k + 1 < n;
-        double da = 0.0, xa = 0.0, bi = 0.0, sc = 0.0;
-        if (inside) {
-            if (up) {
-                da = dir_of(rf[sn][0][tid], rf[sn][1][tid]);
-                xa = __fma_rn(alpha, da, rd[sn][0][tid]);
-            }
-            bi = rd[sk][1][tid];
-            sc = rd[sk][2][tid];
-        }
-        double(*tile)[kUX + 2] = tiles[k & 1];
-        tile[ty + 1][tx + 1] = inside ? xm : 0.0;
-        if (hl.has) tile[hl.sy][hl.sx] = hv;
+        const double da = __fma_rn(minus_beta, (double)rf[sn][1][tid], (double)rf[sn][0][tid]);
+        const double xa = up ? __fma_rn(alpha, da, rd[sn][0][tid]) : 0.0;
         __syncthreads();
         if (inside) {
-            double s = 0.0;
-            s += tile[ty + 1][tx];
-            s += tile[ty + 1][tx + 2];
-            s += tile[ty][tx + 1];
-            s += tile[ty + 2][tx + 1];
-            s += xb;
-            s += xa;
-            const int deg = degxy + (k > 0) + up;
-            PB_GUARD(i, nn * n, kSiteFcgStore) {
-                pn[i] = (float)dm;
-                xn[i] = xm;
+            const double s = tile[ty + 1][tx] + tile[ty + 1][tx + 2] + tile[ty][tx + 1] + tile[ty + 2][tx + 1] + xb + xa;
+            double bi = 0.0, d = up && k > 0 ? d_mid : d_end;
+            if ((some >> (k - z0)) & 1u) {
+                bi = rd[sk][1][tid];
+                d = __fma_rn(__dmul_rn(pw, rd[sk][2][tid]), h2, d);
             }
-            const double r = __dsub_rn(bi, applied(deg, pw, sc, h2, xm, s));
-            PB_GUARD(c, (int64_t)(n + 2) * g.plane, kSiteFcgStore)
-            r32[c] = (float)r;
+            const double r = __dsub_rn(bi, __fma_rn(d, xm, -__dmul_rn(s, h2)));
+            const int64_t dense = k * nn, padded = (int64_t)(k + 1) * g.plane;
+            PB_GUARD(dense + e, nn * n, kSiteFcgStore) {
+                pn[dense + e] = (float)dm;
+                xn[dense + e] = xm;
+            }
+            PB_GUARD(padded + q, (int64_t)(n + 2) * g.plane, kSiteFcgStore)
+            r32[padded + q] = (float)r;
             v[0] = __fma_rn(r, r, v[0]);
-            i += nn;
-            c += g.plane;
         }
         xb = xm;
         xm = xa;
         dm = da;
+    };
+    for (int k = z0; k < z1; k += RING) {  // slots by plane modulo RING, known at compile time
+        step(std::integral_constant<int, 0>(), k);
+        if (k + 1 < z1) step(std::integral_constant<int, 1>(), k + 1);
+        if (k + 2 < z1) step(std::integral_constant<int, 2>(), k + 2);
+        if constexpr (RING == 4)
+            if (k + 3 < z1) step(std::integral_constant<int, 3>(), k + 3);
     }
     cp_wait<0>();
     block_sums<1>(v, shared);
@@ -379,9 +429,10 @@ __device__ __forceinline__ void update_residual_prefetch_body(
 template <int TZC, int RING = kRing>
 __global__ void __launch_bounds__(kUThreads) update_residual_prefetch_kernel(
     const float* __restrict__ z, Pad g, float* p0, float* p1, double* x0, double* x1, const double* __restrict__ b,
-    const double* __restrict__ screen, double pw, const double* __restrict__ scal, const int* __restrict__ flags,
-    float* __restrict__ r32, double* __restrict__ part, int tz) {
-    update_residual_prefetch_body<TZC, RING>(z, g, p0, p1, x0, x1, b, screen, pw, scal, flags, r32, part, tz,
+    const double* __restrict__ screen, const uint32_t* __restrict__ occupied, double pw,
+    const double* __restrict__ scal, const int* __restrict__ flags, float* __restrict__ r32,
+    double* __restrict__ part, int tz) {
+    update_residual_prefetch_body<TZC, RING>(z, g, p0, p1, x0, x1, b, screen, occupied, pw, scal, flags, r32, part, tz,
                                              blockIdx.x, blockIdx.y, blockIdx.z, block_index());
 }
 
@@ -416,14 +467,16 @@ __global__ void loop_kernel(cudaGraphConditionalHandle handle, int use_handle, c
 }
 
 static int direction_planes(int n) {
-    const int64_t tz = tuned(PB_TUNE_FCG_DIRECTION_PLANES, n, planes_of(n));
+    const int64_t tz = tuned(PB_TUNE_FCG_DIRECTION_PLANES, n, direction_planes_of(n));
     return tz < kMinTZ ? kMinTZ : (int)tz;
 }
 static int update_planes(int n) {
-    const int64_t tz = tuned(PB_TUNE_FCG_UPDATE_PLANES, n, planes_of(n));
+    const int64_t tz = tuned(PB_TUNE_FCG_UPDATE_PLANES, n, update_planes_of(n));
     return tz < kMinTZ ? kMinTZ : (int)tz;
 }
-static dim3 flat_grid_of(int n, int tz) { return dim3((n * n + kThreads - 1) / kThreads, (n + tz - 1) / tz); }
+static dim3 flat_grid_of(int n, int tz) {
+    return dim3((n * ((n + kW - 1) / kW) + kThreads - 1) / kThreads, (n + tz - 1) / tz);
+}
 static dim3 tile_grid_of(int n, int tz) {
     return dim3((n + kUX - 1) / kUX, (n + kUY - 1) / kUY, (n + tz - 1) / tz);
 }
@@ -443,20 +496,20 @@ __host__ __device__ inline Pad pad_of(int n) {
 
 __device__ __forceinline__ double aux_double(int64_t bits) { return __longlong_as_double((long long)bits); }
 
-// ptr[0] z, ptr[1] p0, ptr[2] p1, ptr[3] r32, ptr[4] screen, ptr[5] partials.
-__global__ void __launch_bounds__(kThreads, 4) direction_sums_grouped_kernel(const batch::GridDesc* __restrict__ descs,
+// ptr[0] z, ptr[1] p0, ptr[2] p1, ptr[3] r32, ptr[4] screen, ptr[5] partials, ptr[6] occupancy (or null).
+__global__ void __launch_bounds__(kThreads, 6) direction_sums_grouped_kernel(const batch::GridDesc* __restrict__ descs,
                                                                              int count, const int* __restrict__ flags) {
     int bx, by, bz;
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
-    auto run = [&](auto planes) {  // the same instantiation as the single launch of that side
-        direction_sums_body<decltype(planes)::value>(
+    auto run = [&](auto aligned) {
+        direction_sums_body<decltype(aligned)::value>(
             (const float*)d.ptr[0], pad_of((int)d.n), (const float*)d.ptr[1], (const float*)d.ptr[2],
-            (const float*)d.ptr[3], (const double*)d.ptr[4], aux_double(d.aux[0]),
+            (const float*)d.ptr[3], (const double*)d.ptr[4], screen_map(d.ptr[6]), aux_double(d.aux[0]),
             flags + d.cloud * batch::kFlagStride, (double*)d.ptr[5], (int)d.aux[1], bx, by, bx + d.gx * (int64_t)by);
     };
-    if (d.aux[1] == kTZ) run(std::integral_constant<int, kTZ>());
-    else run(std::integral_constant<int, 0>());
+    if (d.aux[2]) run(std::true_type());
+    else run(std::false_type());
 }
 
 // One block per cloud: ptr[0] partials, ptr[1] the cloud's scalars; aux[0] pass-1 blocks.
@@ -470,17 +523,17 @@ __global__ void direction_finish_grouped_kernel(const batch::GridDesc* __restric
 }
 
 // ptr[0] z, ptr[1] p0, ptr[2] p1, ptr[3] x0, ptr[4] x1, ptr[5] b, ptr[6] screen, ptr[7] r32, ptr[8] the
-// cloud's scalars, ptr[9] partials.
+// cloud's scalars, ptr[9] partials, ptr[10] occupancy (or null).
 __global__ void __launch_bounds__(kUThreads, 4) update_residual_grouped_kernel(const batch::GridDesc* __restrict__ descs,
                                                                             int count, const int* __restrict__ flags) {
     int bx, by, bz;
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
-    update_residual_prefetch_body<0>((const float*)d.ptr[0], pad_of((int)d.n), (float*)d.ptr[1], (float*)d.ptr[2],
-                         (double*)d.ptr[3], (double*)d.ptr[4], (const double*)d.ptr[5], (const double*)d.ptr[6],
-                         aux_double(d.aux[0]), (const double*)d.ptr[8], flags + d.cloud * batch::kFlagStride,
-                         (float*)d.ptr[7], (double*)d.ptr[9], (int)d.aux[1], bx, by, bz,
-                         bx + d.gx * ((int64_t)by + d.gy * bz));
+    update_residual_prefetch_body<0>(
+        (const float*)d.ptr[0], pad_of((int)d.n), (float*)d.ptr[1], (float*)d.ptr[2], (double*)d.ptr[3],
+        (double*)d.ptr[4], (const double*)d.ptr[5], (const double*)d.ptr[6], either_map(d.ptr[10], (int)d.n),
+        aux_double(d.aux[0]), (const double*)d.ptr[8], flags + d.cloud * batch::kFlagStride, (float*)d.ptr[7],
+        (double*)d.ptr[9], (int)d.aux[1], bx, by, bz, bx + d.gx * ((int64_t)by + d.gy * bz));
 }
 
 // One block per cloud: ptr[0] partials, ptr[1] output (the cloud's scal + 4); aux[0] blocks.
@@ -527,12 +580,13 @@ int describe_fcg_direction(GridDesc& d) {
     for (int k = 0; k < 6; ++k)
         if (!d.ptr[k]) return fail(PB_ERR_INVALID, "batch fcg direction: bad args");
     if (n < 2 || n > 4097 || d.ptr[1] == d.ptr[2]) return fail(PB_ERR_INVALID, "batch fcg direction: bad args");
-    const int tz = fcg::planes_of(n);  // grouped launches keep the built-in planes per block
+    const int tz = fcg::direction_planes_of(n);  // grouped launches keep the built-in planes per block
     const dim3 g = fcg::flat_grid_of(n, tz);
     d.gx = g.x;
     d.gy = g.y;
     d.gz = 1;
     d.aux[1] = tz;
+    d.aux[2] = fcg::aligned16(d.ptr[0], d.ptr[3]);
     return PB_OK;
 }
 
@@ -542,7 +596,7 @@ int describe_fcg_update(GridDesc& d) {
         if (!d.ptr[k]) return fail(PB_ERR_INVALID, "batch fcg update: bad args");
     if (n < 2 || n > 4097 || d.ptr[1] == d.ptr[2] || d.ptr[3] == d.ptr[4])
         return fail(PB_ERR_INVALID, "batch fcg update: bad args");
-    const int tz = fcg::planes_of(n);
+    const int tz = fcg::update_planes_of(n);
     const dim3 g = fcg::tile_grid_of(n, tz);
     d.gx = g.x;
     d.gy = g.y;
@@ -559,8 +613,8 @@ int describe_fcg_reduce(GridDesc& d) {
 
 // Partial-sum doubles one cloud of side n needs (both FCG passes).
 int64_t fcg_partials(int n) { return (int64_t)fcg::blocks_of(n) * 4; }
-int64_t fcg_direction_blocks(int n) { return fcg::count(fcg::flat_grid_of(n, fcg::planes_of(n))); }
-int64_t fcg_update_blocks(int n) { return fcg::count(fcg::tile_grid_of(n, fcg::planes_of(n))); }
+int64_t fcg_direction_blocks(int n) { return fcg::count(fcg::flat_grid_of(n, fcg::direction_planes_of(n))); }
+int64_t fcg_update_blocks(int n) { return fcg::count(fcg::tile_grid_of(n, fcg::update_planes_of(n))); }
 
 int launch_fcg(int kind, const GridDesc* descs, int count, int64_t blocks, const int* flags, cudaStream_t s) {
     switch (kind) {
@@ -612,10 +666,12 @@ static int fcg_check(int64_t n, size_t workspace_bytes, const void* workspace) {
 // FCG(1) pass 1 after the preconditioner produced z (padded FP32): the step's
 // scalars into scal[0..3] (scal[0] holds the previous (p, Ap) on entry).
 // p0/p1: the two dense FP32 direction buffers, p_prev = p[flags[1] & 1];
-// r32: the padded FP32 residual the preconditioner read.
-extern "C" int pb_fcg_direction_f64(const float* z, const float* p0, const float* p1, const float* r32,
-                                    const double* screen, int64_t n, double point_weight, double* scal,
-                                    const int* flags, void* workspace, size_t workspace_bytes, void* stream) {
+// r32: the padded FP32 residual the preconditioner read; occupancy: the words that
+// pb_refine_start_f64 wrote for this screen and right-hand side, or null.
+extern "C" int pb_fcg_direction_sparse_f64(const float* z, const float* p0, const float* p1, const float* r32,
+                                           const double* screen, const void* occupancy, int64_t n,
+                                           double point_weight, double* scal, const int* flags, void* workspace,
+                                           size_t workspace_bytes, void* stream) {
     using namespace pb::fcg;
     if (n < 2 || n > 4097 || !z || !p0 || !p1 || p0 == p1 || !r32 || !screen || !scal || !flags)
         return fail(PB_ERR_INVALID, "fcg direction: bad args");
@@ -624,26 +680,35 @@ extern "C" int pb_fcg_direction_f64(const float* z, const float* p0, const float
     cudaStream_t s = (cudaStream_t)stream;
     const int tz = direction_planes((int)n);
     const dim3 grid = flat_grid_of((int)n, tz);
-    const bool fixed = tz == kTZ;
-    auto dir = fixed ? direction_sums_kernel<4, kTZ> : direction_sums_kernel<4, 0>;
+    auto dir = direction_sums_kernel<6>;
     switch (tuned(PB_TUNE_FCG_DIRECTION_VARIANT, n, 0)) {
-        case 1: dir = fixed ? direction_sums_kernel<6, kTZ> : direction_sums_kernel<6, 0>; break;
-        case 2: dir = fixed ? direction_sums_kernel<8, kTZ> : direction_sums_kernel<8, 0>; break;
+        case 1: dir = direction_sums_kernel<4>; break;
+        case 2: dir = direction_sums_kernel<8>; break;
         default: break;
     }
-    dir<<<grid, kThreads, 0, s>>>(z, pad_of((int)n), p0, p1, r32, screen, point_weight, flags, part, tz);
+    if (!aligned16(z, r32)) dir = direction_sums_kernel<4, false>;
+    dir<<<grid, kThreads, 0, s>>>(z, pad_of((int)n), p0, p1, r32, screen, tz <= 32 ? screen_map(occupancy) : nullptr,
+                                  point_weight, flags, part, tz);
     PB_CHECK_LAUNCH("fcg direction_sums_kernel");
     direction_finish_kernel<<<1, 1024, 0, s>>>(part, (int)count(grid), flags, scal);
     PB_CHECK_LAUNCH("fcg direction_finish_kernel");
     return PB_OK;
 }
 
+extern "C" int pb_fcg_direction_f64(const float* z, const float* p0, const float* p1, const float* r32,
+                                    const double* screen, int64_t n, double point_weight, double* scal,
+                                    const int* flags, void* workspace, size_t workspace_bytes, void* stream) {
+    return pb_fcg_direction_sparse_f64(z, p0, p1, r32, screen, nullptr, n, point_weight, scal, flags, workspace,
+                                       workspace_bytes, stream);
+}
+
 // FCG(1) pass 2: p_new, x_new = x + alpha p_new and the true residual
 // r = b - A x_new into r32, scal[4] = ||r||^2.  Iterate and direction buffers
-// alternate by parity of flags[1]: x[it & 1] -> x[(it+1) & 1].
-extern "C" int pb_fcg_update_f64(const float* z, float* p0, float* p1, double* x0, double* x1, const double* b,
-                                 const double* screen, float* r32, int64_t n, double point_weight, double* scal,
-                                 const int* flags, void* workspace, size_t workspace_bytes, void* stream) {
+// alternate by parity of flags[1]: x[it & 1] -> x[(it+1) & 1].  occupancy as in pass 1.
+extern "C" int pb_fcg_update_sparse_f64(const float* z, float* p0, float* p1, double* x0, double* x1, const double* b,
+                                        const double* screen, const void* occupancy, float* r32, int64_t n,
+                                        double point_weight, double* scal, const int* flags, void* workspace,
+                                        size_t workspace_bytes, void* stream) {
     using namespace pb::fcg;
     if (n < 2 || n > 4097 || !z || !p0 || !p1 || p0 == p1 || !x0 || !x1 || x0 == x1 || !b || !screen || !r32 ||
         !scal || !flags)
@@ -657,12 +722,20 @@ extern "C" int pb_fcg_update_f64(const float* z, float* p0, float* p1, double* x
     auto upd = fixed ? update_residual_prefetch_kernel<kTZ> : update_residual_prefetch_kernel<0>;
     if (tuned(PB_TUNE_FCG_UPDATE_VARIANT, n, 0) == 4)
         upd = fixed ? update_residual_prefetch_kernel<kTZ, 4> : update_residual_prefetch_kernel<0, 4>;
-    upd<<<grid, dim3(kUX, kUY), 0, s>>>(z, pad_of((int)n), p0, p1, x0, x1, b, screen, point_weight, scal, flags,
+    upd<<<grid, dim3(kUX, kUY), 0, s>>>(z, pad_of((int)n), p0, p1, x0, x1, b, screen,
+                                        tz <= 32 ? either_map(occupancy, (int)n) : nullptr, point_weight, scal, flags,
                                         r32, part, tz);
     PB_CHECK_LAUNCH("fcg update_residual_prefetch_kernel");
     sum_kernel<<<1, 1024, 0, s>>>(part, (int)count(grid), scal + 4);
     PB_CHECK_LAUNCH("fcg sum_kernel");
     return PB_OK;
+}
+
+extern "C" int pb_fcg_update_f64(const float* z, float* p0, float* p1, double* x0, double* x1, const double* b,
+                                 const double* screen, float* r32, int64_t n, double point_weight, double* scal,
+                                 const int* flags, void* workspace, size_t workspace_bytes, void* stream) {
+    return pb_fcg_update_sparse_f64(z, p0, p1, x0, x1, b, screen, nullptr, r32, n, point_weight, scal, flags, workspace,
+                                    workspace_bytes, stream);
 }
 
 // ---- device-driven iteration: a CUDA graph with a WHILE conditional node ------

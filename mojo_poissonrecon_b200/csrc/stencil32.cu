@@ -11,6 +11,7 @@
 #include "batch.cuh"
 #include "common.cuh"
 #include "level32.cuh"
+#include "occupancy.cuh"
 
 namespace pb {
 
@@ -120,12 +121,13 @@ __global__ void sum_partials_kernel(const double* __restrict__ partial, int coun
 // defect and norm that it replaces (257^3: 390 -> 221 us).
 constexpr int kStartZ = 8;
 
-__global__ void __launch_bounds__(256) refine_start_kernel(const double* __restrict__ rhs,
+__global__ void __launch_bounds__(256, 4) refine_start_kernel(const double* __restrict__ rhs,
                                                            const double* __restrict__ screen, Geom g, double pw,
                                                            double* __restrict__ rhs_copy,
                                                            double* __restrict__ screen_copy, double* __restrict__ x0,
                                                            float* __restrict__ D, float* __restrict__ invD,
                                                            float* __restrict__ weights, float* __restrict__ r32,
+                                                           uint32_t* __restrict__ occupancy,
                                                            double* __restrict__ partial) {
     __shared__ double shared[2][32];
     const int n = g.n;
@@ -133,15 +135,19 @@ __global__ void __launch_bounds__(256) refine_start_kernel(const double* __restr
     const int z0 = blockIdx.y * kStartZ, z1 = min(n, z0 + kStartZ);
     const double h = (double)(n - 1), h2 = h * h;
     double rr = 0.0, bb = 0.0;
+    uint32_t screened = 0, any = 0;  // bit z & 31
+    const int y = (int)(t / (unsigned)n), x = (int)(t - (unsigned)y * n);
     if (t < (unsigned)(n * n)) {
-        const int y = (int)(t / (unsigned)n), x = (int)(t - (unsigned)y * n);
         const int degxy = (x > 0) + (x + 1 < n) + (y > 0) + (y + 1 < n);
         const int64_t nn = (int64_t)n * n;
         int64_t i = z0 * nn + t, p = g.at(x, y, z0);
         const float inv6 = (float)(1.0 / (6.0 * h2));
-#pragma unroll 4
+#pragma unroll 2
         for (int z = z0; z < z1; ++z, i += nn, p += g.plane) {
             const double b = rhs[i], sc = screen[i];
+            const uint32_t has = __double_as_longlong(sc) != 0;
+            screened |= has << (z & 31);
+            any |= (has | (uint32_t)(__double_as_longlong(b) != 0)) << (z & 31);
             if (rhs_copy) rhs_copy[i] = b;
             if (screen_copy) screen_copy[i] = sc;
             x0[i] = 0.5;
@@ -156,6 +162,17 @@ __global__ void __launch_bounds__(256) refine_start_kernel(const double* __restr
             r32[p] = (float)r;
             rr += r * r;
             bb += b * b;
+        }
+    }
+    if (occupancy) {  // the warp's nodes lie in one to three words of each map
+        const Occupancy o{n};
+        const uint32_t at = o.at(x, y), peers = __match_any_sync(0xffffffffu, at);
+        screened = __reduce_or_sync(peers, screened);
+        any = __reduce_or_sync(peers, any);
+        if (any && (int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+            uint32_t* word = occupancy + (z0 >> 5) * o.chunk() + at;
+            if (screened) atomicOr(word, screened);
+            atomicOr(word + o.map_words(), any);
         }
     }
     rr = warp_block_sum(rr, shared[0]);
@@ -347,13 +364,17 @@ extern "C" size_t pb_refine_start_workspace_size(int64_t n) {
     return (size_t)g.x * g.y * 2 * sizeof(double) + 256;
 }
 
-// The start of a refined solve (refine_start_kernel).  rhs_copy, screen_copy (either
-// may be null) and x0: dense FP64; the rest padded FP32 (ghosts untouched);
+extern "C" size_t pb_occupancy_size(int64_t n) {
+    return n < 2 || n > 4097 ? 0 : (size_t)Occupancy{(int)n}.words() * sizeof(uint32_t);
+}
+
+// The start of a refined solve (refine_start_kernel).  rhs_copy, screen_copy, occupancy
+// (each may be null; occupancy.cuh, pb_occupancy_size bytes) and x0: dense FP64; the rest padded FP32 (ghosts untouched);
 // *norm2 = ||r||^2, *bnorm = ||b||.
-extern "C" int pb_refine_start_f64(const double* rhs, const double* screen, int64_t n, double point_weight,
-                                   double* rhs_copy, double* screen_copy, double* x0, float* D, float* invD,
-                                   float* weights, float* r32, double* norm2, double* bnorm, void* workspace,
-                                   size_t workspace_bytes, void* stream) {
+extern "C" int pb_refine_start_sparse_f64(const double* rhs, const double* screen, int64_t n, double point_weight,
+                                          double* rhs_copy, double* screen_copy, double* x0, float* D, float* invD,
+                                          float* weights, float* r32, void* occupancy, double* norm2, double* bnorm,
+                                          void* workspace, size_t workspace_bytes, void* stream) {
     if (n < 2 || n > 4097 || !rhs || !screen || !x0 || !D || !invD || !weights || !r32 || !norm2 || !bnorm)
         return fail(PB_ERR_INVALID, "refine start: bad args");
     const dim3 grid = refine_start_grid((int)n);
@@ -361,12 +382,21 @@ extern "C" int pb_refine_start_f64(const double* rhs, const double* screen, int6
     if (!workspace || workspace_bytes < (size_t)blocks * 2 * sizeof(double))
         return fail(PB_ERR_WORKSPACE, "refine start: workspace needs %zu bytes", pb_refine_start_workspace_size(n));
     cudaStream_t s = (cudaStream_t)stream;
+    if (occupancy) PB_CHECK_CUDA(cudaMemsetAsync(occupancy, 0, pb_occupancy_size(n), s), "occupancy");
     refine_start_kernel<<<grid, 256, 0, s>>>(rhs, screen, geom((int)n), point_weight, rhs_copy, screen_copy, x0,
-                                             D, invD, weights, r32, (double*)workspace);
+                                             D, invD, weights, r32, (uint32_t*)occupancy, (double*)workspace);
     PB_CHECK_LAUNCH("refine_start_kernel");
     refine_start_finish_kernel<<<1, 1024, 0, s>>>((const double*)workspace, blocks, norm2, bnorm);
     PB_CHECK_LAUNCH("refine_start_finish_kernel");
     return PB_OK;
+}
+
+extern "C" int pb_refine_start_f64(const double* rhs, const double* screen, int64_t n, double point_weight,
+                                   double* rhs_copy, double* screen_copy, double* x0, float* D, float* invD,
+                                   float* weights, float* r32, double* norm2, double* bnorm, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+    return pb_refine_start_sparse_f64(rhs, screen, n, point_weight, rhs_copy, screen_copy, x0, D, invD, weights, r32,
+                                      nullptr, norm2, bnorm, workspace, workspace_bytes, stream);
 }
 
 extern "C" size_t pb_defect_workspace_size(int64_t n) { return (size_t)defect_blocks((int)(n < 2 ? 2 : n)) * 8 + 256; }

@@ -19,6 +19,7 @@
 
 #include "batch.cuh"
 #include "common.cuh"
+#include "occupancy.cuh"
 
 namespace pb {
 
@@ -540,9 +541,13 @@ static int make_box_map(CUtensorMap* map, const float* base, int n, int P, int w
 // written.
 constexpr int kProTX = 32, kProTY = 8, kProTZ = 16;
 
+// The correction of a coarse plane at the thread's row, c(., y) (the mean of the two
+// coarse rows on odd y), is formed once and serves the three fine planes that it
+// weighs on.  The weights are read where there is screening only (elsewhere 1).
 __device__ __forceinline__ void prolong_add32_body(const float* __restrict__ c, float* __restrict__ f,
-                                                   const float* __restrict__ w, int n, int P, int cn, int cP, int tz,
-                                                   int row, int bx, int by) {
+                                                   const float* __restrict__ w,
+                                                   const uint32_t* __restrict__ screened, int n, int P, int cn, int cP,
+                                                   int tz, int row, int bx, int by) {
     // threads flattened over the plane's (float4 group, y), `row` threads per y:
     // the group count on short rows (full warps), a whole number of warps on
     // long ones (a warp's coarse reads stay on one row)
@@ -552,32 +557,28 @@ __device__ __forceinline__ void prolong_add32_body(const float* __restrict__ c, 
     if (y >= n || k >= groups) return;
     const int x = 4 * k;
     const int z0 = by * tz, z1 = min(n, z0 + tz);
-    const int ya = y >> 1, yb = min(ya + 1, cn - 1);
+    const int ya = y >> 1;
     const float ty = (y & 1) ? 0.5f : 0.f;
     const int64_t cplane = (int64_t)(cn + 2) * cP;
     // coarse row ya, columns 2k .. 2k+2 (offset 4); column 2k+2 <= cn + 1 stays inside the padded row
-    const float* ca = c + (int64_t)(ya + 1) * cP + (2 * k + 4);
-    const int64_t dy = (int64_t)(yb - ya) * cP;
+    const float* ca = c + cplane + (int64_t)(ya + 1) * cP + (2 * k + 4);
+    const int64_t dy = (y & 1) ? cP : 0;  // y odd: row ya + 1 <= cn - 1 exists
     const int valid = min(4, n - x);
-    for (int z = z0; z < z1; ++z) {
-        const int za = z >> 1, zb = min(za + 1, cn - 1);
-        const float wz = (z & 1) ? 0.5f : 0.f;
-        const float* c0 = ca + (int64_t)(za + 1) * cplane;
-        const float* c1 = ca + (int64_t)(zb + 1) * cplane;
-        float q[3];
+    auto correction = [&](int zc, float (&q)[3]) {
+        const float* r = ca + zc * cplane;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const float a0 = c0[i] * (1.f - ty) + c0[dy + i] * ty;
-            const float a1 = c1[i] * (1.f - ty) + c1[dy + i] * ty;
-            q[i] = a0 * (1.f - wz) + a1 * wz;
-        }
+        for (int i = 0; i < 3; ++i) q[i] = r[i] * (1.f - ty) + r[dy + i] * ty;
+    };
+    const int64_t plane = (int64_t)(n + 2) * P;
+    int64_t p = (z0 + 1) * plane + (int64_t)(y + 1) * P + (x + 4);
+    uint32_t some = z1 - z0 <= 32 ? plane_bits(screened, n, x, y, z0) : 0xffffffffu;
+    const auto add = [&](const float (&q)[3], float4 e) {  // one fine plane; e: its values (valid == 4)
         // x interpolation: t = 0 on even x, 1/2 on odd x (coarse 2k + 2 only weighs odd x < n - 1)
         const float v0 = q[0], v1 = q[0] * 0.5f + q[1] * 0.5f, v2 = q[1], v3 = q[1] * 0.5f + q[2] * 0.5f;
-        const int64_t p = ((int64_t)(z + 1) * (n + 2) + (y + 1)) * P + (x + 4);
         PB_GUARD(p + (valid < 4 ? valid : 4) - 1, (int64_t)(n + 2) * (n + 2) * P, kSiteProlong)
         if (valid == 4) {
-            float4 e = *reinterpret_cast<const float4*>(f + p);
-            const float4 s = *reinterpret_cast<const float4*>(w + p);
+            float4 s = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (some & 1u) s = *reinterpret_cast<const float4*>(w + p);
             e.x += s.x * v0;
             e.y += s.y * v1;
             e.z += s.z * v2;
@@ -589,18 +590,49 @@ __device__ __forceinline__ void prolong_add32_body(const float* __restrict__ c, 
             for (int j = 0; j < 3; ++j)
                 if (j < valid) f[p + j] += w[p + j] * v[j];
         }
+        p += plane;
+        some = some >> 1 | (z1 - z0 <= 32 ? 0u : 0x80000000u);
+    };
+    const auto fine = [&](int64_t at) {
+        return valid == 4 ? *reinterpret_cast<const float4*>(f + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float qa[3];
+    correction(z0 >> 1, qa);
+    int z = z0;
+    const auto between = [&](const float (&qb)[3], float4 e) {  // the odd plane between qa and qb, which becomes qa
+        float q[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) q[i] = qa[i] * 0.5f + qb[i] * 0.5f;
+        add(q, e);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) qa[i] = qb[i];
+    };
+    if ((z & 1) && z < z1) {
+        float qb[3];
+        correction((z + 1) >> 1, qb);
+        between(qb, fine(p));
+        ++z;
     }
+    for (; z + 1 < z1; z += 2) {  // an even plane and the odd one above it: their loads together
+        float qb[3];
+        const float4 e0 = fine(p), e1 = fine(p + plane);
+        correction((z >> 1) + 1, qb);
+        add(qa, e0);
+        between(qb, e1);
+    }
+    if (z < z1) add(qa, fine(p));
 }
 
 __global__ void __launch_bounds__(kProTX* kProTY) prolong_add32_kernel(const float* __restrict__ c,
                                                                        float* __restrict__ f,
-                                                                       const float* __restrict__ w, int n, int P,
-                                                                       int cn, int cP, int tz, int row) {
-    prolong_add32_body(c, f, w, n, P, cn, cP, tz, row, blockIdx.x, blockIdx.y);
+                                                                       const float* __restrict__ w,
+                                                                       const uint32_t* __restrict__ screened, int n,
+                                                                       int P, int cn, int cP, int tz, int row) {
+    prolong_add32_body(c, f, w, screened, n, P, cn, cP, tz, row, blockIdx.x, blockIdx.y);
 }
 
-// Grouped (batch.cuh): ptr[0] = coarse, ptr[1] = fine, ptr[2] = weights;
-// aux[0] = planes per block, aux[1] = threads per row.
+// Grouped (batch.cuh): ptr[0] = coarse, ptr[1] = fine, ptr[2] = weights, ptr[3] = occupancy
+// (or null); aux[0] = planes per block, aux[1] = threads per row.
 __global__ void __launch_bounds__(kProTX* kProTY) prolong_add32_grouped_kernel(const batch::GridDesc* __restrict__ descs,
                                                                                int count,
                                                                                const int* __restrict__ flags) {
@@ -608,8 +640,8 @@ __global__ void __launch_bounds__(kProTX* kProTY) prolong_add32_grouped_kernel(c
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
     const int n = (int)d.n, cn = (n + 1) / 2;
-    prolong_add32_body((const float*)d.ptr[0], (float*)d.ptr[1], (const float*)d.ptr[2], n, ((n + 5) + 7) & ~7, cn,
-                       ((cn + 5) + 7) & ~7, (int)d.aux[0], (int)d.aux[1], bx, by);
+    prolong_add32_body((const float*)d.ptr[0], (float*)d.ptr[1], (const float*)d.ptr[2], screen_map(d.ptr[3]), n,
+                       ((n + 5) + 7) & ~7, cn, ((cn + 5) + 7) & ~7, (int)d.aux[0], (int)d.aux[1], bx, by);
 }
 
 }  // namespace pb
@@ -712,8 +744,8 @@ extern "C" int pb_sweep_tma_f32(const float* e_in, float* e_out, const float* rh
 
 // fine += s * trilinear(coarse) (coarse side (n+1)/2), padded layouts, s the
 // fine level's prolongation weights.
-extern "C" int pb_prolong_fac_f32(const float* coarse, float* fine, const float* weights, int64_t fine_n,
-                                  void* stream) {
+extern "C" int pb_prolong_fac_sparse_f32(const float* coarse, float* fine, const float* weights,
+                                         const void* occupancy, int64_t fine_n, void* stream) {
     if (fine_n < 3 || fine_n > 4097 || !coarse || !fine || !weights) return fail(PB_ERR_INVALID, "prolong32: bad args");
     const int n = (int)fine_n, cn = (n + 1) / 2;
     const int groups = (n + 3) / 4;
@@ -723,10 +755,15 @@ extern "C" int pb_prolong_fac_f32(const float* coarse, float* fine, const float*
     const int64_t fill = (int64_t)gxy * n / (4 * kSMs);
     const int tz = (int)tuned(PB_TUNE_PROLONG_PLANES, n, fill < 1 ? 1 : (fill > kProTZ ? kProTZ : fill));
     const dim3 grid(gxy, (n + tz - 1) / tz);
-    prolong_add32_kernel<<<grid, kProTX * kProTY, 0, (cudaStream_t)stream>>>(coarse, fine, weights, n, pitch_for(n),
-                                                                              cn, pitch_for(cn), tz, row);
+    prolong_add32_kernel<<<grid, kProTX * kProTY, 0, (cudaStream_t)stream>>>(
+        coarse, fine, weights, screen_map(occupancy), n, pitch_for(n), cn, pitch_for(cn), tz, row);
     PB_CHECK_LAUNCH("prolong_add32_kernel");
     return PB_OK;
+}
+
+extern "C" int pb_prolong_fac_f32(const float* coarse, float* fine, const float* weights, int64_t fine_n,
+                                  void* stream) {
+    return pb_prolong_fac_sparse_f32(coarse, fine, weights, nullptr, fine_n, stream);
 }
 
 // ---- grouped launches (batch.cuh) ----------------------------------------------------

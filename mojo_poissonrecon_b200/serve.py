@@ -68,6 +68,8 @@ def hierarchy_bytes(n: int) -> int:
     level 0 six padded arrays; every level below it 20 (14 coefficient planes
     and six work arrays); levels of side 17..129 also their packed couplings
     (two colours of 64 + 4 bytes per compact node)."""
+    from . import _native as nat
+
     total = 0
     for i, m in enumerate(_levels(n)):
         if i == 0 and m >= solver32.TMA_MIN_N:
@@ -76,7 +78,8 @@ def hierarchy_bytes(n: int) -> int:
         total += 20 * 4 * _padded(m)
         if m > solver32.COARSE_N:  # packed per colour
             total += 2 * 68 * (m * m * ((m + 1) // 2))
-    return total + 8 * 27 * 27 + 64 * 1024  # 3^3 inverse (FP64), coarse image
+    # 3^3 inverse (FP64), coarse image, occupancy words of level 0
+    return total + 8 * 27 * 27 + 64 * 1024 + int(nat.lib().pb_occupancy_size(n))
 
 
 def footprint_bytes(depth: int, points: int) -> int:

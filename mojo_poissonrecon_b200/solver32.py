@@ -15,7 +15,7 @@ One iteration touches the same buffers every time, so the engine captures it
 once as the body of a CUDA graph WHILE node whose condition a device kernel
 sets from ||r||^2 (pb_loop_condition); a solve is then one graph launch with
 no host synchronisation per iteration.  A solve starts with one pass over the
-right-hand side and screen (pb_refine_start_f64); the coarse levels' set-up is
+right-hand side and screen (pb_refine_start_sparse_f64); the coarse levels' set-up is
 captured once as a second graph.  Engines (hierarchy,
 vectors, graphs) are cached per device, grid side, point weight and slot and
 reused across solves.
@@ -165,6 +165,10 @@ class Hierarchy32:
                 if self.transient_coef:
                     lv.coef = None
         self.inverse = torch.zeros(27 * 27, dtype=torch.float64, device=device)  # of the 3^3 level, FP64
+        # where rhs and screen are not zero on level 0, written by `start`; `where`: its
+        # address while it describes this hierarchy's screen
+        self.occupancy = torch.zeros(self.lib.pb_occupancy_size(n) // 4, dtype=torch.int32, device=device)
+        self.where = None
         # scratch of the separable Galerkin products (27-point fine levels), at most GALERKIN_SCRATCH bytes;
         # hierarchies set up one after another on one stream may share one (galerkin_ws)
         size = galerkin_scratch_bytes(n, self.levels)
@@ -192,7 +196,7 @@ class Hierarchy32:
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for lv in self.levels for t in lv.tensors()) + \
-            self.inverse.numel() * 8 + self.image.numel() * 4 + self.galerkin_ws.numel() * 4
+            self.inverse.numel() * 8 + self.occupancy.numel() * 4 + self.image.numel() * 4 + self.galerkin_ws.numel() * 4
 
     def setup(self, screen: torch.Tensor | None, point_weight: float) -> None:
         """Level 0 from the FP64 screen (D = (deg + pw*screen) h^-2, core.py:150-163;
@@ -200,6 +204,8 @@ class Hierarchy32:
         packed forms, the 3^3 inverse and the coarse image: one library call
         (pb_hierarchy_setup_f32)."""
         self.pw = float(point_weight)
+        if screen is not None:
+            self.where = None
         for i, lv in enumerate(self.levels):  # zero-filled: the kernels write interior nodes only
             if lv.coef is None and not lv.seven:
                 lv.coef = torch.zeros(14, lv.count, dtype=torch.float32, device=self.device)
@@ -223,21 +229,24 @@ class Hierarchy32:
     def start(self, rhs: torch.Tensor, screen: torch.Tensor, point_weight: float, copies, x0, norm2, bnorm,
               workspace: nat.Workspace) -> None:
         """Level 0 and everything else a refined solve starts with, in one pass
-        (pb_refine_start_f64); copies: buffers for rhs and screen, or (None, None)."""
+        (pb_refine_start_sparse_f64); copies: buffers for rhs and screen, or (None, None)."""
         L, lv = self.lib, self.levels[0]
+        self.where = self.occupancy.data_ptr()
         ptr, size = workspace.get(L.pb_refine_start_workspace_size(lv.n))
-        nat.check(L.pb_refine_start_f64(rhs.data_ptr(), screen.data_ptr(), lv.n, float(point_weight),
-                                        *(None if t is None else t.data_ptr() for t in copies), x0.data_ptr(),
-                                        lv.D.data_ptr(), lv.invD.data_ptr(), lv.weights.data_ptr(), lv.rhs.data_ptr(),
-                                        norm2.data_ptr(), bnorm.data_ptr(), ptr, size, self.stream), "refine start")
+        nat.check(L.pb_refine_start_sparse_f64(
+            rhs.data_ptr(), screen.data_ptr(), lv.n, float(point_weight),
+            *(None if t is None else t.data_ptr() for t in copies), x0.data_ptr(), lv.D.data_ptr(),
+            lv.invD.data_ptr(), lv.weights.data_ptr(), lv.rhs.data_ptr(), self.occupancy.data_ptr(),
+            norm2.data_ptr(), bnorm.data_ptr(), ptr, size, self.stream), "refine start")
 
     def _sweep(self, lv: Level32, src, dst, mode: int, coarse=None) -> None:
         """One red-black sweep dst <- S(src); mode 1 starts from zero, mode 2
         first adds the prolongated coarse correction to src in place."""
         L, s = self.lib, self.stream
         if mode == 2:
-            nat.check(L.pb_prolong_fac_f32(coarse.data_ptr(), src.data_ptr(), lv.weights.data_ptr(), lv.n, s),
-                      "prolong32")
+            where = self.where if lv is self.levels[0] else None
+            nat.check(L.pb_prolong_fac_sparse_f32(coarse.data_ptr(), src.data_ptr(), lv.weights.data_ptr(), where, lv.n,
+                                                  s), "prolong32")
             mode = 0
         if not lv.seven:
             nat.check(L.pb_relax27p_f32(None if mode == 1 else src.data_ptr(), dst.data_ptr(), lv.rhs.data_ptr(),
@@ -403,12 +412,13 @@ class RefinedEngine:
         r32 = self.h.levels[0].rhs
         p0, p1 = (t.data_ptr() for t in self.ps)
         x0, x1 = (t.data_ptr() for t in self.xs)
-        nat.check(L.pb_fcg_direction_f64(z.data_ptr(), p0, p1, r32.data_ptr(), self.screen.data_ptr(), self.n,
-                                         self.pw, self.scal.data_ptr(), self.flags.data_ptr(), self.ws_ptr,
-                                         self.ws_size, s), "fcg direction")
-        nat.check(L.pb_fcg_update_f64(z.data_ptr(), p0, p1, x0, x1, self.b.data_ptr(), self.screen.data_ptr(),
-                                      r32.data_ptr(), self.n, self.pw, self.scal.data_ptr(), self.flags.data_ptr(),
-                                      self.ws_ptr, self.ws_size, s), "fcg update")
+        where = self.h.where
+        nat.check(L.pb_fcg_direction_sparse_f64(z.data_ptr(), p0, p1, r32.data_ptr(), self.screen.data_ptr(), where,
+                                                self.n, self.pw, self.scal.data_ptr(), self.flags.data_ptr(),
+                                                self.ws_ptr, self.ws_size, s), "fcg direction")
+        nat.check(L.pb_fcg_update_sparse_f64(z.data_ptr(), p0, p1, x0, x1, self.b.data_ptr(), self.screen.data_ptr(),
+                                             where, r32.data_ptr(), self.n, self.pw, self.scal.data_ptr(),
+                                             self.flags.data_ptr(), self.ws_ptr, self.ws_size, s), "fcg update")
         nat.check(L.pb_loop_condition(handle, self.scal.data_ptr(), self.ctrl.data_ptr(), self.flags.data_ptr(),
                                       MAX_ITER, self.history.data_ptr(), s), "loop condition")
 
