@@ -78,6 +78,10 @@ int pb_octree_codes_f64(const double *points, int64_t point_count, int64_t depth
 size_t pb_octree_workspace_size(int64_t point_count, int64_t depth);
 int pb_octree_count(const double *points, int64_t point_count, int64_t depth,
                     int64_t *level_counts, void *workspace, size_t workspace_bytes, void *stream);
+/* The same, counting into *outside (device int64, may be NULL) the points that are not finite or not in
+ * [0, 1]^3 (build_octree refuses them). */
+int pb_octree_count_checked(const double *points, int64_t point_count, int64_t depth, int64_t *level_counts,
+                            int64_t *outside, void *workspace, size_t workspace_bytes, void *stream);
 int pb_octree_emit(int64_t point_count, int64_t depth, const int64_t *level_counts,
                    int64_t node_count, int64_t *node_depth, int64_t *morton, int64_t *parent,
                    int64_t *child_start, int64_t *child_count, int64_t *point_leaf,

@@ -30,6 +30,7 @@ _SIGNATURES = {
     "pb_octree_codes_f64": ([P, I, I, P, P], C),
     "pb_octree_workspace_size": ([I, I], S),
     "pb_octree_count": ([P, I, I, P, P, S, P], C),
+    "pb_octree_count_checked": ([P, I, I, P, P, P, S, P], C),
     "pb_octree_emit": ([I, I, P, I, P, P, P, P, P, P, P, S, P], C),
     "pb_splat_workspace_size": ([I, I], S),
     "pb_splat_f64": ([P, P, I, I, I, P, P, P, P, P, F, P, P, S, P], C),

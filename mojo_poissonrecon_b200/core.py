@@ -195,10 +195,13 @@ def _octree_device(ctx: _Context, points: torch.Tensor, depth: int) -> dict:
                     point_leaf=torch.empty(0, dtype=torch.int64, device=ctx.device))
     ws = nat.Workspace(ctx.device)  # kept alive across the two phases
     ptr, size = ws.get(L.pb_octree_workspace_size(count, depth))
-    counts = torch.empty(depth + 1, dtype=torch.int64, device=ctx.device)
-    ctx.check(L.pb_octree_count(points.data_ptr(), count, depth, counts.data_ptr(), ptr, size, ctx.stream),
-              "octree count")
-    nodes = int(counts.sum().item())
+    counts = torch.empty(depth + 2, dtype=torch.int64, device=ctx.device)  # per level; points outside the cube
+    ctx.check(L.pb_octree_count_checked(points.data_ptr(), count, depth, counts.data_ptr(),
+                                        counts[depth + 1:].data_ptr(), ptr, size, ctx.stream), "octree count")
+    *levels, outside = counts.tolist()
+    if outside:
+        raise ValueError("octree points must be finite and inside [0, 1]^3")
+    nodes = sum(levels)
     arrays = {k: torch.empty(nodes, dtype=torch.int64, device=ctx.device)
               for k in ("depth", "morton", "parent", "child_start", "child_count")}
     arrays["point_leaf"] = torch.empty(count, dtype=torch.int64, device=ctx.device)
@@ -223,10 +226,6 @@ def build_octree(points, depth: int = 6, *, device_out: bool = False) -> FlatOct
         raise ValueError("depth must be between 0 and 19")
     ctx = _Context()
     dpts = _to_device(points, ctx.device)
-    if dpts.shape[0]:
-        bad = (~torch.isfinite(dpts)).any() | (dpts < 0).any() | (dpts > 1).any()
-        if bool(bad):
-            raise ValueError("octree points must be finite and inside [0, 1]^3")
     return _octree_out(_octree_device(ctx, dpts, depth), device_out)
 
 

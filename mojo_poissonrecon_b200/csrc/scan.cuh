@@ -40,6 +40,20 @@ __device__ __forceinline__ T block_exclusive_scan(T value, T* warp_sums /*[32]*/
     return result;
 }
 
+// Exclusive scan of one row in place by one block of kScanThreads; its sum in every thread.
+__device__ __forceinline__ uint32_t scan_row(uint32_t* row, uint32_t n) {
+    __shared__ uint32_t warp_sums[32];
+    uint32_t before = 0;
+    for (uint32_t base = 0; base < n; base += kScanThreads) {
+        const uint32_t i = base + threadIdx.x, v = i < n ? row[i] : 0u;
+        uint32_t total;
+        const uint32_t run = block_exclusive_scan<uint32_t>(v, warp_sums, total);
+        if (i < n) row[i] = before + run;
+        before += total;
+    }
+    return before;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_tiles(const T* __restrict__ in, int64_t n,
                                                                  T* __restrict__ partial) {
