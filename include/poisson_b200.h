@@ -391,6 +391,9 @@ int pb_residual_restrict_tma_f32(const float *e, const float *rhs, const float *
 size_t pb_galerkin_workspace_size(int64_t fine_n, int fine_is_7pt);
 int pb_galerkin_f32(const float *fine, int64_t fine_n, int fine_is_7pt, const float *fine_weights,
                     float *coarse, void *workspace, size_t workspace_bytes, void *stream);
+int pb_galerkin_sparse_f32(const float *fine, int64_t fine_n, int fine_is_7pt, const float *fine_weights,
+                           const void *occupancy, float *coarse, void *workspace, size_t workspace_bytes,
+                           void *stream);
 /* 14 planes of a 7-point level (diagonal D, off-diagonals -(n-1)^2). */
 int pb_level27_from7_f32(const float *D, int64_t n, float *coef, void *stream);
 /* invD = 1 / diagonal and the prolongation weights of a 27-point level. */
@@ -446,6 +449,12 @@ enum { PB_LEVEL_ARRAYS = 8 };
 int pb_hierarchy_setup_f32(int64_t levels, const int64_t *sides, const void *const *arrays, int64_t first_coarse,
                            const double *screen, double point_weight, void *galerkin_ws, size_t galerkin_bytes,
                            double *inverse, float *image, size_t image_bytes, void *stream);
+/* The same with the occupancy words of level 0's screen (pb_refine_start_sparse_f64; NULL: none), which let the
+ * product from level 0 write constants where there is no screening. */
+int pb_hierarchy_setup_sparse_f32(int64_t levels, const int64_t *sides, const void *const *arrays,
+                                  int64_t first_coarse, const double *screen, double point_weight,
+                                  const void *occupancy, void *galerkin_ws, size_t galerkin_bytes, double *inverse,
+                                  float *image, size_t image_bytes, void *stream);
 
 /* ---- batches of clouds: one grouped launch per solver step ------------------
  * No counterpart in the reference, which solves one cloud at a time and level

@@ -101,6 +101,7 @@ _SIGNATURES = {
     "pb_residual_restrict_tma_f32": ([P, P, P, P, P, I, P, P], C),
     "pb_galerkin_workspace_size": ([I, C], S),
     "pb_galerkin_f32": ([P, I, C, P, P, P, S, P], C),
+    "pb_galerkin_sparse_f32": ([P, I, C, P, P, P, P, S, P], C),
     "pb_level27_from7_f32": ([P, I, P, P], C),
     "pb_level27_finish_f32": ([P, I, P, P, P], C),
     "pb_packed27_size": ([I, ctypes.POINTER(I), ctypes.POINTER(I)], C),
@@ -118,6 +119,7 @@ _SIGNATURES = {
     "pb_batch_launch": ([C, P, I, I, P, I, P], C),
     "pb_batch_loop_condition": ([ctypes.c_ulonglong, P, P, P, I, I, P, P], C),
     "pb_hierarchy_setup_f32": ([I, P, P, I, P, F, P, S, P, P, S, P], C),
+    "pb_hierarchy_setup_sparse_f32": ([I, P, P, I, P, F, P, P, S, P, P, S, P], C),
     "pb_tune_set": ([I, I, I], C),
     "pb_tune_get": ([I, I], I),
     "pb_tune_clear": ([], C),

@@ -42,4 +42,26 @@ __device__ __forceinline__ uint32_t plane_bits(const uint32_t* __restrict__ map,
     return __funnelshift_r(word[0], ((z0 >> 5) + 1) * 32 < n ? word[o.chunk()] : 0u, z0 & 31);
 }
 
+// Whether the five planes, rows and x around (x, y, z), all inside the grid, have none
+// (false without a map; a whole word's 32 nodes count where x reaches one).
+__device__ __forceinline__ bool five_cubed_empty(const uint32_t* __restrict__ map, int n, int x, int y, int z) {
+    if (!map) return false;
+    const Occupancy o{n};
+    const int z0 = z - 2, shift = z0 & 31;
+    const uint32_t low = 0x1fu << shift, high = shift > 27 ? 0x1fu >> (32 - shift) : 0u;
+    const bool two = (x - 2) >> 5 != (x + 2) >> 5;
+    const uint32_t* word = map + (z0 >> 5) * o.chunk() + o.at(x - 2, y - 2);
+    uint32_t any = 0;
+#pragma unroll
+    for (int row = 0; row < 5; ++row, word += o.tiles()) {
+        any |= word[0] & low;
+        if (two) any |= word[1] & low;
+        if (high) {
+            any |= word[o.chunk()] & high;
+            if (two) any |= word[o.chunk() + 1] & high;
+        }
+    }
+    return any == 0;
+}
+
 }  // namespace pb

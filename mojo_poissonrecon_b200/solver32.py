@@ -202,7 +202,7 @@ class Hierarchy32:
         """Level 0 from the FP64 screen (D = (deg + pw*screen) h^-2, core.py:150-163;
         None: `start` has set it up), then each coarser level's Galerkin operator from the one above it, the
         packed forms, the 3^3 inverse and the coarse image: one library call
-        (pb_hierarchy_setup_f32)."""
+        (pb_hierarchy_setup_sparse_f32)."""
         self.pw = float(point_weight)
         if screen is not None:
             self.where = None
@@ -216,11 +216,12 @@ class Hierarchy32:
             for k, t in enumerate(row):
                 arrays[i * A + k] = None if t is None else t.data_ptr()
         sides = (ctypes.c_int64 * K)(*[lv.n for lv in self.levels])
-        nat.check(self.lib.pb_hierarchy_setup_f32(K, sides, arrays, self.first_coarse,
-                                                  None if screen is None else screen.data_ptr(), self.pw,
-                                                  self.galerkin_ws.data_ptr(), self.galerkin_ws.numel() * 4,
-                                                  self.inverse.data_ptr(), self.image.data_ptr(),
-                                                  self.image.numel() * 4, self.stream), "hierarchy setup")
+        nat.check(self.lib.pb_hierarchy_setup_sparse_f32(K, sides, arrays, self.first_coarse,
+                                                         None if screen is None else screen.data_ptr(), self.pw,
+                                                         self.where, self.galerkin_ws.data_ptr(),
+                                                         self.galerkin_ws.numel() * 4, self.inverse.data_ptr(),
+                                                         self.image.data_ptr(), self.image.numel() * 4, self.stream),
+                  "hierarchy setup")
         if self.transient_coef:
             for lv in self.levels:
                 if lv.packed is not None:

@@ -103,3 +103,16 @@ def test_sparse_passes_match_dense(L, n, kind):
         assert status == 0
         got.append(up.view(torch.int32))
     assert torch.equal(*got)
+    if n < 33 or (n - 1) & (n - 2):
+        return
+    got = []
+    for sparse in (False, True):
+        coef = torch.zeros(14, ccount, dtype=torch.float32, device="cuda")
+        if sparse:
+            status = L.pb_galerkin_sparse_f32(D.data_ptr(), n, 1, weights.data_ptr(), occupancy.data_ptr(),
+                                              coef.data_ptr(), None, 0, s)
+        else:
+            status = L.pb_galerkin_f32(D.data_ptr(), n, 1, weights.data_ptr(), coef.data_ptr(), None, 0, s)
+        assert status == 0
+        got.append(coef.view(torch.int32))
+    assert torch.equal(*got)
