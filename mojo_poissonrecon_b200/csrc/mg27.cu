@@ -733,71 +733,61 @@ __global__ void __launch_bounds__(kTRx* kTRy) residual27p_tiled_kernel(
 
 // ---- exact solve on the 3^3 level -----------------------------------------------
 // The 27 x 27 operator of the coarsest level inverted once per set-up by one
-// warp: FP64 Gauss-Jordan without pivoting (the Galerkin operator is
-// symmetric positive definite), lane i owning row i; stored FP64 row-major and
-// applied in FP64 (the coarsest-level solve stays in double precision).
+// block: FP64 Gauss-Jordan without pivoting (the Galerkin operator is
+// symmetric positive definite), a thread per element, the pivot's row and column
+// through shared memory (two by step parity: one barrier a step); stored FP64 row-major
+// and applied in FP64 (the coarsest-level solve stays in double precision).  One warp
+// with a row per lane took 27 us, mostly a serial walk of the rows.
 constexpr int kInvN = 27;
 
-__global__ void __launch_bounds__(32) coarse_inverse_kernel(const float* __restrict__ c, int64_t cs, Geom g,
-                                                            double* __restrict__ inv) {
-    __shared__ double a[kInvN][kInvN + 1];
-    const int lane = threadIdx.x;
-    if (lane < kInvN) {
-        const int x = lane % 3, y = (lane / 3) % 3, z = lane / 9;
-        const int64_t p = g.at(x, y, z);
-        for (int j = 0; j < kInvN; ++j) a[lane][j] = 0.0;
-#pragma unroll
-        for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-            for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-                for (int dx = -1; dx <= 1; ++dx)
-                    if (inside(x + dx, y + dy, z + dz, 3))
-                        a[lane][lane + dx + 3 * dy + 9 * dz] = (double)coupling(c, cs, g, p, dx, dy, dz);
-    }
-    __syncwarp();
+__global__ void __launch_bounds__(32 * kInvN) coarse_inverse_kernel(const float* __restrict__ c, int64_t cs, Geom g,
+                                                                    double* __restrict__ inv) {
+    __shared__ double pivot_row[2][32], pivot_column[2][kInvN];
+    const int i = threadIdx.x >> 5, j = threadIdx.x & 31;  // a warp per row
+    double a = 0.0;
+    const int x = i % 3, y = i / 3 % 3, z = i / 9, dx = j % 3 - x, dy = j / 3 % 3 - y, dz = j / 9 - z;
+    if (j < kInvN && dx * dx <= 1 && dy * dy <= 1 && dz * dz <= 1)
+        a = (double)coupling(c, cs, g, g.at(x, y, z), dx, dy, dz);
     for (int k = 0; k < kInvN; ++k) {
-        const double inv_piv = 1.0 / a[k][k];
-        __syncwarp();
-        if (lane < kInvN) a[k][lane] = lane == k ? inv_piv : a[k][lane] * inv_piv;  // row k / pivot, in parallel
-        __syncwarp();
-        if (lane < kInvN && lane != k) {
-            const double f = a[lane][k];
-            a[lane][k] = 0.0;
-            for (int j = 0; j < kInvN; ++j) a[lane][j] -= f * a[k][j];
-        }
-        __syncwarp();
+        double *row = pivot_row[k & 1], *column = pivot_column[k & 1];
+        if (i == k) row[j] = a;
+        if (j == k) column[i] = a;
+        __syncthreads();
+        const double inv_piv = 1.0 / row[k];
+        const double r = j == k ? inv_piv : row[j] * inv_piv;  // row k / pivot
+        a = i == k ? r : (j == k ? 0.0 : a) - column[i] * r;
     }
-    if (lane < kInvN)
-        for (int j = 0; j < kInvN; ++j) inv[lane * kInvN + j] = a[lane][j];
+    if (j < kInvN) inv[i * kInvN + j] = a;
 }
 
-// ---- levels of side <= 9 in one block, from shared memory -------------------------
+// ---- levels of side <= 9 in one block ---------------------------------------------
 // The first level of side <= 9 and those below it (9, 5, 3) run in one block.
 // Their operators do not change during a solve, so set-up writes them once
 // into a compact image (pb_coarse27_image_f32): per level above the last, the
 // 27 couplings of every node (offsets (dz, dy, dx) in lexicographic order, zero
-// outside the grid), 1/diagonal and the prolongation weights, node-major; then
-// the 3^3 inverse (FP64).  Each cycle copies the image into shared memory and keeps e,
-// rhs and the residual of every level there in padded cubes ((n+2)^3 floats,
-// zero ghosts), so global memory sees only the first level's rhs and its
-// correction.
+// outside the grid; one coupling of all nodes after another), 1/diagonal and the
+// prolongation weights; then the 3^3 inverse (FP64).
+//
+// A thread owns one node of one level, a level's threads its even nodes and then its
+// odd ones (the colours), and keeps the node's couplings, weight, right-hand side and
+// value in registers; the values go to shared memory split by colour, two copies of
+// each, so that a colour's pass reads one copy and writes the other with one barrier,
+// and its lanes read consecutive words.  Bound by latency: with the couplings in
+// shared memory and two barriers a pass a cycle took 31 us.
 constexpr int kC27N = 9;
 constexpr int kC27Threads = 1024;
 constexpr int kC27MaxLevels = 3;  // 9, 5, 3
-static_assert(kC27N * kC27N * kC27N <= kC27Threads, "one node per thread on the largest level");
+constexpr int round32(int v) { return (v + 31) & ~31; }
+static_assert(round32(9 * 9 * 9) + round32(5 * 5 * 5) + 27 <= kC27Threads, "one node per thread over all levels");
 
 __host__ __device__ inline int round4(int v) { return (v + 3) & ~3; }
-__host__ __device__ inline int cube_size(int n) { return (n + 2) * (n + 2) * (n + 2); }
 
-// Float offsets of the image sections and of the shared work cubes (after the image).
+// Float offsets of the image sections.
 struct CoarseLayout {
     int count;
     int n[kC27MaxLevels];
     int coef[kC27MaxLevels], invD[kC27MaxLevels], fac[kC27MaxLevels], inverse;
     int image;  // floats of the image (a multiple of 4)
-    int e[kC27MaxLevels], rhs[kC27MaxLevels], res[kC27MaxLevels];
-    int total;  // floats of shared memory
 };
 
 __host__ __device__ inline CoarseLayout coarse_layout(int count, const int* sizes) {
@@ -818,40 +808,13 @@ __host__ __device__ inline CoarseLayout coarse_layout(int count, const int* size
     c.inverse = off;  // 16-byte aligned: doubles
     off += round4(2 * kInvN * kInvN);
     c.image = off;
-    for (int l = 0; l < count; ++l) {
-        const int m = round4(cube_size(sizes[l]));
-        c.e[l] = off;
-        c.rhs[l] = off + m;
-        c.res[l] = off + 2 * m;
-        off += 3 * m;
-    }
-    c.total = off;
     return c;
 }
-
-__device__ __forceinline__ int cube_at(int x, int y, int z, int n) { return ((z + 1) * (n + 2) + (y + 1)) * (n + 2) + (x + 1); }
 
 __device__ __forceinline__ void unflatten(int i, int n, int& x, int& y, int& z) {
     x = i % n;
     y = (i / n) % n;
     z = i / (n * n);
-}
-
-// sum over the 27 (or 26) offsets of a_K e[J+K], in the couplings' order.
-__device__ __forceinline__ float stencil_cube(const float* a, const float* e, int c, int n, bool skip_centre) {
-    const int sy = n + 2, sz = (n + 2) * (n + 2);
-    float s = 0.0f;
-    int k = 0;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-        for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-            for (int dx = -1; dx <= 1; ++dx, ++k) {
-                if (skip_centre && !(dx || dy || dz)) continue;
-                s += a[k] * e[c + dx + dy * sy + dz * sz];
-            }
-    return s;
 }
 
 // One node's couplings, 1/diagonal and weight into the image (set-up).
@@ -871,117 +834,184 @@ __global__ void coarse_image_kernel(const float* __restrict__ c, int64_t cs, Geo
         for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
             for (int dx = -1; dx <= 1; ++dx, ++k)
-                coef_out[27 * i + k] = inside(x + dx, y + dy, z + dz, n) ? coupling(c, cs, g, p, dx, dy, dz) : 0.0f;
+                coef_out[(int64_t)k * N + i] = inside(x + dx, y + dy, z + dz, n) ? coupling(c, cs, g, p, dx, dy, dz) : 0.0f;
     invD_out[i] = invD[p];
     fac_out[i] = fac[p];
 }
 
-// Red-black ordered sweeps in place on a cube: each colour's new values are
-// computed from the current iterate and written after a barrier, so
-// same-colour neighbours are read from the previous iterate, as the
-// multi-block colour passes do.
-__device__ void cube_relax(const float* cf, const float* invD, const float* rhs, float* e, int n, int iters) {
-    const int N = n * n * n, i = threadIdx.x;
-    int x = 0, y = 0, z = 0;
-    if (i < N) unflatten(i, n, x, y, z);
-    const int c = cube_at(x, y, z, n);
-    for (int it = 0; it < iters; ++it)
-        for (int colour = 0; colour < 2; ++colour) {
-            const bool mine = i < N && ((x + y + z) & 1) == colour;
-            float v = 0.0f;
-            if (mine) v = (rhs[c] - stencil_cube(cf + 27 * i, e, c, n, true)) * invD[i];
-            __syncthreads();
-            if (mine) e[c] = v;
-            __syncthreads();
-        }
+// A level's values in shared memory: the padded cube of side N + 2 (zero ghosts) by the
+// parity of the linear index (a node's colour and its index's parity differ by one, so
+// a colour is one parity), two copies.
+template <int N>
+struct Cube {
+    static constexpr int M = N + 2, SIZE = M * M * M, HALF = (SIZE + 1) / 2;
+    float e[2][2][HALF];  // by parity of the index, copy
+    float res[SIZE];      // weighted residual, not split
+    static __device__ __forceinline__ int at(int x, int y, int z) { return ((z + 1) * M + (y + 1)) * M + (x + 1); }
+};
+
+// What a thread holds of its node.
+struct Node27 {
+    int level = -1, x, y, z, c, colour;  // c: index in the padded cube
+    float a[27], inv, fac, rhs, e;
+};
+
+// sum over the 26 neighbours, and the node itself where CENTRE, of a_K e[J + K] in the couplings' order.
+template <int N, bool CENTRE>
+__device__ __forceinline__ float stencil_cube(const Cube<N>& cube, const Node27& v, const int (&copy)[2]) {
+    constexpr int M = Cube<N>::M;
+    const int odd = v.c & 1;
+    const float* same = &cube.e[odd][copy[odd]][v.c >> 1];
+    const float* other = &cube.e[odd ^ 1][copy[odd ^ 1]][(v.c >> 1) + odd];
+    float s = 0.0f;
+    int k = 0;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+            for (int dx = -1; dx <= 1; ++dx, ++k) {
+                const int d = dx + dy * M + dz * M * M;
+                if (d == 0) {
+                    if (CENTRE) s += v.a[k] * v.e;
+                } else {
+                    s += v.a[k] * ((d & 1) ? other[(d - 1) / 2] : same[d / 2]);
+                }
+            }
+    return s;
 }
 
-__device__ __forceinline__ void coarse27_body(const float4* __restrict__ image, const CoarseLayout& lay,
+// Red-black ordered sweeps: a colour's new values come from the current iterate (its own
+// colour's neighbours included) and go to its other copy, as the multi-block colour
+// passes do.  Every thread of the block calls it; from_zero: e is zero.
+template <int N>
+__device__ __forceinline__ void cube_relax(Cube<N>& cube, Node27& v, int level, int (&copy)[2], int iters,
+                                           bool from_zero) {
+    for (int pass = 0; pass < 2 * iters; ++pass) {
+        const int colour = pass & 1, parity = colour ^ 1;
+        if (v.level == level && v.colour == colour) {
+            const float s = from_zero && pass == 0 ? 0.0f : stencil_cube<N, false>(cube, v, copy);
+            v.e = (v.rhs - s) * v.inv;
+            cube.e[parity][copy[parity] ^ 1][v.c >> 1] = v.e;
+        }
+        copy[parity] ^= 1;
+        __syncthreads();
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void cube_residual(Cube<N>& cube, const Node27& v, int level, const int (&copy)[2]) {
+    if (v.level == level) cube.res[v.c] = v.fac * (v.rhs - stencil_cube<N, true>(cube, v, copy));
+    __syncthreads();
+}
+
+// The restricted residual at coarse node (x, y, z).
+template <int N>
+__device__ __forceinline__ float cube_restrict(const Cube<N>& cube, int x, int y, int z) {
+    constexpr int M = Cube<N>::M;
+    const float* r = cube.res + Cube<N>::at(2 * x, 2 * y, 2 * z);
+    float s = 0.0f;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+            for (int dx = -1; dx <= 1; ++dx)
+                s += r[dx + dy * M + dz * M * M] * (float)((dx ? 1 : 2) * (dy ? 1 : 2) * (dz ? 1 : 2));
+    return s * (1.0f / 64.0f);
+}
+
+// e += weight * trilinear coarse correction, the mean of the 8 corners (a corner repeated
+// on even axes); value(x, y, z): the coarse level's.
+template <int N, typename Value>
+__device__ __forceinline__ void cube_prolong(Cube<N>& cube, Node27& v, int level, const int (&copy)[2], Value value) {
+    if (v.level == level) {
+        const int x0 = v.x >> 1, y0 = v.y >> 1, z0 = v.z >> 1;
+        const int x1 = x0 + (v.x & 1), y1 = y0 + (v.y & 1), z1 = z0 + (v.z & 1);
+        v.e += v.fac * (0.125f * (value(x0, y0, z0) + value(x1, y0, z0) + value(x0, y1, z0) + value(x1, y1, z0) +
+                                  value(x0, y0, z1) + value(x1, y0, z1) + value(x0, y1, z1) + value(x1, y1, z1)));
+        const int odd = v.c & 1;
+        cube.e[odd][copy[odd]][v.c >> 1] = v.e;
+    }
+    __syncthreads();
+}
+
+// V(pre, post) on the first level and `inner` sweeps each way on the one between; sides (9, 5, 3), (5, 3) or (3).
+__device__ __forceinline__ void coarse27_body(const float* __restrict__ image, const CoarseLayout& lay,
                                               const float* __restrict__ rhs0, float* __restrict__ e0, Geom g0,
                                               int pre, int post, int inner) {
-    extern __shared__ float4 smem4[];
-    float* sm = reinterpret_cast<float*>(smem4);
+    __shared__ struct {
+        Cube<9> nine;
+        Cube<5> five;
+    } cubes;
+    __shared__ double inverse[kInvN * kInvN], rhs3[kInvN];
+    __shared__ float e3[kInvN];
     const int tid = threadIdx.x;
-    for (int i = tid; i < lay.image / 4; i += kC27Threads) smem4[i] = image[i];
-    for (int i = lay.image + tid; i < lay.total; i += kC27Threads) sm[i] = 0.0f;
-    __syncthreads();
-    {
-        const int n = lay.n[0];
-        if (tid < n * n * n) {
-            int x, y, z;
-            unflatten(tid, n, x, y, z);
-            sm[lay.rhs[0] + cube_at(x, y, z, n)] = rhs0[g0.at(x, y, z)];
-        }
-    }
-    __syncthreads();
-    const int count = lay.count;
-    for (int l = 0; l < count; ++l) {
-        const int n = lay.n[l];
-        float* e = sm + lay.e[l];
-        const float* rhs = sm + lay.rhs[l];
-        if (l == count - 1) {  // side 3: e = A^-1 rhs
-            if (tid < kInvN) {
-                const double* inv = reinterpret_cast<const double*>(sm + lay.inverse);
-                double v = 0.0;
-                for (int j = 0; j < kInvN; ++j)
-                    v += inv[tid * kInvN + j] * (double)rhs[cube_at(j % 3, (j / 3) % 3, j / 9, 3)];
-                e[cube_at(tid % 3, (tid / 3) % 3, tid / 9, 3)] = (float)v;
+    for (int i = tid; i < (int)(sizeof(cubes) / sizeof(float)); i += kC27Threads) reinterpret_cast<float*>(&cubes)[i] = 0.0f;
+    if (tid < kInvN * kInvN) inverse[tid] = reinterpret_cast<const double*>(image + lay.inverse)[tid];
+    Node27 v;
+    int first = 0;  // the level's first thread; the last level's 27 threads come after the others
+#pragma unroll
+    for (int l = 0; l < kC27MaxLevels; ++l) {
+        if (l >= lay.count) break;
+        const int n = lay.n[l], count = n * n * n, t = tid - first;
+        if (t >= 0 && t < count) {
+            v.level = l;
+            const int even = (count + 1) / 2;
+            const int i = l + 1 == lay.count ? t : t < even ? 2 * t : 2 * (t - even) + 1;
+            unflatten(i, n, v.x, v.y, v.z);
+            v.colour = (v.x + v.y + v.z) & 1;
+            v.c = ((v.z + 1) * (n + 2) + (v.y + 1)) * (n + 2) + (v.x + 1);
+            v.e = 0.0f;
+            if (l == 0) v.rhs = rhs0[g0.at(v.x, v.y, v.z)];
+            if (l + 1 < lay.count) {
+#pragma unroll
+                for (int k = 0; k < 27; ++k) v.a[k] = image[lay.coef[l] + k * count + i];
+                v.inv = image[lay.invD[l] + i];
+                v.fac = image[lay.fac[l] + i];
             }
-            __syncthreads();
-            break;
         }
-        const float* cf = sm + lay.coef[l];
-        cube_relax(cf, sm + lay.invD[l], rhs, e, n, l == 0 ? pre : inner);  // e starts at zero
-        float* res = sm + lay.res[l];
-        if (tid < n * n * n) {
-            int x, y, z;
-            unflatten(tid, n, x, y, z);
-            const int c = cube_at(x, y, z, n);
-            res[c] = sm[lay.fac[l] + tid] * (rhs[c] - stencil_cube(cf + 27 * tid, e, c, n, false));
-        }
-        __syncthreads();
-        const int cn = lay.n[l + 1], sy = n + 2, sz = (n + 2) * (n + 2);
-        if (tid < cn * cn * cn) {
-            int x, y, z;
-            unflatten(tid, cn, x, y, z);
-            const int c = cube_at(2 * x, 2 * y, 2 * z, n);
-            float s = 0.0f;
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy)
-                    for (int dx = -1; dx <= 1; ++dx)
-                        s += res[c + dx + dy * sy + dz * sz] * (float)((dx ? 1 : 2) * (dy ? 1 : 2) * (dz ? 1 : 2));
-            sm[lay.rhs[l + 1] + cube_at(x, y, z, cn)] = s * (1.0f / 64.0f);
-        }
-        __syncthreads();
+        first += round32(count);
     }
-    for (int l = count - 2; l >= 0; --l) {
-        const int n = lay.n[l], cn = lay.n[l + 1];
-        float* e = sm + lay.e[l];
-        const float* ec = sm + lay.e[l + 1];
-        if (tid < n * n * n) {
-            int x, y, z;
-            unflatten(tid, n, x, y, z);
-            // trilinear: the mean of the 8 corners, a corner repeated on even axes
-            const int x0 = x >> 1, y0 = y >> 1, z0 = z >> 1;
-            const int x1 = x0 + (x & 1), y1 = y0 + (y & 1), z1 = z0 + (z & 1);
-            const float v = 0.125f * (ec[cube_at(x0, y0, z0, cn)] + ec[cube_at(x1, y0, z0, cn)] +
-                                      ec[cube_at(x0, y1, z0, cn)] + ec[cube_at(x1, y1, z0, cn)] +
-                                      ec[cube_at(x0, y0, z1, cn)] + ec[cube_at(x1, y0, z1, cn)] +
-                                      ec[cube_at(x0, y1, z1, cn)] + ec[cube_at(x1, y1, z1, cn)]);
-            e[cube_at(x, y, z, n)] += sm[lay.fac[l] + tid] * v;
-        }
-        __syncthreads();
-        cube_relax(sm + lay.coef[l], sm + lay.invD[l], sm + lay.rhs[l], e, n, l == 0 ? post : inner);
+    __syncthreads();
+    const int last = lay.count - 1;
+    int copy9[2] = {0, 0}, copy5[2] = {0, 0};
+    if (lay.n[0] == 9) {
+        cube_relax<9>(cubes.nine, v, 0, copy9, pre, true);
+        cube_residual<9>(cubes.nine, v, 0, copy9);
+        if (v.level == 1) v.rhs = cube_restrict<9>(cubes.nine, v.x, v.y, v.z);
     }
-    const int n = lay.n[0];
-    if (tid < n * n * n) {
-        int x, y, z;
-        unflatten(tid, n, x, y, z);
-        e0[g0.at(x, y, z)] = sm[lay.e[0] + cube_at(x, y, z, n)];
+    const int level5 = lay.count - 2;  // -1: none
+    if (level5 >= 0) {
+        cube_relax<5>(cubes.five, v, level5, copy5, level5 == 0 ? pre : inner, true);
+        cube_residual<5>(cubes.five, v, level5, copy5);
+        if (v.level == last) v.rhs = cube_restrict<5>(cubes.five, v.x, v.y, v.z);
     }
+    const int own3 = (v.z * 3 + v.y) * 3 + v.x;
+    if (v.level == last) rhs3[own3] = (double)v.rhs;
+    __syncthreads();
+    if (v.level == last) {  // side 3: e = A^-1 rhs
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < kInvN; ++j) sum += inverse[own3 * kInvN + j] * rhs3[j];
+        e3[own3] = v.e = (float)sum;
+    }
+    __syncthreads();
+    if (level5 >= 0) {
+        cube_prolong<5>(cubes.five, v, level5, copy5, [&](int x, int y, int z) { return e3[(z * 3 + y) * 3 + x]; });
+        cube_relax<5>(cubes.five, v, level5, copy5, level5 == 0 ? post : inner, false);
+    }
+    if (lay.n[0] == 9) {
+        cube_prolong<9>(cubes.nine, v, 0, copy9, [&](int x, int y, int z) {
+            const int c = Cube<5>::at(x, y, z);
+            return cubes.five.e[c & 1][copy5[c & 1]][c >> 1];
+        });
+        cube_relax<9>(cubes.nine, v, 0, copy9, post, false);
+    }
+    if (v.level == 0) e0[g0.at(v.x, v.y, v.z)] = v.e;
 }
 
-__global__ void __launch_bounds__(kC27Threads) coarse27_kernel(const float4* __restrict__ image, CoarseLayout lay,
+__global__ void __launch_bounds__(kC27Threads) coarse27_kernel(const float* __restrict__ image, CoarseLayout lay,
                                                                const float* __restrict__ rhs0,
                                                                float* __restrict__ e0, Geom g0, int pre, int post,
                                                                int inner) {
@@ -1034,7 +1064,7 @@ __global__ void __launch_bounds__(kC27Threads) coarse27_grouped_kernel(const bat
     int bx, by, bz;
     const batch::GridDesc& d = batch::locate(descs, count, blockIdx.x, bx, by, bz);
     if (!batch::cloud_active(flags, d.cloud)) return;
-    coarse27_body((const float4*)d.ptr[0], lay, (const float*)d.ptr[1], (float*)d.ptr[2], geom((int)d.n),
+    coarse27_body((const float*)d.ptr[0], lay, (const float*)d.ptr[1], (float*)d.ptr[2], geom((int)d.n),
                   (int)d.aux[0], (int)d.aux[1], (int)d.aux[2]);
 }
 
@@ -1140,7 +1170,7 @@ extern "C" int pb_level27_finish_f32(const float* coef, int64_t n, float* invD, 
 // Inverse (27 x 27, FP32 row-major) of a 27-point level of side 3.
 extern "C" int pb_coarse_inverse_f64(const float* coef, int64_t n, double* inverse, void* stream) {
     if (n != 3 || !coef || !inverse) return fail(PB_ERR_INVALID, "coarse inverse: side must be 3");
-    coarse_inverse_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(coef, padded_size(3), geom(3), inverse);
+    coarse_inverse_kernel<<<1, 32 * kInvN, 0, (cudaStream_t)stream>>>(coef, padded_size(3), geom(3), inverse);
     PB_CHECK_LAUNCH("coarse_inverse_kernel");
     return PB_OK;
 }
@@ -1203,12 +1233,8 @@ extern "C" int pb_coarse27_cycle_f32(int64_t count, const int64_t* sizes, const 
     if (pre < 0 || post < 0 || inner < 0 || pre > 64 || post > 64 || inner > 64)
         return fail(PB_ERR_INVALID, "coarse27 cycle: sweep counts must be in [0, 64]");
     const CoarseLayout lay = coarse_layout((int)count, sz);
-    const size_t smem = (size_t)lay.total * sizeof(float);
-    PB_CHECK_CUDA(cudaFuncSetAttribute(coarse27_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                  "coarse27 smem");
-    coarse27_kernel<<<1, kC27Threads, smem, (cudaStream_t)stream>>>(reinterpret_cast<const float4*>(image), lay,
-                                                                     rhs, e, geom(sz[0]), (int)pre, (int)post,
-                                                                     (int)inner);
+    coarse27_kernel<<<1, kC27Threads, 0, (cudaStream_t)stream>>>(image, lay, rhs, e, geom(sz[0]), (int)pre, (int)post,
+                                                                  (int)inner);
     PB_CHECK_LAUNCH("coarse27_kernel");
     return PB_OK;
 }
@@ -1387,10 +1413,7 @@ int launch_coarse27(const GridDesc* descs, int count, int64_t blocks, int first_
     }
     if (sz[levels - 1] != 3) return fail(PB_ERR_INVALID, "batch coarse27: first side must be 9, 5 or 3");
     const CoarseLayout lay = coarse_layout(levels, sz);
-    const size_t smem = (size_t)lay.total * sizeof(float);
-    PB_CHECK_CUDA(cudaFuncSetAttribute(coarse27_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                  "batch coarse27 smem");
-    coarse27_grouped_kernel<<<(unsigned)blocks, kC27Threads, smem, s>>>(descs, count, flags, lay);
+    coarse27_grouped_kernel<<<(unsigned)blocks, kC27Threads, 0, s>>>(descs, count, flags, lay);
     PB_CHECK_LAUNCH("coarse27_grouped_kernel");
     return PB_OK;
 }
