@@ -171,57 +171,82 @@ struct Cells {  // the occupied cells
 
 // Touched nodes: (occupied cell, corner) pairs whose cell is the first occupied one around the
 // node.  A node's slot in the list and its place among the contributions come from counters, warp
-// by warp: their order changes from run to run, the contents of a slot do not.
+// by warp: their order changes from run to run, the contents of a slot do not.  A thread takes a
+// cell with its 27 neighbours (their lookups serve all eight corners, and consecutive cells of a
+// row share sectors): bound by L1 lookups, 1M points at 257^3 71 us with a thread per corner, now 18.
 struct Nodes {
     uint32_t *node, *base, *length;
     uint32_t* slot_of;  // dense node -> slot + 1 (may be null)
     uint32_t* counters;  // slots, contributions
 };
 
-__global__ void __launch_bounds__(256) touched_nodes_kernel(Cells g, const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(128) touched_nodes_kernel(Cells g, const uint32_t* __restrict__ keys,
                                                             const uint32_t* __restrict__ cells, Nodes out) {
-    const uint64_t total = 8ull * *cells, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t total = *cells, stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t - lane < total; t += stride) {
-        uint32_t node = 0, length = 0;
+        uint32_t node = 0, points[27], owned = 0, sum = 0;  // points of the cells around; owned corners
         if (t < total) {
-            const uint32_t cell = keys[g.heads[t >> 3]], corner = (uint32_t)t & 7;
-            const uint32_t row = g.by_c.div(cell), cz = g.by_c.div(row);
-            const uint32_t x = cell - row * g.c + (corner & 1), y = row - cz * g.c + ((corner >> 1) & 1),
-                           z = cz + (corner >> 2);
+            const uint32_t cell = keys[g.heads[t]];
+            const uint32_t row = g.by_c.div(cell), z = g.by_c.div(row), y = row - z * g.c, x = cell - row * g.c;
             node = (z * g.n + y) * g.n + x;
-            uint32_t r[8];  // the cells around the node, whose corner k it is of cell node - k
 #pragma unroll
-            for (int k = 0; k < 8; ++k) r[k] = g.at(x - (k & 1), y - ((k >> 1) & 1), z - (k >> 2));
-            bool owner = true;  // no occupied cell before this one: cells ascend as k descends
+            for (int k = 0; k < 27; ++k) points[k] = g.at(x + (k % 3 - 1), y + (k / 3 % 3 - 1), z + (k / 9 - 1));
 #pragma unroll
-            for (int k = 0; k < 8; ++k) owner = owner && (k <= (int)corner || r[k] == 0);
-            if (owner)
+            for (int k = 0; k < 27; ++k)
+                if (points[k]) points[k] = g.heads[points[k]] - g.heads[points[k] - 1];
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (r[k]) length += g.heads[r[k]] - g.heads[r[k] - 1];
+            for (int corner = 0; corner < 8; ++corner) {
+                // the cells around the corner's node, whose corner k it is; they ascend as k descends, and the
+                // node is the cell's own if none occupied comes before it
+                uint32_t length = 0, before = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const uint32_t v = points[((corner & 1) - (k & 1) + 1) + 3 * (((corner >> 1) & 1) - ((k >> 1) & 1) + 1) +
+                                              9 * ((corner >> 2) - (k >> 2) + 1)];
+                    length += v;
+                    if (k > corner) before |= v;
+                }
+                if (before == 0) {
+                    owned |= 1u << corner;
+                    sum += length;
+                }
+            }
         }
-        uint32_t sum = length;  // inclusive over the warp
+        const uint32_t nodes = __popc(owned);
+        uint32_t slots = nodes, contributions = sum;  // inclusive over the warp
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
-            if (lane >= o) sum += v;
+            const uint32_t a = __shfl_up_sync(0xffffffffu, slots, o), b = __shfl_up_sync(0xffffffffu, contributions, o);
+            if (lane >= o) {
+                slots += a;
+                contributions += b;
+            }
         }
-        const unsigned mine = __ballot_sync(0xffffffffu, length != 0);
         uint32_t slot0 = 0, base0 = 0;
-        if (lane == 31 && mine) {
-            slot0 = atomicAdd(out.counters, (uint32_t)__popc(mine));
-            base0 = atomicAdd(out.counters + 1, sum);
+        if (lane == 31 && slots) {
+            slot0 = atomicAdd(out.counters, slots);
+            base0 = atomicAdd(out.counters + 1, contributions);
         }
-        slot0 = __shfl_sync(0xffffffffu, slot0, 31);
-        base0 = __shfl_sync(0xffffffffu, base0, 31);
-        if (length) {
-            const uint32_t slot = slot0 + __popc(mine & ((1u << lane) - 1u));
-            out.node[slot] = node;
-            out.base[slot] = base0 + sum - length;
-            out.length[slot] = length;
-            if (out.slot_of) out.slot_of[node] = slot + 1;
-        }
+        uint32_t slot = __shfl_sync(0xffffffffu, slot0, 31) + slots - nodes;
+        uint32_t base = __shfl_sync(0xffffffffu, base0, 31) + contributions - sum;
+        if (owned)
+#pragma unroll
+            for (int corner = 0; corner < 8; ++corner)
+                if (owned >> corner & 1u) {
+                    uint32_t length = 0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        length += points[((corner & 1) - (k & 1) + 1) + 3 * (((corner >> 1) & 1) - ((k >> 1) & 1) + 1) +
+                                         9 * ((corner >> 2) - (k >> 2) + 1)];
+                    const uint32_t at = node + (corner & 1) + ((corner >> 1) & 1) * g.n + (corner >> 2) * g.n * g.n;
+                    out.node[slot] = at;
+                    out.base[slot] = base;
+                    out.length[slot] = length;
+                    if (out.slot_of) out.slot_of[at] = slot + 1;
+                    ++slot;
+                    base += length;
+                }
     }
 }
 
@@ -392,7 +417,17 @@ __global__ void __launch_bounds__(256) assemble_compact_kernel(const uint32_t* _
 // Each sample's k attributes are splatted with its pass-1 weights w (the
 // screening weights), per node in sample order: sum w a_c for c < k and, last,
 // sum w.  One thread per (node, channel); DENSE: into planes of n^3, else rows of
-// k + 1 per slot.
+// k + 1 per slot, from attributes in the points' sorted order (gather_attributes_kernel):
+// the walk waits on its loads, and `order` would be one more in the chain of each.
+__global__ void __launch_bounds__(256) gather_attributes_kernel(const double* __restrict__ attributes,
+                                                                const uint32_t* __restrict__ order, int64_t count,
+                                                                uint32_t channels, double* __restrict__ sorted) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (uint64_t)count * channels) return;
+    const uint32_t place = (uint32_t)(i / channels), c = (uint32_t)(i - (uint64_t)place * channels);
+    sorted[i] = attributes[(uint64_t)order[place] * channels + c];
+}
+
 template <bool DENSE>
 __global__ void __launch_bounds__(256) attribute_sums_kernel(Nodes nodes, const uint32_t* __restrict__ list,
                                                              const Frac* __restrict__ frac,
@@ -410,7 +445,7 @@ __global__ void __launch_bounds__(256) attribute_sums_kernel(Nodes nodes, const 
             const uint32_t item = in[t], place = item & ((1u << kPlaceBits) - 1u);
             const Frac f = load32(frac + place);
             const double w = corner_weight(f.x, f.y, f.z, f.weight, (int)(item >> kPlaceBits));
-            if (f.weight != 0.0) sum += c < channels ? w * attributes[(int64_t)order[place] * channels + c] : w;
+            if (f.weight != 0.0) sum += c < channels ? w * attributes[(int64_t)(DENSE ? order[place] : place) * channels + c] : w;
         }
         sums[DENSE ? c * plane + nodes.node[slot] : i] = sum;
     }
@@ -561,7 +596,7 @@ struct Splat {
         PB_TRY(exclusive_scan<uint32_t>(rank, rank, count, cells, w, s));
         cell_table_kernel<<<blocks, 256, 0, s>>>(keys, rank, count, cells, heads, table);
         PB_CHECK_LAUNCH("cell_table_kernel");
-        touched_nodes_kernel<<<(unsigned)std::min<int64_t>(blocks_for(8 * count, 256), 16 * kSMs), 256, 0, s>>>(
+        touched_nodes_kernel<<<(unsigned)std::min<int64_t>(blocks_for(count, 128), 32 * kSMs), 128, 0, s>>>(
             geometry(), keys, cells, nodes);
         PB_CHECK_LAUNCH("touched_nodes_kernel");
         return PB_OK;
@@ -718,6 +753,7 @@ static size_t interpolate_ws_bytes(int64_t count, int64_t n, int64_t channels) {
         const int64_t cap = Splat::node_capacity(count, n);
         o.carve(w, count, cap, cubed(n - 1), cubed(n), false);
         w.take<double>(cap * (channels + 1));
+        w.take<double>(count * channels);
         Splat::carve_scratch(w, count);
     });
 }
@@ -806,11 +842,15 @@ extern "C" int pb_interpolate_attributes_f64(const double* points, const double*
     Splat o;
     o.carve(w, point_count, cap, cubed(n - 1), cubed(n), false);
     double* sums = w.take<double>(cap * (channels + 1));
+    double* sorted = w.take<double>(point_count * channels);
     PB_TRY(o.group(points, normals, n, (int)confidence, w, s));
     merge_kernel<false><<<o.node_blocks(), 256, 0, s>>>(o.geometry(), o.nodes, o.vals, o.frac, o.list, nullptr, nullptr);
     PB_CHECK_LAUNCH("merge_kernel");
+    gather_attributes_kernel<<<blocks_for(point_count * channels, 256), 256, 0, s>>>(attributes, o.vals, point_count,
+                                                                                    (uint32_t)channels, sorted);
+    PB_CHECK_LAUNCH("gather_attributes_kernel");
     attribute_sums_kernel<false><<<o.node_blocks((int)channels + 1), 256, 0, s>>>(
-        o.nodes, o.list, o.frac, o.vals, attributes, (uint32_t)channels, 0, sums);
+        o.nodes, o.list, o.frac, nullptr, sorted, (uint32_t)channels, 0, sums);
     PB_CHECK_LAUNCH("attribute_sums_kernel");
     sample_slots_kernel<<<blocks_for(vertex_count * channels, 256), 256, 0, s>>>(
         vertices, vertex_count, map, n, o.nodes.slot_of, sums, (uint32_t)channels, out);
