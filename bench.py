@@ -405,7 +405,7 @@ def kernel_rooflines(eng, n: int, L) -> list:
            (("sweep", 7), ("restrict", 8), ("direction", 5), ("update", 6))}  # PB_TUNE_*_VARIANT
     rr_name = {2: "tma::residual_restrict_tma_kernel", 3: "residual_restrict32_wide_kernel"}.get(
         var["restrict"], "residual_restrict32_kernel")
-    dir_name = f"fcg::direction_sums_kernel<{(4, 6, 8)[var['direction']]}>"
+    dir_name = f"fcg::direction_sums_kernel<{(6, 4, 8)[var['direction']]}>"
     upd_name = f"fcg::update_residual_prefetch_kernel<24, {4 if var['update'] == 4 else 3}>"
     rr_at = len(out)
     rr_args = (l0.ea.data_ptr(), l0.rhs.data_ptr(), l0.D.data_ptr(), l0.weights.data_ptr(), l1.rhs.data_ptr(), n)
@@ -414,18 +414,19 @@ def kernel_rooflines(eng, n: int, L) -> list:
               16 * N + 4 * N1)
     else:
         timed(f"{rr_name} (level 0)", lambda s: L.pb_residual_restrict_f32(*rr_args, s), 16 * N + 4 * N1)
-    timed("prolong_add32_kernel (level 0)", lambda s: L.pb_prolong_fac_f32(
-        l1.ea.data_ptr(), l0.eb.data_ptr(), l0.weights.data_ptr(), n, s), 12 * N + 4 * N1)
+    # b, the screen and the weights are read only around the samples: their bytes are not counted
+    timed("prolong_add32_kernel (level 0)", lambda s: L.pb_prolong_fac_sparse_f32(
+        l1.ea.data_ptr(), l0.eb.data_ptr(), l0.weights.data_ptr(), h.where, n, s), 8 * N + 4 * N1)
     timed("relax27p_kernel x2 (one sweep, level 1, packed FP16)", lambda s: L.pb_relax27p_f32(
         l1.ea.data_ptr(), l1.eb.data_ptr(), l1.rhs.data_ptr(), *l1.packed_ptrs(), l1.n, s), 68 * N1)
-    timed(dir_name, lambda s: L.pb_fcg_direction_f64(
-        l0.ea.data_ptr(), p0, p1, l0.rhs.data_ptr(), eng.screen.data_ptr(), n, eng.pw,
-        eng.scal.data_ptr(), eng.flags.data_ptr(), eng.ws_ptr, eng.ws_size, s), 20 * N)
+    timed(dir_name, lambda s: L.pb_fcg_direction_sparse_f64(
+        l0.ea.data_ptr(), p0, p1, l0.rhs.data_ptr(), eng.screen.data_ptr(), h.where, n, eng.pw,
+        eng.scal.data_ptr(), eng.flags.data_ptr(), eng.ws_ptr, eng.ws_size, s), 12 * N)
     if n == 257 and var["restrict"] != 2:  # the committed capture is of the per-thread-load kernels
         out[rr_at]["traffic"] = read_profile_traffic(RESTRICT_PROFILE)
-    timed(upd_name, lambda s: L.pb_fcg_update_f64(
-        l0.ea.data_ptr(), p0, p1, x0, x1, eng.b.data_ptr(), eng.screen.data_ptr(),
-        l0.rhs.data_ptr(), n, eng.pw, eng.scal.data_ptr(), eng.flags.data_ptr(), eng.ws_ptr, eng.ws_size, s), 48 * N)
+    timed(upd_name, lambda s: L.pb_fcg_update_sparse_f64(
+        l0.ea.data_ptr(), p0, p1, x0, x1, eng.b.data_ptr(), eng.screen.data_ptr(), h.where,
+        l0.rhs.data_ptr(), n, eng.pw, eng.scal.data_ptr(), eng.flags.data_ptr(), eng.ws_ptr, eng.ws_size, s), 32 * N)
     h.check_status()
     return out
 

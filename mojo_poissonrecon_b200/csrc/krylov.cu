@@ -139,7 +139,7 @@ __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z,
         const int64_t nn = (int64_t)n * n;
         const int inside = min(kW, n - x);
         int64_t i = (int64_t)z0 * nn + (int64_t)y * n + x, c = g.at(x, y, z0);
-        uint32_t some = plane_bits(occupied, n, x, y, z0);
+        int some = (int)plane_bits(occupied, n, x, y, z0);  // signed: without a map the shifts leave it all ones
         double zb[kW], zm[kW];
         widen(wide<ALIGNED>(z + c - g.plane), zb);
         widen(wide<ALIGNED>(z + c), zm);
@@ -153,7 +153,7 @@ __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z,
                 for (int j = 0; j < kW; ++j)
                     if (j < inside) prev[j] = pp[i + j];
             double sc[kW] = {};
-            if (some & 1u)
+            if (some & 1)
 #pragma unroll
                 for (int j = 0; j < kW; ++j)
                     if (j < inside) sc[j] = screen[i + j];
@@ -334,6 +334,9 @@ __device__ __forceinline__ void update_residual_prefetch_body(
     // planes of the block where a warp's row of the tile has b or screening
     const uint32_t some =
         y < n ? plane_bits(occupied, n, bx, y, z0) & (0xffffffffu >> max(0, 32 - (z1 - z0))) : 0u;
+    auto has_source = [&](int k) -> bool {  // deeper blocks than a word come without a map: every bit set
+        return TZC > 0 && TZC <= 32 ? some >> (k - z0) & 1u : (int)some >> min(k - z0, 31) & 1;
+    };
     // A slot that nothing is copied to holds zeros: nodes outside the domain, and p in the first step.
     for (int sl = 0; sl < RING; ++sl) {
         if (!inside) rd[sl][0][tid] = 0.0, rf[sl][0][tid] = 0.0f;
@@ -352,7 +355,7 @@ __device__ __forceinline__ void update_residual_prefetch_body(
             cp_async8(&rd[sl][0][tid], xc + dense + e);
             cp_async4(&rf[sl][0][tid], z + padded + q);
             if (!first) cp_async4(&rf[sl][1][tid], pp + dense + e);
-            if (k < z1 && ((some >> (k - z0)) & 1u)) {
+            if (k < z1 && has_source(k)) {
                 cp_async8(&rd[sl][1][tid], b + dense + e);
                 cp_async8(&rd[sl][2][tid], screen + dense + e);
             }
@@ -396,7 +399,7 @@ __device__ __forceinline__ void update_residual_prefetch_body(
         if (inside) {
             const double s = tile[ty + 1][tx] + tile[ty + 1][tx + 2] + tile[ty][tx + 1] + tile[ty + 2][tx + 1] + xb + xa;
             double bi = 0.0, d = up && k > 0 ? d_mid : d_end;
-            if ((some >> (k - z0)) & 1u) {
+            if (has_source(k)) {
                 bi = rd[sk][1][tid];
                 d = __fma_rn(__dmul_rn(pw, rd[sk][2][tid]), h2, d);
             }

@@ -3,8 +3,8 @@
 Reference: python/mojo_poissonrecon/core.py:141-193 (_v_cycle) and :267-296
 (hierarchy, cycle loop, final residual).  The reference keeps one NumPy grid
 per level and drives the native kernels level by level; here the hierarchy
-lives in HBM as torch tensors and every operator is a libpoisson_b200 kernel
-on one CUDA stream.
+lives in HBM as torch tensors, by colour from side 33 up, and all cycles of a solve
+are queued on one CUDA stream by one library call (pb_vcycles_f64).
 
 Two solve modes:
 

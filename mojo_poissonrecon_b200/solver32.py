@@ -4,11 +4,11 @@ FCG(1) (the default, ``RefinedEngine``): the FP32 V-cycle preconditions FP64
 flexible conjugate gradients:
 
     x = 0.5                                  (the reference's initial guess, core.py:270)
-    r = b - A x                              FP64 (pb_defect_f64)
+    r = b - A x                              FP64 (pb_refine_start_sparse_f64)
     while ||r|| > tol * ||b||:               evaluated on the device
         z = V-cycle on A e = r, e = 0        FP32
-        p = z - beta p;  x += alpha p;  r = b - A x                 FP64 (pb_fcg_direction_f64,
-                                                                         pb_fcg_update_f64;
+        p = z - beta p;  x += alpha p;  r = b - A x                 FP64 (pb_fcg_direction_sparse_f64,
+                                                                         pb_fcg_update_sparse_f64;
                                                                          p stored in FP32)
 
 One iteration touches the same buffers every time, so the engine captures it
@@ -30,7 +30,7 @@ operators with screening-scaled transfers (mg27.cu), smoothed by
 COARSE_SWEEPS sweeps each way (on levels of side > 9 with their couplings
 packed per colour in FP16), which cut the cycles needed for a given residual
 2-4x against the reference's rediscretised hierarchy.  Levels of side <= 9
-run in a single launch from shared memory, the 3^3 level solved exactly with
+run in a single launch of one block, the 3^3 level solved exactly with
 its inverse (built once per set-up).  Convergence is always measured with the
 reference's FP64 operator.
 """

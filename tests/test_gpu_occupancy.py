@@ -116,3 +116,52 @@ def test_sparse_passes_match_dense(L, n, kind):
         assert status == 0
         got.append(coef.view(torch.int32))
     assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("kind", ("shell", "all"))
+def test_planes_beyond_a_word(L, kind):
+    """Blocks deeper than the 32 planes of a word read everything: pass 2 per node as ever, pass 1's sums to rounding."""
+    from mojo_poissonrecon_b200 import tune
+
+    n, s = 129, torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(3)
+    dev = lambda a, t=torch.float64: torch.from_numpy(np.ascontiguousarray(a)).to(t).cuda()
+    b, screen = (dev(a) for a in system(n, 5, kind))
+    pitch, count = geometry(L, n)
+    D, invD, weights, r32, zp = (torch.zeros(count, dtype=torch.float32, device="cuda") for _ in range(5))
+    zp.view(n + 2, n + 2, pitch)[1:-1, 1:-1, 4:4 + n].copy_(dev(rng.normal(size=(n, n, n)), torch.float32))
+    norms = torch.empty(2, dtype=torch.float64, device="cuda")
+    ws = torch.empty(max(L.pb_refine_start_workspace_size(n), L.pb_fcg_workspace_size(n)), dtype=torch.uint8,
+                     device="cuda")
+    occupancy = torch.empty(L.pb_occupancy_size(n) // 4, dtype=torch.int32, device="cuda")
+    x0 = torch.empty_like(b)
+    assert L.pb_refine_start_sparse_f64(b.data_ptr(), screen.data_ptr(), n, 4.0, None, None, x0.data_ptr(),
+                                        D.data_ptr(), invD.data_ptr(), weights.data_ptr(), r32.data_ptr(),
+                                        occupancy.data_ptr(), norms.data_ptr(), norms.data_ptr() + 8, ws.data_ptr(),
+                                        ws.numel(), s) == 0
+    ps = [dev(rng.normal(size=(n, n, n)), torch.float32) for _ in range(2)]
+    xs = [dev(rng.normal(size=(n, n, n))) for _ in range(2)]
+    flags = torch.tensor([0, 1, 0, 0], dtype=torch.int32, device="cuda")
+    got = []
+    for planes in (0, 48):
+        if planes:
+            L.pb_tune_set(tune.FCG_DIRECTION_PLANES, n, planes)
+            L.pb_tune_set(tune.FCG_UPDATE_PLANES, n, planes)
+        try:
+            p, xx, r = [t.clone() for t in ps], [t.clone() for t in xs], r32.clone()
+            sums, scal = (torch.full((8,), 3.0, dtype=torch.float64, device="cuda") for _ in range(2))
+            assert L.pb_fcg_direction_sparse_f64(zp.data_ptr(), p[0].data_ptr(), p[1].data_ptr(), r.data_ptr(),
+                                                 screen.data_ptr(), occupancy.data_ptr(), n, 4.0, sums.data_ptr(),
+                                                 flags.data_ptr(), ws.data_ptr(), ws.numel(), s) == 0
+            assert L.pb_fcg_update_sparse_f64(zp.data_ptr(), p[0].data_ptr(), p[1].data_ptr(), xx[0].data_ptr(),
+                                              xx[1].data_ptr(), b.data_ptr(), screen.data_ptr(), occupancy.data_ptr(),
+                                              r.data_ptr(), n, 4.0, scal.data_ptr(), flags.data_ptr(), ws.data_ptr(),
+                                              ws.numel(), s) == 0
+            got.append(([*p, *xx, r], sums[:4].cpu().numpy()))
+        finally:
+            L.pb_tune_set(tune.FCG_DIRECTION_PLANES, n, 0)
+            L.pb_tune_set(tune.FCG_UPDATE_PLANES, n, 0)
+    for a, c in zip(got[0][0], got[1][0]):
+        assert torch.equal(a, c)
+    # sums of 2.1M products in another order: relative 2.1e6 eps of their magnitudes at the very most
+    assert np.allclose(got[0][1], got[1][1], rtol=1e-9, atol=0)
