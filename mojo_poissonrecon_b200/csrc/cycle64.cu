@@ -45,7 +45,8 @@ __device__ __forceinline__ double reciprocal(double d) {
 // and 3 run on the first 384, 64 and 32 threads (their nodes of one colour)
 // with named barriers of that many threads.  Measured on B200: a depth-5
 // reconstruction of 2,000 points (five cycles) 3.56 -> 1.21 ms, 13,337 points
-// at depth 6 (four cycles) 3.38 -> 1.48 ms.
+// at depth 6 (four cycles) 3.38 -> 1.48 ms; 0.9 and 1.2 ms since 33^3 and 17^3 run
+// in a cluster (below), which leaves this kernel the devices that cannot place one.
 //
 // A side is odd, so the colour of a node is the lowest bit of its linear index i
 // and its six neighbours (i +- 1, i +- N, i +- N^2) have the other colour: each

@@ -322,9 +322,9 @@ __global__ void __launch_bounds__(128) galerkin_z_kernel(const float* __restrict
 
 // The same product for a small coarse level, one warp per coarse node: a lane takes one
 // fine node i of the support, contracts its 27 couplings axis by axis with the weights
-// P(o + d - 2m) of its own place, and the lanes' sums are added.  The three stages
-// take 6 to 8 us each however small the level; this takes as long as one of them up to
-// coarse side 17 (4,913 warps), and more than all three at 33 (35,937).
+// P(o + d - 2m) of its own place, and the lanes' sums are added.  Below some size the
+// three stages take 6 to 8 us each however small the level; this takes 12 us at coarse
+// side 17 and 5 below it, but 55 at 33 against 37 for the stages.
 constexpr int kSmallCoarse = 17;
 
 __global__ void __launch_bounds__(128) galerkin_small_kernel(const float* __restrict__ c, int64_t cs,
