@@ -118,7 +118,7 @@ __global__ void sum_partials_kernel(const double* __restrict__ partial, int coun
 // degree / 2, exactly, so no neighbour is read.  Threads flattened over a plane's
 // (x, y), a few planes each.  Bound by memory: 16 bytes read and 24 (40 with the
 // copies) written per node, against 108 of the two dense copies, level set-up, fill,
-// defect and norm that it replaces (257^3: 390 -> 221 us).
+// defect and norm that it replaces (257^3: 390 -> 209 us, the occupancy words included).
 constexpr int kStartZ = 8;
 
 __global__ void __launch_bounds__(256, 4) refine_start_kernel(const double* __restrict__ rhs,
