@@ -10,7 +10,8 @@
 // value: the same additions, in the same order, as the reference.  The merge
 // leaves the node's contributions (sorted place of the point, corner) as a list,
 // which pass 2 (both passes address the same eight nodes per sample) and the
-// attribute sums then only walk.
+// attribute sums then only walk.  Where points crowd, a node's long list is put in
+// order and summed by many threads (below: long lists).
 //
 // Against one record per (point, corner) sorted by node and five dense grids
 // (B200, 1M noisy points at depth 8): the sort handles 1M keys instead of 8M (370 ->
@@ -177,8 +178,21 @@ struct Cells {  // the occupied cells
 struct Nodes {
     uint32_t *node, *base, *length;
     uint32_t* slot_of;  // dense node -> slot + 1 (may be null)
-    uint32_t* counters;  // slots, contributions
+    uint32_t* counters;  // slots, contributions, units, long lists
+    uint2* units;        // (slot, part) of the long lists, kUnit contributions each
+    uint32_t* longs;     // slots of the long lists
+    uint32_t long_over;  // a list is long beyond this many contributions (long_over_of)
 };
+constexpr uint32_t kUnit = 256;
+
+// Where a list counts as long.  One thread per list waits for its loads, which only many
+// lists side by side hide, and the larger the grid the more nodes a surface touches; a
+// block per list costs a few microseconds however short the list.  Splat and assembly,
+// us, with the line at 64 / 128 / 512: 100,000 points at 33^3 211 / 273 / 363; 200,000 at
+// 65^3 329 / 279 / 277, a million 860 / 881 / 1,056; a million at 129^3 1,048 / 887 / 567,
+// two million 1,788 / 1,744 / 1,021; at 257^3 four million 4,116 / 3,268 / 1,708.
+constexpr uint32_t kLongOver = 64;  // the least of them
+static uint32_t long_over_of(int64_t n) { return n <= 33 ? kLongOver : n <= 65 ? 128 : 512; }
 
 __global__ void __launch_bounds__(128) touched_nodes_kernel(Cells g, const uint32_t* __restrict__ keys,
                                                             const uint32_t* __restrict__ cells, Nodes out) {
@@ -244,23 +258,141 @@ __global__ void __launch_bounds__(128) touched_nodes_kernel(Cells g, const uint3
                     out.base[slot] = base;
                     out.length[slot] = length;
                     if (out.slot_of) out.slot_of[at] = slot + 1;
+                    if (length > out.long_over) {
+                        out.longs[atomicAdd(out.counters + 3, 1u)] = slot;
+                        const uint32_t parts = (length + kUnit - 1) / kUnit, first = atomicAdd(out.counters + 2, parts);
+                        for (uint32_t part = 0; part < parts; ++part) out.units[first + part] = make_uint2(slot, part);
+                    }
                     ++slot;
                     base += length;
                 }
     }
 }
 
-// Merges each node's lists into its contributions, (sorted point | corner << 29) in point order,
-// and, SUMS, adds pass 1 (capi.mojo:171-172): density += 2w, screen += w.  Cursors, current and next
-// point of all eight lists stay in registers; the next point is read an addition ahead.
 constexpr uint32_t kPlaceBits = 29, kNone = 0xFFFFFFFFu;
 
+// ---- long lists -------------------------------------------------------------------
+// One thread's walk waits for its loads at every contribution, which many short lists
+// hide and a long one does not (a million points at depth 3: lists of 30,000).  A long
+// list is put in order by ranks: a contribution's place is the number of points before
+// it in each of the eight sorted lists, all searched at once, a thread per contribution.
+// Its sums keep the reference's order, one addition after another, but only the
+// additions wait for each other: seven warps of a block read the contributions and form
+// their values in shared memory a tile ahead of the threads that add them.
+// Splat and assembly of a million points, one thread per list -> this: at depth 2 338 ->
+// 4.1 ms, 3 82 -> 1.4, 4 18.3 -> 0.95, 5 4.5 -> 0.85; half of them in a thousandth of
+// the surface, at depth 6, 468 -> 6.4.  What is left is the chain of additions of the
+// longest list.
+
+// Part unit.y of the list of slot unit.x.
+__device__ __forceinline__ void rank_unit(const Cells& g, const Nodes& nodes, const uint32_t* __restrict__ order,
+                                          uint32_t* __restrict__ list, uint2 unit) {
+    const uint32_t node = nodes.node[unit.x], row = g.by_n.div(node), z = g.by_n.div(row), x = node - row * g.n,
+                   y = row - z * g.n;
+    uint32_t start[8], size[8], most = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t r = g.at(x - (k & 1), y - ((k >> 1) & 1), z - (k >> 2));
+        start[k] = r ? g.heads[r - 1] : 0u;
+        size[k] = r ? g.heads[r] - start[k] : 0u;
+        most = max(most, size[k]);
+    }
+    uint32_t left = unit.y * kUnit + threadIdx.x, place = kNone, corner = 0;  // of the lists one after another
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (place == kNone) {
+            if (left < size[k]) {
+                place = start[k] + left;
+                corner = k;
+            } else {
+                left -= size[k];
+            }
+        }
+    if (place == kNone) return;  // past the last list
+    const uint32_t point = order[place];
+    uint32_t before[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (uint32_t step = 0x80000000u >> __clz(most); step; step >>= 1)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t at = before[k] + step;
+            if (at <= size[k] && order[start[k] + at - 1] < point) before[k] = at;
+        }
+    uint32_t rank = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) rank += before[k];
+    list[nodes.base[unit.x] + rank] = place | corner << kPlaceBits;
+}
+
+constexpr int kAhead = 224;  // contributions of a tile: one per thread of the seven reading warps
+
+// acc + the list's values of chain threadIdx.x, in order, in the first CHAINS threads (of 256);
+// values(contribution, v): its value in each chain.
+template <int CHAINS, typename Values>
+__device__ __forceinline__ double add_in_order(const uint32_t* __restrict__ in, uint32_t length, double acc,
+                                               Values&& values) {
+    __shared__ double tiles[2][CHAINS][kAhead];
+    const int reader = (int)threadIdx.x - 32;
+    const uint32_t count = (length + kAhead - 1) / kAhead;
+    for (uint32_t t = 0; t <= count; ++t) {  // tile t is read while tile t - 1 is added
+        if (reader >= 0) {
+            const uint32_t i = t * kAhead + reader;
+            if (i < length) {
+                double v[CHAINS];
+                values(in[i], v);
+#pragma unroll
+                for (int c = 0; c < CHAINS; ++c) tiles[t & 1][c][reader] = v[c];
+            }
+        } else if (t > 0 && threadIdx.x < CHAINS) {
+            const double* v = tiles[(t - 1) & 1][threadIdx.x];
+            const uint32_t n = min((uint32_t)kAhead, length - (t - 1) * kAhead);
+#pragma unroll 16
+            for (uint32_t j = 0; j < n; ++j) acc += v[j];
+        }
+        __syncthreads();
+    }
+    return acc;
+}
+
+// Pass 1 (capi.mojo:171-172) of the long lists.
+__global__ void __launch_bounds__(256) long_sums_kernel(Nodes nodes, const uint32_t* __restrict__ list,
+                                                        const Frac* __restrict__ frac, double* __restrict__ density,
+                                                        double* __restrict__ screen) {
+    const uint32_t count = nodes.counters[3];
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t slot = nodes.longs[i];
+        double* grid = threadIdx.x == 0 ? density : screen;
+        const uint32_t node = nodes.node[slot];
+        const double acc = add_in_order<2>(list + nodes.base[slot], nodes.length[slot],
+                                           threadIdx.x < 2 ? grid[node] : 0.0, [&](uint32_t item, double (&v)[2]) {
+                                               const Frac f = load32(frac + (item & ((1u << kPlaceBits) - 1u)));
+                                               v[1] = corner_weight(f.x, f.y, f.z, f.weight, (int)(item >> kPlaceBits));
+                                               v[0] = 2.0 * v[1];
+                                           });
+        if (threadIdx.x < 2) grid[node] = acc;
+    }
+}
+
+// Merges each node's lists into its contributions, (sorted point | corner << 29) in point order,
+// and, SUMS, adds pass 1 (capi.mojo:171-172): density += 2w, screen += w.  Cursors, current and next
+// point of all eight lists stay in registers; the next point is read an addition ahead.  The last
+// unit_blocks blocks rank the long lists: behind the others, they delay nothing where there are none
+// (50,000 points at depth 6 173 -> 162 us; 159 without them).
 template <bool SUMS>
 __global__ void __launch_bounds__(256) merge_kernel(Cells g, Nodes nodes, const uint32_t* __restrict__ order,
                                                     const Frac* __restrict__ frac, uint32_t* __restrict__ list,
-                                                    double* __restrict__ density, double* __restrict__ screen) {
-    const uint32_t count = nodes.counters[0];
-    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
+                                                    double* __restrict__ density, double* __restrict__ screen,
+                                                    uint32_t unit_blocks) {
+    const uint32_t merge_blocks = gridDim.x - unit_blocks;
+    if (blockIdx.x >= merge_blocks) {
+        const uint32_t units = nodes.counters[2];
+        for (uint32_t u = blockIdx.x - merge_blocks; u < units; u += unit_blocks)
+            rank_unit(g, nodes, order, list, nodes.units[u]);
+        return;
+    }
+    const uint32_t count = nodes.counters[0], stride = merge_blocks * blockDim.x;
+    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += stride) {
+        const uint32_t length = nodes.length[slot];
+        if (length > nodes.long_over) continue;
         const uint32_t node = nodes.node[slot], row = g.by_n.div(node), z = g.by_n.div(row), x = node - row * g.n,
                        y = row - z * g.n;
         uint32_t* __restrict__ out = list + nodes.base[slot];
@@ -281,7 +413,6 @@ __global__ void __launch_bounds__(256) merge_kernel(Cells g, Nodes nodes, const 
             d = density[node];
             s = screen[node];
         }
-        const uint32_t length = nodes.length[slot];
         for (uint32_t t = 0; t < length; ++t) {
             uint32_t least = point[0];
 #pragma unroll
@@ -335,16 +466,46 @@ __global__ void __launch_bounds__(256) density_factor_kernel(int64_t count, int6
 
 // Pass 2 (capi.mojo:221-223): V -= n_hat * (w * res / factor), per node in point order, into dense
 // grids or, COMPACT, into v[slot]; and the density divided by samples_per_node (core.py:255; COMPACT:
-// only the touched nodes, 0 / samples_per_node being 0 elsewhere).
+// only the touched nodes, 0 / samples_per_node being 0 elsewhere).  The last long_blocks blocks take the
+// long lists.
 template <bool COMPACT>
 __global__ void __launch_bounds__(256) vector_kernel(Nodes nodes, const uint32_t* __restrict__ list,
                                                      const Frac* __restrict__ frac, const Unit* __restrict__ unit,
                                                      double res, double* __restrict__ vx, double* __restrict__ vy,
                                                      double* __restrict__ vz, double* __restrict__ density,
-                                                     double samples_per_node) {
-    const uint32_t count = nodes.counters[0];
-    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
+                                                     double samples_per_node, uint32_t long_blocks) {
+    auto values = [&](uint32_t item, double (&v)[3]) {  // what a contribution takes from V
+        const uint32_t place = item & ((1u << kPlaceBits) - 1u);
+        const Frac f = load32(frac + place);
+        const Unit u = load32(unit + place);
+        const double w = corner_weight(clamp01(f.x), clamp01(f.y), clamp01(f.z), f.weight, (int)(item >> kPlaceBits));
+        const double vw = w * res / u.factor;
+        v[0] = u.x * vw;
+        v[1] = u.y * vw;
+        v[2] = u.z * vw;
+    };
+    const uint32_t walk_blocks = gridDim.x - long_blocks;
+    if (blockIdx.x >= walk_blocks) {
+        const uint32_t longs = nodes.counters[3];
+        for (uint32_t i = blockIdx.x - walk_blocks; i < longs; i += long_blocks) {
+            const uint32_t slot = nodes.longs[i], node = nodes.node[slot], at = COMPACT ? slot : node;
+            double* grid = threadIdx.x == 0 ? vx : threadIdx.x == 1 ? vy : vz;
+            const double acc = add_in_order<3>(list + nodes.base[slot], nodes.length[slot],
+                                               !COMPACT && threadIdx.x < 3 ? grid[at] : 0.0,
+                                               [&](uint32_t item, double (&v)[3]) {
+                                                   values(item, v);
+#pragma unroll
+                                                   for (int c = 0; c < 3; ++c) v[c] = -v[c];
+                                               });
+            if (threadIdx.x < 3) grid[at] = acc;
+            if (COMPACT && threadIdx.x == 0) density[node] = density[node] / samples_per_node;
+        }
+        return;
+    }
+    const uint32_t count = nodes.counters[0], stride = walk_blocks * blockDim.x;
+    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += stride) {
         const uint32_t node = nodes.node[slot], length = nodes.length[slot];
+        if (length > nodes.long_over) continue;
         const uint32_t* __restrict__ in = list + nodes.base[slot];
         const uint32_t at = COMPACT ? slot : node;
         double ax = 0.0, ay = 0.0, az = 0.0;
@@ -355,14 +516,11 @@ __global__ void __launch_bounds__(256) vector_kernel(Nodes nodes, const uint32_t
         }
 #pragma unroll 4
         for (uint32_t t = 0; t < length; ++t) {
-            const uint32_t item = in[t], place = item & ((1u << kPlaceBits) - 1u);
-            const Frac f = load32(frac + place);
-            const Unit u = load32(unit + place);
-            const double w = corner_weight(clamp01(f.x), clamp01(f.y), clamp01(f.z), f.weight, (int)(item >> kPlaceBits));
-            const double vw = w * res / u.factor;
-            ax -= u.x * vw;
-            ay -= u.y * vw;
-            az -= u.z * vw;
+            double v[3];
+            values(in[t], v);
+            ax -= v[0];
+            ay -= v[1];
+            az -= v[2];
         }
         vx[at] = ax;
         vy[at] = ay;
@@ -538,6 +696,8 @@ struct Splat {
     Nodes nodes;
     unsigned long long* accepted;
 
+    // Lists longer than `over`, at most: a node has a point at most once.
+    int64_t longs_at_most(uint32_t over = kLongOver) const { return count > over ? 8 * count / over : 0; }
     static int64_t node_capacity(int64_t count, int64_t n) { return std::min(8 * count, n * n * n); }
 
     // nodes_at_most: node_capacity(count, n), or 8 count where n is not known; table: carved unless given later
@@ -557,7 +717,9 @@ struct Splat {
         nodes.node = w.take<uint32_t>(nodes_at_most);
         nodes.base = w.take<uint32_t>(nodes_at_most);
         nodes.length = w.take<uint32_t>(nodes_at_most);
-        nodes.counters = w.take<uint32_t>(2);
+        nodes.counters = w.take<uint32_t>(4);
+        nodes.units = w.take<uint2>(8 * count / kUnit + longs_at_most());
+        nodes.longs = w.take<uint32_t>(longs_at_most());
         accepted = w.take<unsigned long long>(1);
         table = table_cells ? w.take<uint32_t>(table_cells) : nullptr;
         nodes.slot_of = map_nodes ? w.take<uint32_t>(map_nodes) : nullptr;
@@ -575,10 +737,11 @@ struct Splat {
     // Up to the touched nodes; keys and vals are the sorted ones afterwards.
     int group(const double* points, const double* normals, int64_t side, int confidence, Workspace& w, cudaStream_t s) {
         n = side;
+        nodes.long_over = long_over_of(n);
         const int64_t c = n - 1;
         const unsigned blocks = blocks_for(count, 256);
         PB_CHECK_CUDA(cudaMemsetAsync(accepted, 0, sizeof(unsigned long long), s), "splat accepted");
-        PB_CHECK_CUDA(cudaMemsetAsync(nodes.counters, 0, 2 * sizeof(uint32_t), s), "splat counters");
+        PB_CHECK_CUDA(cudaMemsetAsync(nodes.counters, 0, 4 * sizeof(uint32_t), s), "splat counters");
         PB_CHECK_CUDA(cudaMemsetAsync(table, 0, (size_t)(c * c * c) * sizeof(uint32_t), s), "splat table");
         if (nodes.slot_of)
             PB_CHECK_CUDA(cudaMemsetAsync(nodes.slot_of, 0, (size_t)(n * n * n) * sizeof(uint32_t), s), "splat map");
@@ -606,10 +769,22 @@ struct Splat {
         return (unsigned)std::min<int64_t>(blocks_for(node_capacity(count, n) * per_node, 256), 16 * kSMs);
     }
 
-    // Pass 1 into dense grids.
-    int pass1(double* density, double* screen, cudaStream_t s) const {
-        merge_kernel<true><<<node_blocks(), 256, 0, s>>>(geometry(), nodes, vals, frac, list, density, screen);
+    // Blocks for the long lists (four resident ones per SM) and for their parts; none where no list can be long.
+    unsigned long_blocks() const { return (unsigned)std::min<int64_t>(longs_at_most(nodes.long_over), 4 * kSMs); }
+    unsigned unit_blocks() const {
+        return long_blocks() ? (unsigned)std::min<int64_t>(8 * count / kUnit + 1, 16 * kSMs) : 0;
+    }
+
+    // The nodes' contributions in order; pass 1 into dense grids unless they are null.
+    int merge(double* density, double* screen, cudaStream_t s) const {
+        const unsigned ranks = unit_blocks(), blocks = ranks + node_blocks();
+        (density ? merge_kernel<true> : merge_kernel<false>)<<<blocks, 256, 0, s>>>(geometry(), nodes, vals, frac, list,
+                                                                                   density, screen, ranks);
         PB_CHECK_LAUNCH("merge_kernel");
+        if (density && long_blocks()) {
+            long_sums_kernel<<<long_blocks(), 256, 0, s>>>(nodes, list, frac, density, screen);
+            PB_CHECK_LAUNCH("long_sums_kernel");
+        }
         return PB_OK;
     }
 
@@ -619,8 +794,8 @@ struct Splat {
         density_factor_kernel<<<blocks_for(count, 256), 256, 0, s>>>(count, n, keys, frac, samples_per_node, density,
                                                                      unit);
         PB_CHECK_LAUNCH("density_factor_kernel");
-        (compact ? vector_kernel<true> : vector_kernel<false>)<<<node_blocks(), 256, 0, s>>>(
-            nodes, list, frac, unit, (double)(n - 1), vx, vy, vz, density, samples_per_node);
+        (compact ? vector_kernel<true> : vector_kernel<false>)<<<long_blocks() + node_blocks(), 256, 0, s>>>(
+            nodes, list, frac, unit, (double)(n - 1), vx, vy, vz, density, samples_per_node, long_blocks());
         PB_CHECK_LAUNCH("vector_kernel");
         return PB_OK;
     }
@@ -691,7 +866,7 @@ extern "C" int pb_splat_f64(const double* points, const double* normals, int64_t
     Splat o;
     o.carve(w, point_count, Splat::node_capacity(point_count, n), cubed(n - 1), 0, true);
     PB_TRY(o.group(points, normals, n, (int)confidence, w, s));
-    PB_TRY(o.pass1(density, screen, s));
+    PB_TRY(o.merge(density, screen, s));
     PB_TRY(o.pass2(density, samples_per_node, vx, vy, vz, false, s));
     return o.store_accepted(accepted, s);
 }
@@ -728,7 +903,7 @@ extern "C" int pb_splat_assemble_f64(const double* points, const double* normals
     CompactVectors v;
     v.carve(w, cap);
     PB_TRY(o.group(points, normals, n, (int)confidence, w, s));
-    PB_TRY(o.pass1(density, screen, s));
+    PB_TRY(o.merge(density, screen, s));
     PB_TRY(o.pass2(density, samples_per_node, v.x, v.y, v.z, true, s));
     const int planes = n >= 129 ? 8 : 2;
     assemble_compact_kernel<<<dim3(blocks_for(n * n, 256), (unsigned)((n + planes - 1) / planes)), 256, 0, s>>>(
@@ -789,8 +964,7 @@ extern "C" int pb_splat_attributes_f64(const double* points, const double* norma
     o.carve(w, point_count, 8 * point_count, 0, 0, false);
     o.table = (uint32_t*)grids;  // the cells' table until the nodes' contributions are listed
     PB_TRY(o.group(points, normals, n, (int)confidence, w, s));
-    merge_kernel<false><<<o.node_blocks(), 256, 0, s>>>(o.geometry(), o.nodes, o.vals, o.frac, o.list, nullptr, nullptr);
-    PB_CHECK_LAUNCH("merge_kernel");
+    PB_TRY(o.merge(nullptr, nullptr, s));
     PB_CHECK_CUDA(cudaMemsetAsync(grids, 0, bytes, s), "splat attributes zero");
     attribute_sums_kernel<true><<<o.node_blocks((int)channels + 1), 256, 0, s>>>(
         o.nodes, o.list, o.frac, o.vals, attributes, (uint32_t)channels, cubed(n), grids);
@@ -844,8 +1018,7 @@ extern "C" int pb_interpolate_attributes_f64(const double* points, const double*
     double* sums = w.take<double>(cap * (channels + 1));
     double* sorted = w.take<double>(point_count * channels);
     PB_TRY(o.group(points, normals, n, (int)confidence, w, s));
-    merge_kernel<false><<<o.node_blocks(), 256, 0, s>>>(o.geometry(), o.nodes, o.vals, o.frac, o.list, nullptr, nullptr);
-    PB_CHECK_LAUNCH("merge_kernel");
+    PB_TRY(o.merge(nullptr, nullptr, s));
     gather_attributes_kernel<<<blocks_for(point_count * channels, 256), 256, 0, s>>>(attributes, o.vals, point_count,
                                                                                     (uint32_t)channels, sorted);
     PB_CHECK_LAUNCH("gather_attributes_kernel");
