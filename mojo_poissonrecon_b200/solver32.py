@@ -448,7 +448,7 @@ class RefinedEngine:
         """Level 0, x[0] = 0.5 and its residual (FP32, for the first V-cycle), ||r||^2,
         ||b||; iteration counter and first-step flag reset.  Engines that are not
         lean copy rhs and screen: their graph reads them there."""
-        copies = (None, None) if self.lean else (self.b, self.screen)
+        copies = [None if own is t else own for own, t in ((self.b, rhs), (self.screen, screen))]
         self.h.start(rhs, screen, self.pw, copies, self.xs[0], self.norm2, self.bnorm, self.ws)
         self.flags.zero_()
         self.flags[0:1].fill_(1)
@@ -496,9 +496,19 @@ class RefinedEngine:
         self.setup_graph.replay()
         self.lib.pb_note_launches(self.prologue_launches)  # the replayed kernels, for the launch counter
 
+    def _dense(self, grid: torch.Tensor, own: torch.Tensor | None) -> torch.Tensor:
+        """`grid` where the kernels can read it as it is (a dense FP64 cube on this
+        device), else a copy in `own` (None: a new grid), by the rules of Tensor.copy_."""
+        if (grid.dtype == torch.float64 and grid.device == self.flags.device and tuple(grid.shape) == (self.n,) * 3
+                and grid.is_contiguous()):
+            return grid
+        return (self._f64() if own is None else own).copy_(grid)
+
     def _solve(self, rhs: torch.Tensor, screen: torch.Tensor, tol: float, max_cycles: int):
         L, s = self.lib, nat.stream_handle()
         stats = SolveStats()
+        rhs = self._dense(rhs, None if self.lean else self.b)
+        screen = self._dense(screen, None if self.lean else self.screen)
         if self.lean:
             self.screen, self.b = screen, rhs
             self._vectors()
