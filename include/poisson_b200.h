@@ -434,8 +434,7 @@ int pb_coarse27_cycle_f32(int64_t count, const int64_t *sizes, const float *imag
                           int64_t pre, int64_t post, int64_t inner, void *stream);
 
 /* A whole preconditioner hierarchy's set-up from one call: the launches of
- * pb_level_setup_f32 (level 0 from the FP64 screen, or, screen NULL, none: its arrays are there
- * already; for a 27-point level 0 also
+ * pb_level_setup_f32 (level 0 from the FP64 screen; for a 27-point level 0 also
  * pb_level27_from7_f32 and pb_level27_finish_f32), then per level l >= 1
  * pb_galerkin_f32 from level l-1, pb_level27_finish_f32, and pb_pack27_f32 of
  * level l-1 when it is packed; pb_coarse_inverse_f64 of the last level and
@@ -450,7 +449,8 @@ int pb_hierarchy_setup_f32(int64_t levels, const int64_t *sides, const void *con
                            const double *screen, double point_weight, void *galerkin_ws, size_t galerkin_bytes,
                            double *inverse, float *image, size_t image_bytes, void *stream);
 /* The same with the occupancy words of level 0's screen (pb_refine_start_sparse_f64; NULL: none), which let the
- * product from level 0 write constants where there is no screening. */
+ * product from level 0 write constants where there is no screening.  screen NULL: level 0's arrays D, invD and
+ * weights are there already (pb_refine_start_sparse_f64 writes them), no pb_level_setup_f32. */
 int pb_hierarchy_setup_sparse_f32(int64_t levels, const int64_t *sides, const void *const *arrays,
                                   int64_t first_coarse, const double *screen, double point_weight,
                                   const void *occupancy, void *galerkin_ws, size_t galerkin_bytes, double *inverse,

@@ -1486,6 +1486,7 @@ extern "C" int pb_hierarchy_setup_f32(int64_t levels, const int64_t* sides, cons
                                       int64_t first_coarse, const double* screen, double point_weight,
                                       void* galerkin_ws, size_t galerkin_bytes, double* inverse, float* image,
                                       size_t image_bytes, void* stream) {
+    if (!screen) return fail(PB_ERR_INVALID, "hierarchy setup: null screen");
     return pb_hierarchy_setup_sparse_f32(levels, sides, arrays, first_coarse, screen, point_weight, nullptr, galerkin_ws,
                                          galerkin_bytes, inverse, image, image_bytes, stream);
 }
