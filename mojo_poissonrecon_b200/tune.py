@@ -8,8 +8,8 @@ its launchers consult; this module fills it by measurement:
 * for each parameter and side it times every candidate value with CUDA events
   (the median of `repeats` launches after warm-up launches) on synthetic
   buffers of that side, and keeps the fastest;
-* results are cached in a JSON file keyed by the GPU's name and the side
-  (MPR_B200_TUNE_CACHE, default ~/.cache/mojo_poissonrecon_b200/tune.json),
+* results are cached in a JSON file keyed by the GPU's name, the side and
+  KERNELS (MPR_B200_TUNE_CACHE, default ~/.cache/mojo_poissonrecon_b200/tune.json),
   so a process applies the stored choice without measuring again.
 
 Parameters searched (PB_TUNE_*): the TMA sweep's planes per block (z chunk),
@@ -44,6 +44,9 @@ SEARCHED = (SWEEP_VARIANT, SWEEP_Z_CHUNK, RESTRICT_VARIANT, RESTRICT_PLANES, PRO
             FCG_UPDATE_VARIANT, RELAX27_VARIANT, RESIDUAL27_VARIANT)
 # Searched per packed level side of the hierarchy (not per the top side).
 PER_LEVEL = (RELAX27_VARIANT, RESIDUAL27_VARIANT)
+# Counts the changes of what a stored value means or was measured on (a parameter's
+# codes, the kernels behind it): a choice made for other kernels is not applied.
+KERNELS = 2
 _LOCK = threading.Lock()
 
 
@@ -113,7 +116,7 @@ def store_cache(entries: dict, path: str | None = None) -> None:
 
 
 def cache_key(gpu: str, n: int) -> str:
-    return f"{gpu}|n={n}"
+    return f"{gpu}|n={n}|kernels={KERNELS}"
 
 
 def apply(lib, gpu: str, n: int, path: str | None = None) -> dict:
