@@ -6,8 +6,9 @@ of launch parameters per grid side (pb_tune_set, include/poisson_b200.h) that
 its launchers consult; this module fills it by measurement:
 
 * for each parameter and side it times every candidate value with CUDA events
-  (the median of `repeats` launches after warm-up launches) on synthetic
-  buffers of that side, and keeps the fastest;
+  (the median of `repeats` launches after warm-up launches) as the solver
+  launches it, on the system of a surface sampled at that side, and keeps the
+  fastest;
 * results are cached in a JSON file keyed by the GPU's name, the side and
   KERNELS (MPR_B200_TUNE_CACHE, default ~/.cache/mojo_poissonrecon_b200/tune.json),
   so a process applies the stored choice without measuring again.
@@ -137,6 +138,17 @@ def gpu_name(device=None) -> str:
     return torch.cuda.get_device_name(device)
 
 
+def shell_system(n: int, device):
+    """(rhs, screen) with the zeros of a sampled sphere's system: screening in the
+    cells at the surface (1 to 2 % of the nodes at 257^3), a right-hand side up to
+    one node further out."""
+    import torch
+
+    at = torch.arange(n, dtype=torch.float64, device=device) - (n - 1) / 2
+    away = ((at**2)[:, None, None] + (at**2)[:, None] + at**2).sqrt_().sub_(0.35 * (n - 1)).abs_()
+    return (away < 2.0).double() * (n - 1) ** 2, (away < 1.0).double() * 0.5
+
+
 def autotune(n: int, device=None, repeats: int = 10, params=None, path: str | None = None,
              write: bool = True) -> dict:
     """Measure every parameter's candidates at side n on `device`, set the
@@ -155,12 +167,16 @@ def autotune(n: int, device=None, repeats: int = 10, params=None, path: str | No
     l0, l1 = h.levels[0], h.levels[1]
     if not l0.seven:
         raise ValueError(f"autotuning needs a level 0 on the TMA sweep (side >= 33, got {n})")
-    for t in (l0.invD, l0.rhs, l0.ea, l0.eb, l0.D, l0.weights, l1.ea):
-        t.uniform_(0.0, 1.0, generator=gen)
+    b, screen = shell_system(n, dev)
     f64 = lambda: torch.rand((n, n, n), dtype=torch.float64, device=dev, generator=gen)
     f32 = lambda: torch.rand((n, n, n), dtype=torch.float32, device=dev, generator=gen)
-    x0, x1, b, screen = f64(), f64(), f64(), f64()
+    x0, x1 = f64(), f64()
     p0, p1 = f32(), f32()
+    norms = torch.empty(2, dtype=torch.float64, device=dev)
+    h.start(b, screen, 4.0, (None, None), x0, norms[:1], norms[1:], nat.Workspace(dev))  # level 0, occupancy words
+    h.setup(None, 4.0)
+    for t in (l0.ea, l0.eb, l1.ea):
+        t.uniform_(0.0, 1.0, generator=gen)
     scal = torch.tensor([1.0, 0.5, 0.25, 0.0, 0.0, 0, 0, 0], dtype=torch.float64, device=dev)
     flags = torch.tensor([0, 0, 1, 0], dtype=torch.int32, device=dev)
     ws = nat.Workspace(dev)
@@ -183,17 +199,16 @@ def autotune(n: int, device=None, repeats: int = 10, params=None, path: str | No
                     nat.check(lib.pb_residual_restrict_f32(*args, s), "restrict")
             return restrict
         if param == PROLONG_PLANES:
-            return lambda: nat.check(lib.pb_prolong_fac_f32(l1.ea.data_ptr(), l0.eb.data_ptr(),
-                                                            l0.weights.data_ptr(), n, s), "prolong")
+            return lambda: nat.check(lib.pb_prolong_fac_sparse_f32(l1.ea.data_ptr(), l0.eb.data_ptr(),
+                                                                   l0.weights.data_ptr(), h.where, n, s), "prolong")
         if param in (FCG_DIRECTION_PLANES, FCG_DIRECTION_VARIANT):
-            return lambda: nat.check(lib.pb_fcg_direction_f64(l0.ea.data_ptr(), p0.data_ptr(), p1.data_ptr(),
-                                                              l0.rhs.data_ptr(), screen.data_ptr(), n, 4.0,
-                                                              scal.data_ptr(), flags.data_ptr(), ws_ptr, ws_size, s),
-                                     "fcg direction")
-        return lambda: nat.check(lib.pb_fcg_update_f64(l0.ea.data_ptr(), p0.data_ptr(), p1.data_ptr(),
-                                                       x0.data_ptr(), x1.data_ptr(), b.data_ptr(), screen.data_ptr(),
-                                                       l0.rhs.data_ptr(), n, 4.0, scal.data_ptr(), flags.data_ptr(),
-                                                       ws_ptr, ws_size, s), "fcg update")
+            return lambda: nat.check(lib.pb_fcg_direction_sparse_f64(
+                l0.ea.data_ptr(), p0.data_ptr(), p1.data_ptr(), l0.rhs.data_ptr(), screen.data_ptr(), h.where, n, 4.0,
+                scal.data_ptr(), flags.data_ptr(), ws_ptr, ws_size, s), "fcg direction")
+        return lambda: nat.check(lib.pb_fcg_update_sparse_f64(
+            l0.ea.data_ptr(), p0.data_ptr(), p1.data_ptr(), x0.data_ptr(), x1.data_ptr(), b.data_ptr(),
+            screen.data_ptr(), h.where, l0.rhs.data_ptr(), n, 4.0, scal.data_ptr(), flags.data_ptr(), ws_ptr, ws_size,
+            s), "fcg update")
 
     def level_launch(param, lv, nxt):  # one packed sweep or residual-restriction on level lv
         if param == RELAX27_VARIANT:
