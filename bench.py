@@ -24,6 +24,7 @@ Prints one JSON line on rank 0.
 from __future__ import annotations
 
 import argparse
+import datetime
 import gc
 import json
 import os
@@ -87,27 +88,40 @@ def workload(points: int, seed: int = 1):
 # ---- clocks sampled during the timed region ------------------------------------
 
 class ClockSampler:
+    """nvidia-smi's samples between mark() and the end of the `with` block.  It takes some 0.3 s to
+    start, longer than a short timed region, so it starts before the warm-up, and the samples of the
+    region are told by their times."""
+
+    STARTUP = 0.7  # seconds until it has surely started
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
-              "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
+              "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap,timestamp")
 
     def __init__(self, device_index: int):
         self.device_index = device_index
         self.proc = None
         self.path = None
+        self.begin = self.end = None
 
     def __enter__(self):
+        self.begin = time.time()
         fd, self.path = tempfile.mkstemp(suffix=".csv")
         os.close(fd)
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.device_index}", f"--query-gpu={self.FIELDS}", "--format=csv,noheader",
-                 "-lms", "100", "-f", self.path], stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
+                 "-lms", "20", "-f", self.path], stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
         except OSError:
             self.proc = None
         return self
 
+    def mark(self) -> None:
+        """The timed region starts here."""
+        time.sleep(max(0.0, self.STARTUP - (time.time() - self.begin)))
+        self.begin = time.time()
+
     def __exit__(self, *exc):
+        self.end = time.time()
         if self.proc is not None:
             self.proc.terminate()
             try:
@@ -115,13 +129,20 @@ class ClockSampler:
             except subprocess.TimeoutExpired:
                 self.proc.kill()
 
+    @staticmethod
+    def time_of(stamp: str) -> float:  # 2026/01/31 23:59:59.123, local time
+        try:
+            return datetime.datetime.strptime(stamp, "%Y/%m/%d %H:%M:%S.%f").timestamp()
+        except ValueError:
+            return float("nan")
+
     def summary(self) -> dict:
         rows = []
         try:
             with open(self.path, encoding="utf8") as f:
                 for line in f:
                     parts = [p.strip() for p in line.split(",")]
-                    if len(parts) >= 9:
+                    if len(parts) >= 10 and self.begin <= self.time_of(parts[9]) <= self.end:
                         rows.append(parts)
         finally:
             if self.path and os.path.exists(self.path):
@@ -206,22 +227,23 @@ def run_ours(args, rank: int, world: int, dist) -> dict | None:
     def refined_e2e():
         return mpr.reconstruct(host_p, host_n, precision="fp32_refined", device_out=False, **common)
 
-    for _ in range(args.warmup):
-        refined_device()
-        if not args.profile:
-            fp64_device()
-            refined_e2e()
-    torch.cuda.synchronize()
-
-    # The warmed-up heap (torch, the engines, their graphs) goes to the permanent
-    # generation, so a full collection of it cannot land inside a timed step; a
-    # serving process does the same once after start-up.
-    gc.collect()
-    gc.freeze()
-
-    # headline: FP32-refined, inputs resident in HBM
-    launches0 = lib.pb_launch_count()
     with ClockSampler(local) as clocks:
+        for _ in range(args.warmup):
+            refined_device()
+            if not args.profile:
+                fp64_device()
+                refined_e2e()
+        torch.cuda.synchronize()
+
+        # The warmed-up heap (torch, the engines, their graphs) goes to the permanent
+        # generation, so a full collection of it cannot land inside a timed step; a
+        # serving process does the same once after start-up.
+        gc.collect()
+        gc.freeze()
+
+        # headline: FP32-refined, inputs resident in HBM
+        clocks.mark()
+        launches0 = lib.pb_launch_count()
         total_ms, per = timed(refined_device, args.steps)
     launches = lib.pb_launch_count() - launches0
     clock_info = clocks.summary()
