@@ -8,7 +8,9 @@
 // and is replaced by index 0 or the store is skipped, so the kernel finishes
 // without touching memory outside its arrays and the host reads the word
 // (pb_check_status).  In the normal build the helpers compile to the plain
-// index arithmetic and PB_GUARD to nothing.
+// index arithmetic and PB_GUARD to nothing.  The checked build also runs the FP64
+// V-cycle without the 16-block cluster (cycle64.cu: cluster_possible), so that the
+// form for devices without one is tested as well.
 #pragma once
 
 #include <stdint.h>
