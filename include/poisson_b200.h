@@ -148,8 +148,10 @@ int pb_relax_f64(double *solution, const double *rhs, const double *screen, int6
  * hierarchy of sides 2^k + 1 <= 1025, finest first, halving down to 3 (no counterpart in the
  * reference, whose driver calls the operators; same bits as those).  grids: four device pointers per
  * level, (iterate, right-hand side, screening flags, dense screen): the first three hold
- * pb_vcycle_level_size's doubles, doubles and bytes in a layout of the library's own (levels of side
- * <= 17: dense, no flags; below the first of these only the screen is read) and are prepared by
+ * pb_vcycle_level_size's doubles, doubles and bytes in a layout of the library's own (dense, no flags:
+ * levels of side <= 17, and 33 where the current device can place a cluster of 16 blocks; below the
+ * first of these only the screen is read).  The layout depends on the device, so all these calls on one
+ * hierarchy are made with the same current device.  The levels are prepared by
  * pb_vcycle_setup_f64 from the finest dense right-hand side, the finest iterate starting at `init`;
  * the screens are the caller's, dense, and non-negative as point_weight is.  norm (may be null) gets
  * the finest ||rhs - A x||_2 after the last cycle; pb_vcycle_field_f64 the finest iterate as a dense
@@ -426,7 +428,7 @@ size_t pb_coarse27_image_size(int64_t count, const int64_t *sizes);
 int pb_coarse27_image_f32(int64_t count, const int64_t *sizes, const float *const *coef,
                           const float *const *invD, const float *const *weights, const double *inverse,
                           float *image, size_t image_bytes, void *stream);
-/* The V-cycle over those levels in shared memory: (pre, post) sweeps on the
+/* The V-cycle over those levels in one block: (pre, post) sweeps on the
  * first, `inner` each way on the others, the last solved with its inverse.
  * rhs: the first level's right-hand side (padded layout); e receives its
  * correction. */
@@ -491,7 +493,7 @@ int pb_hierarchy_setup_sparse_f32(int64_t levels, const int64_t *sides, const vo
  *   FCG_DIRECTION_FINISH   partials, the cloud's scalars; aux[0] = the cloud's
  *                          pb_batch_fcg_blocks(n, 0)
  *   FCG_UPDATE             z, p0, p1, x0, x1, b, screen, r32, the cloud's scalars,
- *                          partials; aux[0] = point weight bits
+ *                          partials, [occupancy]; aux[0] = point weight bits
  *   FCG_SUM                partials, the cloud's scalars + 4; aux[0] =
  *                          pb_batch_fcg_blocks(n, 1)
  * Partials: pb_batch_fcg_partials(n) doubles per cloud. */
@@ -556,8 +558,8 @@ int pb_batch_loop_condition(unsigned long long handle, const double *scal, const
  *                          plane (a ring slot refilled one step earlier)
  *   FCG_UPDATE_VARIANT     pb_fcg_update_f64: planes prefetched into shared memory by
  *                          cp.async: 0 (and 1 to 3) = the next two, 4 = three
- * The plane counts also apply to the grouped launches described after they are
- * set.  value 0 clears an entry.  Results do not depend on these values, except
+ * The sweep's, restriction's and prolongation's plane counts also apply to the
+ * grouped launches described after they are set.  value 0 clears an entry.  Results do not depend on these values, except
  * the FCG passes' planes per block: they shape the inner products' partial-sum
  * trees, so another value changes results by rounding. */
 enum {

@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(kTailThreads) tail_kernel(const TailArgs a) {
 // last plane is stored to the neighbour's copy too; a phase then ends with one
 // cluster barrier.  The levels below run on block 0 as above.  A node's index,
 // colour and place follow the rule of the tail with the block's own even origin.
-// Measured on B200: a V(3,3) cycle from 33^3 down 124 -> 69 us.
+// Measured on B200: a V(3,3) cycle from 33^3 down 124 -> 68 us within a call of several
+// (336 us for the five of a depth-5 reconstruction); a call of one takes 95, set-up included.
 constexpr int kClusterBlocks = 16, kClusterThreads = 832;  // 1634 nodes of a colour (last block) in two rounds
 
 template <int N, int PLANES>
@@ -1043,7 +1044,8 @@ static dim3 norm_grid(const Split& g) { return dim3(tiles(g.n * g.groups, 256), 
 static int norm_blocks(const Split& g) { return norm_grid(g).x * norm_grid(g).y; }
 
 // Planes a block of the relaxation marches.  257^3: 1 plane 61 us, 2: 51, 4: 48, 6: 47, 8: 48, 16: 51; 129^3: 2 or
-// 4: 8.3, 1: 10.3, 8: 12.4; smaller levels are one wave of latency whatever the split, so one plane each.
+// 4: 8.3, 1: 10.3, 8: 12.4; smaller levels are one wave of latency whatever the split, so one plane each.  Whole
+// cycles: 513^3 4 planes 6.19 ms, 6: 6.15, 8: 6.19, 16: 6.53; 1025^3 4: 47.8, 6: 46.9, 12: 45.8, 24: 46.5.
 static int relax_planes(int n) { return n >= 257 ? 6 : n >= 129 ? 4 : 1; }
 
 template <bool ZERO, bool SPARSE>
@@ -1133,7 +1135,8 @@ static int check_grids(int64_t levels, const int64_t* sides, void* const* grids,
 using namespace pb;
 
 // Sizes of one level of pb_vcycles_f64's hierarchy: doubles of its iterate (and
-// of its right-hand side), bytes of its screening flags.  Sides <= 17 are dense.
+// of its right-hand side), bytes of its screening flags.  Sides <= 17 are dense, and so is 33
+// where the current device can place a cluster of 16 blocks.
 extern "C" int pb_vcycle_level_size(int64_t n, int64_t* doubles, int64_t* flag_bytes) {
     if (n < 3 || n > 1025 || !doubles || !flag_bytes) return fail(PB_ERR_INVALID, "vcycle level size: bad args");
     if (cycle64::tail_side(n)) {
@@ -1197,7 +1200,7 @@ extern "C" size_t pb_vcycle_workspace_size(int64_t n) {
 // `cycles` V(pre, post) cycles of the FP64 multigrid (core.py:141-193) on a
 // hierarchy of sides 2^k + 1, finest first, halving down to 3.  grids: per level
 // (iterate, right-hand side, screening flags, dense screen), prepared by
-// pb_vcycle_setup_f64; levels below the first of side <= 17 need only the screen.
+// pb_vcycle_setup_f64; levels below the first dense one (pb_vcycle_level_size) need only the screen.
 // norm (may be null): the finest level's ||rhs - A x||_2 after the last cycle.
 extern "C" int pb_vcycles_f64(int64_t levels, const int64_t* sides, void* const* grids, double point_weight,
                               int64_t pre, int64_t post, int64_t cycles, double* norm, void* workspace,

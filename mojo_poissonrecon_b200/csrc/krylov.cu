@@ -38,7 +38,9 @@ namespace fcg {
 // Planes per block of the two passes unless the autotuner chose otherwise.  A block
 // walks its planes one after another, so small grids take fewer planes for more
 // blocks: at 65^3, 24 planes leave 81 blocks of pass 2 for 148 SMs (26.6 us), 4 planes
-// 459; pass 1 at 257^3 takes 85 us with 24 planes and 79 with 12, at 513^3 417 and 443.
+// 459; pass 1 at 257^3 takes 85 us with 24 planes and 79 with 12, at 513^3 419 and 443.
+// (Times here and below are of a pass by itself, the L2 overwritten before it; inside a solve
+// pass 1 takes 62 us at 257^3 and 386 at 513^3, pass 2 131 and 978.)
 // Partial sums are sized for the shallowest depth a launch may use, kMinTZ.
 constexpr int kTZ = 24, kMinTZ = 4, kThreads = 128;
 __host__ __device__ constexpr int update_planes_of(int n) { return n <= 65 ? 4 : n <= 129 ? 8 : kTZ; }
@@ -116,7 +118,7 @@ __device__ __forceinline__ double applied(int degree, double pw, double screen, 
 // row's end add zeros.  Bound by latency and by the conversions to double (16 a cycle
 // and SM), not by memory: one x per thread converts 8 values a node and reads the
 // screen everywhere (513^3: 508 us), four x 5.5 and the screen only where it is
-// not zero (417; two x 495).
+// not zero (419; two x 495).
 template <bool ALIGNED>
 __device__ __forceinline__ void direction_sums_body(const float* __restrict__ z, Pad g, const float* __restrict__ p0,
                                                     const float* __restrict__ p1, const float* __restrict__ r32,
@@ -275,7 +277,7 @@ struct Halo {
 // iterates keeps its barrier).  The march is unrolled by the ring, so that slots are
 // constants, and a plane's part of an address is the block's: 155 instructions per 32
 // nodes instead of 225, and bound by the shared-memory pipe (72 %) and issue (64 %).
-// 257^3 157 -> 146 us, 513^3 1240 -> 1013.  Tried: two rows per thread with the loads
+// 257^3 157 -> 147 us, 513^3 1240 -> 1011.  Tried: two rows per thread with the loads
 // ahead in registers (200 us at 257^3, it waits on them in order), and whole rows
 // copied 16 bytes at a time for all threads (165 us: fewer wavefronts, more
 // instructions).  RING = 3 by default, 4 as a tuning variant.

@@ -70,8 +70,8 @@ GALERKIN_SCRATCH = 512 << 20  # bytes; larger Galerkin products run in slabs of 
 # profilers that do not follow kernels inside a graph's conditional node.
 EAGER_LOOP = False
 
-# When true, each engine captures its per-solve prologue (set-up, start, norm)
-# once as a CUDA graph and replays it.
+# When true, each engine captures the coarse levels' set-up of a solve once as a
+# CUDA graph and replays it (the one-pass start before it reads the caller's grids).
 SETUP_GRAPH = True
 
 # Graph captures (the iteration loops here and in batch.py, the prologue graph)
